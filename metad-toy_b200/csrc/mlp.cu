@@ -5,7 +5,7 @@
 // bias representation: src/grids/GH_t0_uniformGrid.cu, GH_t1_sparseGrid.cu).
 //
 // Kernels
-//   k_hillsum_batch   exact FP64 V and dV/ds for a batch of points (hill tiles in shared memory)
+//   hillsum_batch     exact FP64 V and dV/ds for a batch of points (hillsum.cu)
 //   k_hillsum_point   exact FP64 V and dV/ds at one point, hills spread over the grid
 //   k_mlp_tile        128 points per CTA: layer 1 and 3 on CUDA cores, the 128 x 128
 //                     layer and its two backward contractions on tcgen05 (TMEM accumulators)
@@ -28,6 +28,7 @@
 
 #include "../../include/metad_b200.h"
 #include "common.cuh"
+#include "hillsum.h"
 #include "umma.cuh"
 
 namespace mtd {
@@ -337,52 +338,10 @@ __global__ void k_mlp_gradsum(int ntiles, const float *__restrict__ part, float 
     g[q] = s;
 }
 
-// Hills packed as [c0 c1 c2 c3 w 1/(2 sigma^2) 1/sigma^2 0] (FP64).  A hill
-// farther than sqrt(80) sigma from the point contributes below h e^-40
-// (4e-18 h) and is skipped; its gradient term is smaller still.
-constexpr int kHillTile = 256;
+// Hills packed as in hillsum.h.  A hill farther than sqrt(80) sigma from the
+// point contributes below h e^-40 (4e-18 h) and is skipped; its gradient term
+// is smaller still.
 constexpr double kExpCut = 40.0;
-
-// Points and gradients are rows of `ps` / `gs` doubles (kIn, or D for caller
-// layouts); a gradient row of D < gs leaves the rest unwritten.
-__global__ void __launch_bounds__(256) k_hillsum_batch(int D, int npts, const double *__restrict__ pts, int ps, int nh,
-                                                       const double *__restrict__ hills, double *V, double *dV,
-                                                       int gs) {
-    __shared__ double sh[kHillTile * 8];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double s[kIn] = {0, 0, 0, 0};
-    if (i < npts)
-        for (int k = 0; k < D; ++k) s[k] = pts[(size_t)i * ps + k];
-    double v = 0.0, g[kIn] = {0, 0, 0, 0};
-    for (int h0 = 0; h0 < nh; h0 += kHillTile) {
-        const int nt = min(kHillTile, nh - h0);
-        __syncthreads();
-        for (int e = threadIdx.x; e < nt * 8; e += blockDim.x) sh[e] = hills[(size_t)h0 * 8 + e];
-        __syncthreads();
-        for (int h = 0; h < nt; ++h) {
-            const double *c = sh + 8 * h;
-            double r2 = 0.0, d[kIn];
-#pragma unroll
-            for (int k = 0; k < kIn; ++k) {
-                d[k] = k < D ? s[k] - c[k] : 0.0;
-                r2 += d[k] * d[k];
-            }
-            const double a = r2 * c[5];
-            if (a < kExpCut) {
-                const double e = c[4] * exp(-a);
-                v += e;
-#pragma unroll
-                for (int k = 0; k < kIn; ++k) g[k] -= e * d[k] * c[6];
-            }
-        }
-    }
-    if (i < npts) {
-        V[i] = v;
-        if (dV)
-            for (int k = 0; k < min(gs, kIn); ++k)
-                if (k < D || gs == kIn) dV[(size_t)i * gs + k] = g[k];
-    }
-}
 
 // Caller points (rows of D doubles) to the network's normalised FP32 inputs.
 __global__ void k_nb_inputs(int D, int npts, const double *__restrict__ pts, double lo0, double lo1, double lo2,
@@ -524,6 +483,12 @@ struct mtd_nnbias {
     double lo[kIn] = {0, 0, 0, 0}, hi[kIn] = {1, 1, 1, 1};
     double vscale = 1.0;
     cudaStream_t st = nullptr;
+    // scratch of the batched hill sum (grown on demand), the stream of its
+    // last user and an event behind that use: a call on another stream waits
+    void *d_hs = nullptr;
+    size_t cap_hs = 0;
+    cudaStream_t hs_st = nullptr;
+    cudaEvent_t hs_ev = nullptr;
     std::string err;
     std::vector<double> hills;   // packed, 8 doubles per hill
     double *d_hills = nullptr;
@@ -619,6 +584,39 @@ mtd_status nb_refresh_forward(mtd_nnbias *b) {
     return MTD_OK;
 }
 
+// The batched hill sum with its scratch: the object's, or during a stream
+// capture memory of the graph's own (the object's may have grown, and so
+// moved, by the time the graph runs).
+cudaError_t nb_hillsum(mtd_nnbias *b, int npts, const double *pts, int ps, double *V, double *dV, int gs,
+                       cudaStream_t st) {
+    const size_t need = hillsum_scratch(npts, b->nh);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(st, &cap);
+    if (e != cudaSuccess) return e;
+    void *scratch = b->d_hs;
+    if (cap != cudaStreamCaptureStatusNone) {
+        if ((e = cudaMallocAsync(&scratch, need, st)) != cudaSuccess) return e;
+    } else if (need > b->cap_hs) {
+        if ((e = cudaEventSynchronize(b->hs_ev)) != cudaSuccess) return e;
+        cudaFree(b->d_hs);
+        b->d_hs = nullptr;
+        b->cap_hs = 0;
+        if ((e = cudaMalloc(&b->d_hs, need + need / 4)) != cudaSuccess) return e;
+        b->cap_hs = need + need / 4;
+        scratch = b->d_hs;
+    } else if (st != b->hs_st) {
+        if ((e = cudaStreamWaitEvent(st, b->hs_ev, 0)) != cudaSuccess) return e;
+    }
+    e = hillsum_batch(b->D, b->lo, b->hi, npts, pts, ps, b->nh, b->d_hills, V, dV, gs, scratch, st);
+    if (cap != cudaStreamCaptureStatusNone) {
+        const cudaError_t ef = cudaFreeAsync(scratch, st);
+        return e != cudaSuccess ? e : ef;
+    }
+    b->hs_st = st;
+    const cudaError_t er = cudaEventRecord(b->hs_ev, st);
+    return e != cudaSuccess ? e : er;
+}
+
 // Exact FP64 V (and dV) at host points, computed on the device.
 mtd_status nb_exact_host(mtd_nnbias *b, int npts, const double *pts, double *V, double *dV) {
     if (npts <= 0) return MTD_OK;
@@ -630,12 +628,11 @@ mtd_status nb_exact_host(mtd_nnbias *b, int npts, const double *pts, double *V, 
     NB_CU(cudaMalloc(&d_V, sizeof(double) * npts), "values");
     NB_CU(cudaMalloc(&d_dV, sizeof(double) * (size_t)npts * kIn), "gradients");
     cudaMemcpyAsync(d_p, p4.data(), sizeof(double) * p4.size(), cudaMemcpyHostToDevice, b->st);
-    k_hillsum_batch<<<(npts + 255) / 256, 256, 0, b->st>>>(b->D, npts, d_p, kIn, b->nh, b->d_hills, d_V, d_dV,
-                                                           kIn);
+    const cudaError_t el = nb_hillsum(b, npts, d_p, kIn, d_V, d_dV, kIn, b->st);
     std::vector<double> g((size_t)npts * kIn);
     cudaMemcpyAsync(V, d_V, sizeof(double) * npts, cudaMemcpyDeviceToHost, b->st);
     cudaMemcpyAsync(g.data(), d_dV, sizeof(double) * g.size(), cudaMemcpyDeviceToHost, b->st);
-    const cudaError_t e = cudaStreamSynchronize(b->st);
+    const cudaError_t es = cudaStreamSynchronize(b->st), e = el != cudaSuccess ? el : es;
     cudaFree(d_p);
     cudaFree(d_V);
     cudaFree(d_dV);
@@ -716,6 +713,7 @@ mtd_status mtd_nnbias_create(int D, const double *lo, const double *hi, unsigned
     b->seed = seed;
     NB_CU(cudaGetDevice(&b->device), "device");
     NB_CU(cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking), "stream");
+    NB_CU(cudaEventCreateWithFlags(&b->hs_ev, cudaEventDisableTiming), "event");
     NB_CU(cudaMalloc(&b->d_master, sizeof(float) * kNPpad), "params");
     NB_CU(cudaMalloc(&b->d_mom, sizeof(float) * kNPpad), "params");
     NB_CU(cudaMalloc(&b->d_vel, sizeof(float) * kNPpad), "params");
@@ -755,9 +753,10 @@ void mtd_nnbias_destroy(mtd_nnbias *b) {
     if (b->st) cudaStreamSynchronize(b->st);
     void *ptrs[] = {b->d_hills, b->d_master, b->d_mom, b->d_vel, b->d_W1, b->d_b1, b->d_b2, b->d_w3, b->d_b3,
                     b->d_W2, b->d_W2t, b->d_part, b->d_loss, b->d_err, b->d_pt, b->d_pout, b->d_ppart,
-                    b->d_ticket, b->d_xt, b->d_tt, b->d_bx, b->d_by, b->d_bds};
+                    b->d_ticket, b->d_xt, b->d_tt, b->d_bx, b->d_by, b->d_bds, b->d_hs};
     for (void *p : ptrs)
         if (p) cudaFree(p);
+    if (b->hs_ev) cudaEventDestroy(b->hs_ev);
     if (b->st) cudaStreamDestroy(b->st);
     delete b;
 }
@@ -769,7 +768,8 @@ mtd_status mtd_nnbias_add_hills(mtd_nnbias *b, int n, const double *centers, con
     if (!b || n < 0 || (n > 0 && (!centers || !heights || !sigmas))) return MTD_ERR_INVALID_ARG;
     for (int h = 0; h < n; ++h) {
         if (!(sigmas[h] > 0)) return nb_fail(b, MTD_ERR_INVALID_ARG, "hill widths must be positive");
-        double rec[8] = {0, 0, 0, 0, heights[h], 0.5 / (sigmas[h] * sigmas[h]), 1.0 / (sigmas[h] * sigmas[h]), 0};
+        const double s2 = sigmas[h] * sigmas[h];
+        double rec[8] = {0, 0, 0, 0, heights[h], 0.5 / s2, 1.0 / s2, 2.0 * kExpCut * s2};
         for (int k = 0; k < b->D; ++k) rec[k] = centers[(size_t)h * b->D + k];
         b->hills.insert(b->hills.end(), rec, rec + 8);
     }
@@ -1011,8 +1011,7 @@ mtd_status mtd_nnbias_eval_device(mtd_nnbias *b, int npts, const double *d_pts, 
             if (d_dV) NB_CU(cudaMemsetAsync(d_dV, 0, sizeof(double) * npts * b->D, st), "bias");
             return MTD_OK;
         }
-        k_hillsum_batch<<<nb, 256, 0, st>>>(b->D, npts, d_pts, b->D, b->nh, b->d_hills, d_V, d_dV, b->D);
-        NB_CU(cudaGetLastError(), "exact hill sum");
+        NB_CU(nb_hillsum(b, npts, d_pts, b->D, d_V, d_dV, b->D, st), "exact hill sum");
         return MTD_OK;
     }
     if (npts > b->cap_b) {

@@ -1,0 +1,112 @@
+"""The batched exact hill sum (csrc/hillsum.cu) against its NumPy restatement.
+
+Sizes at the edges of the 32-point warps, the 32-hill groups and the splits of
+the hills over warps and clusters; hills along a trajectory and in random
+order, of unequal widths; points outside the box and not finite.
+
+Tolerance, per point: the exponent x = r^2 / (2 s^2) <= 40 carries at most 4
+roundings (2^-53 relative each), so a term is off by at most 40 * 4 * 2^-53 =
+1.8e-14 relative, plus a few 2^-53 of the evaluation and the sum; hills beyond
+the cut miss h e^-40 each.  1e-13 of the sum of the terms' magnitudes.
+"""
+import numpy as np
+import pytest
+
+import mtd
+import systems
+
+pytestmark = pytest.mark.gpu
+
+
+def _hills(n, D, seed, walk):
+    rng = np.random.default_rng(seed)
+    c = systems.cv4_hills(n=n, seed=seed)[0] if walk else \
+        systems.CV4_LO + (systems.CV4_HI - systems.CV4_LO) * rng.random((n, 4))
+    return np.ascontiguousarray(c[:, :D]), rng.uniform(-0.002, 0.005, n), rng.uniform(0.01, 0.04, n)
+
+
+def _sum(p, c, h, s):
+    V, dV = np.zeros(len(p)), np.zeros_like(p)
+    aV, adV = np.zeros(len(p)), np.zeros_like(p)
+    for ck, hk, sk in zip(c, h, s):
+        d = p - ck
+        e = hk * np.exp(-(d * d).sum(1) / (2 * sk * sk))
+        g = -e[:, None] * d / (sk * sk)
+        V += e
+        dV += g
+        aV += np.abs(e)
+        adV += np.abs(g)
+    return V, dV, aV, adV
+
+
+@pytest.mark.parametrize("npts,nh,D,walk", [(1, 1, 4, True), (31, 32, 1, True), (32, 33, 2, False), (33, 65, 3, True),
+                                            (257, 1000, 4, False), (1000, 1023, 4, True), (5000, 31, 3, False),
+                                            (3001, 2500, 4, True)])
+def test_batch_matches_oracle(npts, nh, D, walk):
+    import torch
+
+    lo, hi = systems.CV4_LO[:D], systems.CV4_HI[:D]
+    c, h, s = _hills(nh, D, npts, walk)
+    p = lo + (hi - lo) * (1.2 * np.random.default_rng(nh).random((npts, D)) - 0.1)
+    nb = mtd.NNBias(lo, hi)
+    nb.add_hills(c, h, s)
+    V, dV, aV, adV = _sum(p, c, h, s)
+    cut = nh * np.abs(h).max() * np.exp(-40.0)
+    got = [nb.exact(p)]
+    d_p = torch.from_numpy(p).cuda()
+    d_v = torch.full((npts,), np.nan, dtype=torch.float64, device="cuda")
+    d_g = torch.full((npts, D), np.nan, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    nb.eval_device(npts, d_p.data_ptr(), d_v.data_ptr(), d_g.data_ptr(), use_nn=0)
+    torch.cuda.synchronize()
+    got.append((d_v.cpu().numpy(), d_g.cpu().numpy()))
+    for gv, gd in got:
+        assert np.all(np.abs(gv - V) <= 1e-13 * aV + cut)
+        assert np.all(np.abs(gd - dV) <= 1e-13 * adV + 10 * cut / s.min())
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+    nb.close()
+
+
+def test_points_and_hills_that_are_not_finite_count_nothing():
+    c, h, s = _hills(70, 4, 3, True)
+    p = np.array([c[5], c[40], c[5], c[69]]) + 0.001
+    p[1, 2], p[2, 0] = np.nan, np.inf
+    c2 = np.insert(c, [10, 50], [[np.nan] * 4, [np.inf, 0, 0, 0]], axis=0)
+    h2, s2 = np.insert(h, [10, 50], 1.0), np.insert(s, [10, 50], 0.02)
+    out = []
+    for args in ((c, h, s), (c2, h2, s2)):
+        nb = mtd.NNBias(systems.CV4_LO, systems.CV4_HI)
+        nb.add_hills(*args)
+        out.append(nb.exact(p))
+        nb.close()
+    V, dV, aV, adV = _sum(p[[0, 3]], c, h, s)
+    for gv, gd in out:
+        assert np.all(gv[1:3] == 0) and np.all(gd[1:3] == 0)
+        assert np.all(np.abs(gv[[0, 3]] - V) <= 1e-13 * aV + 1e-18)
+        assert np.all(np.abs(gd[[0, 3]] - dV) <= 1e-13 * adV + 1e-15)
+
+
+def test_batch_replays_from_a_captured_graph():
+    import torch
+
+    c, h, s = _hills(300, 4, 8, True)
+    nb = mtd.NNBias(systems.CV4_LO, systems.CV4_HI)
+    nb.add_hills(c, h, s)
+    rng = np.random.default_rng(1)
+    p = [systems.CV4_LO + (systems.CV4_HI - systems.CV4_LO) * rng.random((500, 4)) for _ in range(2)]
+    d_p = torch.from_numpy(p[0]).cuda()
+    d_v, d_g = torch.zeros(500, dtype=torch.float64, device="cuda"), torch.zeros((500, 4), dtype=torch.float64,
+                                                                                 device="cuda")
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    st = torch.cuda.Stream()
+    with torch.cuda.graph(g, stream=st):
+        nb.eval_device(500, d_p.data_ptr(), d_v.data_ptr(), d_g.data_ptr(), use_nn=0, stream=st.cuda_stream)
+    for q in p:
+        d_p.copy_(torch.from_numpy(q))
+        g.replay()
+        torch.cuda.synchronize()
+        V, dV = nb.exact(q)
+        assert np.array_equal(d_v.cpu().numpy(), V) and np.array_equal(d_g.cpu().numpy(), dV)
+    del g
+    nb.close()
