@@ -263,14 +263,14 @@ mtd_status mtd_autotune(mtd_ctx *ctx, int n, const double *d_x, const int *d_mas
 mtd_status mtd_set_tuning(mtd_ctx *ctx, int neighbor_shape, int q_block, int lambda_block);
 
 /* Shapes of the STRU_FACTOR_K passes, chosen by mtd_autotune when the deck
- * has that CAL: k-vectors per pass over the atoms of the value pass (4, 8 or
- * 16: a register tile of partial sums) and the unroll depth of the force
+ * has that CAL: phases a thread has in flight in the value pass (4, 8 or 16: a
+ * pair of k-vectors by 2, 4 or 8 atoms) and the unroll depth of the force
  * pass's loop over k (1, 2 or 4).  Every k is summed in the same order
  * whatever the shape, so the results are bitwise identical.  Defaults 8, 2. */
 mtd_status mtd_sk_tiles(mtd_ctx *ctx, int *q_values, int *q_force);
 /* Every tuned shape: neighbour search, q block, lambda block (0 = 256),
  * skin-list q pass with its filter in a separate loop (1) or merged with the
- * sum (0), S(k) value-pass k-tile and force-pass unroll. */
+ * sum (0), S(k) value-pass phases in flight and force-pass unroll. */
 mtd_status mtd_get_tuning(mtd_ctx *ctx, int out[6]);
 mtd_status mtd_set_tuning_all(mtd_ctx *ctx, const int in[6]);
 mtd_status mtd_set_sk_tiles(mtd_ctx *ctx, int q_values, int q_force);

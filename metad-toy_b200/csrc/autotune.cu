@@ -98,7 +98,7 @@ mtd_status autotune_idle(mtd_ctx *c, int n, const double *d_x, const int *d_mask
         }
     }
     c->tune_l = bl;
-    // S(k) shapes: k-vectors per pass of the value pass, unroll depth of the force pass
+    // S(k) shapes: phases in flight of the value pass, unroll depth of the force pass
     for (Unit &u : c->units) {
         if (u.kind != CAL_STRU_FACTOR_K) continue;
         best = 1e30f;

@@ -283,6 +283,71 @@ __device__ __forceinline__ void halfturn_sincos_f32(double u, float &s, float &c
     c = __uint_as_float(__float_as_uint(c0) ^ sgn);
 }
 
+// The k-vector passes' form of the same, for a pair of phases: the FP64 sum
+// k.x runs on top of kTurnBase = 1.5 * 2^20, whose last bit is worth 2^-32, so
+// each of its three FMAs rounds the phase to 2^-33 half turns (1.2e-10, where
+// the FP32 remainder itself rounds to 1.5e-8) and the low word of the result
+// is the remainder f = u - n in units of 2^-32, signed, with the parity of n
+// in the bit above it and the low word's sign.  Three FP64 additions and the
+// FP64-to-FP32 conversion (0.44 warp instructions per clock and SM, against
+// 0.95 for the integer one) are gone.  Valid for |u| < 2^18 (kTurnMax).
+constexpr double kTurnBase = 1572864.0;
+constexpr double kTurnMax = 262144.0;
+
+__device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
+// (-1)^n of a phase as a sign mask.
+__device__ __forceinline__ unsigned turn_sign(double t) {
+    return ((unsigned)__double2hiint(t) << 31) ^ ((unsigned)__double2loint(t) & 0x80000000u);
+}
+// sin(pi f) (and cos(pi f)) of two based phases, unsigned, by the polynomials
+// of halfturn_sincos_f32_parts on FP32 pairs (the same roundings per element;
+// one instruction for two FMAs).
+__device__ __forceinline__ float2 turn_sin2(double ta, double tb, float2 &s0) {
+    const float2 zi = make_float2((float)__double2loint(ta), (float)__double2loint(tb));
+    const float2 z = __fmul2_rn(zi, dup2(2.3283064365386963e-10f));   // 2^-32: exact
+    const float2 z2 = __fmul2_rn(z, z);
+    float2 p = __ffma2_rn(z2, dup2(kSinP4), dup2(kSinP3));
+    p = __ffma2_rn(p, z2, dup2(kSinP2));
+    p = __ffma2_rn(p, z2, dup2(kSinP1));
+    p = __ffma2_rn(p, z2, dup2(kSinP0));
+    s0 = __fmul2_rn(p, z);
+    return z2;
+}
+__device__ __forceinline__ void turn_sincos2(double ta, double tb, float2 &s0, float2 &c0) {
+    const float2 z2 = turn_sin2(ta, tb, s0);
+    float2 q = __ffma2_rn(z2, dup2(kCosQ5), dup2(kCosQ4));
+    q = __ffma2_rn(q, z2, dup2(kCosQ3));
+    q = __ffma2_rn(q, z2, dup2(kCosQ2));
+    q = __ffma2_rn(q, z2, dup2(kCosQ1));
+    c0 = __ffma2_rn(q, z2, dup2(kCosQ0));
+}
+
+// FP64: sin(pi f) = f S(f^2) and cos(pi f) = C(f^2) on |f| <= 1/2 by their
+// Taylor polynomials (remainders (pi/2)^23 / 23! = 1e-18 and (pi/2)^22 / 22! =
+// 2e-17), for a phase u in half turns rounded to the nearest integer as above.
+// s and c come with the sign (-1)^n; |u| < 2^51.
+template <bool COS> __device__ __forceinline__ void halfturn_sincos_f64(double u, double &s, double &c) {
+    constexpr double S[11] = {3.141592653589793, -5.16771278004997, 2.5501640398773455, -0.5992645293207921,
+                              0.08214588661112823, -0.0073704309457143504, 0.00046630280576761255,
+                              -2.1915353447830217e-05, 7.952054001475513e-07, -2.2948428997269873e-08,
+                              5.392664662608129e-10};
+    constexpr double C[11] = {1.0, -4.934802200544679, 4.0587121264167685, -1.3352627688545895, 0.2353306303588932,
+                              -0.02580689139001406, 0.0019295743094039231, -0.0001046381049248457,
+                              4.303069587032947e-06, -1.3878952462213771e-07, 3.604730797462501e-09};
+    constexpr double kRound = 6755399441055744.0;   // 1.5 * 2^52
+    const double t = u + kRound, f = u - (t - kRound), z = f * f;
+    const unsigned sgn = (unsigned)__double2loint(t) << 31;
+    double p = S[10], q = C[10];
+#pragma unroll
+    for (int k = 9; k >= 0; --k) {
+        p = fma(p, z, S[k]);
+        if (COS) q = fma(q, z, C[k]);
+    }
+    p *= f;
+    s = __hiloint2double(__double2hiint(p) ^ (int)sgn, __double2loint(p));
+    if (COS) c = __hiloint2double(__double2hiint(q) ^ (int)sgn, __double2loint(q));
+}
+
 // The same for a phase in radians (one FP64 multiply by 1 / pi first).
 __device__ __forceinline__ void phase_sincos_f32(double ph, float &s, float &c) {
     halfturn_sincos_f32(ph * kInvPi, s, c);

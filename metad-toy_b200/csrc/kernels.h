@@ -301,7 +301,7 @@ struct SkDev {
     double *ngroup;             // group count
     const double *coef;         // alpha
     int fp64;
-    int qv, qf;                 // k-vectors per pass of the value pass (4 / 8 / 16), unroll of the force pass (1 / 2 / 4)
+    int qv, qf;                 // phases in flight per thread of the value pass (4 / 8 / 16), unroll of the force pass (1 / 2 / 4)
 };
 void launch_sk_values(const SkDev &d, cudaStream_t st);
 void launch_sk_forces(const SkDev &d, const double *f_src, double *f_dst, const SysDev &s, const CellGrid &g,

@@ -12,6 +12,9 @@
 // the sums over atoms are FP64 block partials reduced in a fixed order.
 #include "kernels.h"
 
+#include <algorithm>
+#include <type_traits>
+
 namespace mtd {
 
 namespace {
@@ -151,235 +154,329 @@ __global__ void __launch_bounds__(kBlock) k_debye_force(DebyeDev<T> d, const dou
 }
 
 // ------------------------------------------------------------------ S(k)
-constexpr int kSkBlocks = 148 * 4;  // grid for the partial sums (4 blocks per SM: more atoms per thread, fewer block sums)
-// Shapes the autotuner picks (SkDev::qv, ::qf): QV k-vectors per pass over
-// the atoms in the partial-sum pass (a register tile of 2 QV sums per thread),
-// and the unroll depth U of the force pass's loop over k.  Every k is summed
-// in the same order whatever the shape, so all give bitwise-identical
-// results.  In mixed precision the phase (k / pi).x is formed in FP64 (B200
-// runs FP64 at half the FP32 rate), reduced to half a turn in FP64 and
-// finished with FP32 polynomials (halfturn_sincos_f32); a per-dimension FP32
-// phase-table variant (three shared-memory loads and an FP32 reduction per
-// pair) measured 2.2x slower and was removed.
+// The value pass sums exp(i k.x) with the k-vectors over the threads: a thread
+// keeps a pair of them and its sums in registers and goes through atoms staged
+// in shared memory, so nothing is summed across lanes until its block is done.
+// (With the atoms over the threads, and every k's sums reduced over the block
+// in FP64, those reductions were 10 of 26 instructions per atom-k pair.)
+// In mixed precision the phase (k / pi).x is formed in FP64 (B200 runs FP64 at
+// half the FP32 rate) with its fraction left in the low word (kTurnBase), and
+// finished with FP32 polynomials on the pair of k-vectors (turn_sincos2); a
+// per-dimension FP32 phase-table variant (three shared-memory loads and an
+// FP32 reduction per pair) measured 2.2x slower and was removed.
+// The shapes the autotuner picks (SkDev::qv: 2, 4 or 8 atoms in flight per
+// thread in the value pass; SkDev::qf: the unroll depth of the force pass's
+// loop over k) leave every sum's order as it is.
+constexpr int kSkBlocks = 148 * 4;   // resident blocks of both passes
+constexpr int kSkChunk = 512;        // atoms staged at a time in the value pass
+constexpr int kSkFlush = 8;          // atoms summed in FP32 before they join the FP64 sums
 
-template <bool FP64, int QV> __global__ void __launch_bounds__(256) k_sk_partial(SkDev d) {
-    constexpr int kSkChunk = 2 * QV;   // reals per register tile
-    pdl_entry();
-    __shared__ double smem[kSkChunk * 32];
-    extern __shared__ double kk[];   // 3K
-    // mixed precision: k / pi, so the phases come out in half turns
-    for (int t = threadIdx.x; t < 3 * d.K; t += blockDim.x) kk[t] = FP64 ? d.k[t] : d.k[t] * kInvPi;
+// Largest |component| of k / pi over all k-vectors, on every thread of the
+// block: |u| of an atom is at most that times |x| + |y| + |z|.
+__device__ __forceinline__ double sk_kmax(const SkDev &d, double *smem /* 8 */) {
+    double m = 0.0;
+    for (int t = threadIdx.x; t < 3 * d.K; t += blockDim.x) m = fmax(m, fabs(d.k[t]) * kInvPi);
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) smem[threadIdx.x >> 5] = m;
     __syncthreads();
-    double cnt = 0.0;
-    for (int k0 = 0; k0 < d.K; k0 += QV) {
-        double acc[kSkChunk];
-        // mixed precision: a thread's few atoms (grid-stride, about n / (592 * 256))
-        // are summed in FP32, every sum across threads and blocks in FP64
-        float facc[kSkChunk];
+    for (int w = 0; w < (int)blockDim.x >> 5; ++w) m = fmax(m, smem[w]);
+    return m;
+}
+
+// sin(pi f), cos(pi f) (unsigned) and the sign masks of one atom's phases with
+// a pair of k-vectors (/ pi); far: beyond the base's range or not finite, the
+// phase is then rounded in FP64.
+__device__ __forceinline__ void sk_pair(bool far, double2 kx, double2 ky, double2 kz, double x, double y, double z,
+                                        float2 &s0, float2 &c0, unsigned &ga, unsigned &gb) {
+    if (!far) {
+        const double ta = fma(kz.x, z, fma(ky.x, y, fma(kx.x, x, kTurnBase)));
+        const double tb = fma(kz.y, z, fma(ky.y, y, fma(kx.y, x, kTurnBase)));
+        turn_sincos2(ta, tb, s0, c0);
+        ga = turn_sign(ta);
+        gb = turn_sign(tb);
+    } else {
+        ga = halfturn_sincos_f32_parts(kx.x * x + ky.x * y + kz.x * z, s0.x, c0.x);
+        gb = halfturn_sincos_f32_parts(kx.y * x + ky.y * y + kz.y * z, s0.y, c0.y);
+    }
+}
+
+// Threads are streams of np (a tile's pairs of k) each: stream s of S takes
+// staged atoms s, s + S, ....  Block b sums atoms b * per .. (b + 1) * per - 1.
+// Bound by the SM's dispatch: 21 instructions per atom-k pair, of which the 3
+// FP64 and 7 paired FP32 ones take two cycles each (38 cycles a pair are
+// measured, the FMA pipe is 46 % busy).  1,048,576 atoms x 96 k: 147 us before
+// (26 instructions with 6 FP64 and the slow conversion, atoms over the
+// threads), 112 now; FP64 at 108,000 x 24: 22 us (sincos()), 17 now.
+template <bool FP64, int U> __global__ void __launch_bounds__(256, FP64 ? 2 : 4) k_sk_partial(SkDev d, int per) {
+    pdl_entry();
+    __shared__ double2 xy[kSkChunk];
+    __shared__ double zz[kSkChunk];
+    __shared__ double smem[8];
+    __shared__ int wcount[2][8];
+    const int np = (d.K + 1) / 2, ntile = (np + 63) / 64, TP = (np + ntile - 1) / ntile, S = (int)blockDim.x / TP;
+    const int st = threadIdx.x / TP, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int a0 = min(blockIdx.x * per, d.nown), a1 = min(a0 + per, d.nown);
+    const double reach = FP64 ? 0.0 : kTurnMax / fmax(sk_kmax(d, smem), 1e-300);
+    int total = 0;
+    for (int tile = 0; tile < ntile; ++tile) {
+        const int p = tile * TP + (int)threadIdx.x % TP;
+        const bool active = st < S && p < np;
+        double2 kv[3];
 #pragma unroll
-        for (int t = 0; t < kSkChunk; ++t) {
-            acc[t] = 0.0;
-            facc[t] = 0.f;
-        }
-        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < d.nown; i += gridDim.x * blockDim.x) {
-            if (d.mask && !(d.mask[i] & d.groupbit)) continue;
-            if (k0 == 0) cnt += 1.0;
-            const double x = d.x[3 * i], y = d.x[3 * i + 1], z = d.x[3 * i + 2];
+        for (int c = 0; c < 3; ++c)   // an odd K is filled up with a zero vector, whose sums are not written
+            kv[c] = make_double2(active ? d.k[6 * p + c] * kInvPi : 0.0,
+                                 active && 2 * p + 1 < d.K ? d.k[6 * p + 3 + c] * kInvPi : 0.0);
+        double c64[2] = {0.0, 0.0}, s64[2] = {0.0, 0.0};
+        for (int c0 = a0; c0 < a1; c0 += kSkChunk) {
+            // the group's atoms of the chunk, in order
+            double px[2], py[2], pz[2];
+            bool keep[2], is_far = false;
+            unsigned ball[2];
+            __syncthreads();
 #pragma unroll
-            for (int q = 0; q < QV; ++q) {
-                const int kq = k0 + q;
-                if (kq < d.K) {
-                    const double ph = kk[3 * kq] * x + kk[3 * kq + 1] * y + kk[3 * kq + 2] * z;
-                    if (FP64) {
-                        double s, c;
-                        sincos(ph, &s, &c);
-                        acc[2 * q] += c;
-                        acc[2 * q + 1] += s;
+            for (int r = 0; r < 2; ++r) {
+                const int i = c0 + (int)threadIdx.x + 256 * r;
+                keep[r] = i < a1 && (!d.mask || (d.mask[i] & d.groupbit));
+                ball[r] = __ballot_sync(0xffffffffu, keep[r]);
+                if (lane == 0) wcount[r][warp] = __popc(ball[r]);
+                if (keep[r]) {
+                    px[r] = d.x[3 * i];
+                    py[r] = d.x[3 * i + 1];
+                    pz[r] = d.x[3 * i + 2];
+                    is_far = is_far || !(fabs(px[r]) + fabs(py[r]) + fabs(pz[r]) < reach);
+                }
+            }
+            __syncthreads();
+            int m = 0;
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                int at = m + __popc(ball[r] & ((1u << lane) - 1));
+                for (int w = 0; w < 8; ++w) {
+                    if (w < warp) at += wcount[r][w];
+                    m += wcount[r][w];
+                }
+                if (keep[r]) {
+                    xy[at] = make_double2(px[r], py[r]);
+                    zz[at] = pz[r];
+                }
+            }
+            const bool any_far = __syncthreads_or(is_far && !FP64);
+            total += m;
+            if (!active) continue;
+            int j = st;
+            if constexpr (FP64) {
+#pragma unroll U
+                for (; j < m; j += S) {
+                    const double2 q = xy[j];
+                    const double z = zz[j];
+                    double s, c;
+                    halfturn_sincos_f64<true>(fma(kv[2].x, z, fma(kv[1].x, q.y, kv[0].x * q.x)), s, c);
+                    c64[0] += c;
+                    s64[0] += s;
+                    halfturn_sincos_f64<true>(fma(kv[2].y, z, fma(kv[1].y, q.y, kv[0].y * q.x)), s, c);
+                    c64[1] += c;
+                    s64[1] += s;
+                }
+            } else {
+                while (j < m) {
+                    float2 fc = make_float2(0.f, 0.f), fs = fc;
+                    auto add = [&](int e, bool far) {
+                        const double2 q = xy[e];
+                        float2 s0, c0f;
+                        unsigned ga, gb;
+                        sk_pair(far, kv[0], kv[1], kv[2], q.x, q.y, zz[e], s0, c0f, ga, gb);
+                        // the sign (-1)^n as a factor of exact FMAs: the same sums
+                        // as adding the signed sin and cos
+                        const float2 sg = make_float2(__uint_as_float(0x3f800000u | ga), __uint_as_float(0x3f800000u | gb));
+                        fc = __ffma2_rn(sg, c0f, fc);
+                        fs = __ffma2_rn(sg, s0, fs);
+                    };
+                    if (!any_far && j + (kSkFlush - 1) * S < m) {
+#pragma unroll U
+                        for (int e = 0; e < kSkFlush; ++e) add(j + e * S, false);
                     } else {
-                        // the sign (-1)^n as a factor of exact FMAs: the same
-                        // sums as adding the signed sin and cos
-                        float s0, c0;
-                        const unsigned sgn = halfturn_sincos_f32_parts(ph, s0, c0);
-                        const float sg = __uint_as_float(0x3f800000u | sgn);
-                        facc[2 * q] = fmaf(sg, c0, facc[2 * q]);
-                        facc[2 * q + 1] = fmaf(sg, s0, facc[2 * q + 1]);
+                        for (int e = j; e < min(m, j + kSkFlush * S); e += S) {
+                            const double2 q = xy[e];
+                            add(e, !(fabs(q.x) + fabs(q.y) + fabs(zz[e]) < reach));
+                        }
                     }
+                    j += kSkFlush * S;
+                    c64[0] += (double)fc.x;
+                    c64[1] += (double)fc.y;
+                    s64[0] += (double)fs.x;
+                    s64[1] += (double)fs.y;
                 }
             }
         }
-        if (!FP64) {
-#pragma unroll
-            for (int t = 0; t < kSkChunk; ++t) acc[t] = facc[t];
-        }
-        // the chunk's 2 QV block totals land on the lanes of warp 0 (lane l:
-        // value l >> (5 - log2(2 QV))), which write them side by side
-        const double tot = block_sum_spread<kSkChunk>(acc, smem);
-        constexpr int kSh = 5 - Log2NV<kSkChunk>::v;
-        if (threadIdx.x < 32 && (threadIdx.x & ((1 << kSh) - 1)) == 0) {
-            const int v = threadIdx.x >> kSh;
-            if (k0 + (v >> 1) < d.K) d.partials[(size_t)blockIdx.x * (2 * d.K + 2) + 2 * k0 + v] = tot;
-        }
+        // the streams' sums in stream order; partials are one row of blocks per value
         __syncthreads();
+        static_assert(sizeof(xy) >= 4 * 256 * sizeof(double), "the sums fit over the staged atoms");
+        double *red = &xy[0].x;
+        red[threadIdx.x] = c64[0];
+        red[256 + threadIdx.x] = s64[0];
+        red[512 + threadIdx.x] = c64[1];
+        red[768 + threadIdx.x] = s64[1];
+        __syncthreads();
+        for (int e = threadIdx.x; e < 4 * TP; e += blockDim.x) {
+            const int v = 4 * (tile * TP + e % TP) + e / TP;
+            if (v >= 2 * d.K) continue;
+            double sum = 0.0;
+            for (int q = 0; q < S; ++q) sum += red[e / TP * 256 + q * TP + e % TP];
+            d.partials[(size_t)v * d.nblocks + blockIdx.x] = sum;
+        }
     }
-    double c1[1] = {cnt};
-    block_sum<1>(c1, smem);
-    if (threadIdx.x == 0) d.partials[(size_t)blockIdx.x * (2 * d.K + 2) + 2 * d.K] = c1[0];
+    if (threadIdx.x == 0) d.partials[(size_t)(2 * d.K) * d.nblocks + blockIdx.x] = (double)(total / ntile);
 }
 
-// One block per output value (2K rho components + the group count).
+// One warp per output value (2K rho components + the group count).
 __global__ void __launch_bounds__(256) k_sk_reduce(SkDev d) {
     pdl_entry();
-    __shared__ double smem[32];
-    const int v = blockIdx.x;
-    double acc[1] = {0.0};
-    for (int b = threadIdx.x; b < d.nblocks; b += blockDim.x) acc[0] += d.partials[(size_t)b * (2 * d.K + 2) + v];
-    block_sum<1>(acc, smem);
-    if (threadIdx.x == 0) {
-        if (v < 2 * d.K) d.rho[v] = acc[0];
-        else *d.ngroup = acc[0];
+    const int v = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (v > 2 * d.K) return;
+    double acc = 0.0;
+    for (int b = lane; b < d.nblocks; b += 32) acc += d.partials[(size_t)v * d.nblocks + b];
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) {
+        if (v < 2 * d.K) d.rho[v] = acc;
+        else *d.ngroup = acc;
     }
 }
 
-// FP64 force pass: one atom per thread, FP64 sincos of the FP64 phase.
-template <int U>
-__global__ void __launch_bounds__(256) k_sk_force(SkDev d, const double *__restrict__ f_src, double *__restrict__ f_dst,
-                                                  SysDev s, CellGrid g, double *vpart) {
-    pdl_entry();
-    __shared__ double smem[6 * 32];
-    extern __shared__ double kk[];   // 3K doubles of k, then 2K of rho
-    double *rr = kk + 3 * d.K;
-    for (int t = threadIdx.x; t < 3 * d.K; t += blockDim.x) kk[t] = d.k[t];
-    for (int t = threadIdx.x; t < 2 * d.K; t += blockDim.x) rr[t] = d.rho[t];
-    __syncthreads();
-    const double a = d.coef[0];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double vir[6] = {0, 0, 0, 0, 0, 0};
-    if (i < d.n) {
-        double gx = 0, gy = 0, gz = 0;
-        if (i < d.nown && (!d.mask || (d.mask[i] & d.groupbit))) {
-            const double x = d.x[3 * i], y = d.x[3 * i + 1], z = d.x[3 * i + 2];
-#pragma unroll U
-            for (int q = 0; q < d.K; ++q) {
-                const double ph = kk[3 * q] * x + kk[3 * q + 1] * y + kk[3 * q + 2] * z;
-                double sn, cs;
-                sincos(ph, &sn, &cs);
-                const double w = -rr[2 * q] * sn + rr[2 * q + 1] * cs;
-                gx += w * kk[3 * q];
-                gy += w * kk[3 * q + 1];
-                gz += w * kk[3 * q + 2];
-            }
+// f_dst = f_src + (gx, gy, gz) of atom i and its virial term.
+__device__ __forceinline__ void sk_apply(const SkDev &d, const SysDev &s, const CellGrid &g, int i, double gx,
+                                         double gy, double gz, const double *__restrict__ f_src,
+                                         double *__restrict__ f_dst, bool virial, double (&vir)[6]) {
+    f_dst[3 * i] = f_src[3 * i] + gx;
+    f_dst[3 * i + 1] = f_src[3 * i + 1] + gy;
+    f_dst[3 * i + 2] = f_src[3 * i + 2] + gz;
+    if (virial) {
+        double ux = d.x[3 * i], uy = d.x[3 * i + 1], uz = d.x[3 * i + 2];
+        if (s.image) {
+            int ix, iy, iz;
+            unpack_image(s.image[i], ix, iy, iz);
+            ux += ix * g.L[0];
+            uy += iy * g.L[1];
+            uz += iz * g.L[2];
         }
-        const double fx = -a * gx, fy = -a * gy, fz = -a * gz;
-        f_dst[3 * i] = f_src[3 * i] + fx;
-        f_dst[3 * i + 1] = f_src[3 * i + 1] + fy;
-        f_dst[3 * i + 2] = f_src[3 * i + 2] + fz;
-        if (vpart) {
-            double ux = d.x[3 * i], uy = d.x[3 * i + 1], uz = d.x[3 * i + 2];
-            if (s.image) {
-                int ix, iy, iz;
-                unpack_image(s.image[i], ix, iy, iz);
-                ux += ix * g.L[0];
-                uy += iy * g.L[1];
-                uz += iz * g.L[2];
-            }
-            vir[0] = fx * ux; vir[1] = fy * uy; vir[2] = fz * uz;
-            vir[3] = fx * uy; vir[4] = fx * uz; vir[5] = fy * uz;
-        }
-    }
-    if (vpart) {
-        block_sum<6>(vir, smem);
-        if (threadIdx.x == 0)
-            for (int t = 0; t < 6; ++t) vpart[blockIdx.x * 8 + t] = vir[t];
+        vir[0] = gx * ux; vir[1] = gy * uy; vir[2] = gz * uz;
+        vir[3] = gx * uy; vir[4] = gx * uz; vir[5] = gy * uz;
     }
 }
 
-// Mixed-precision force pass: AT atoms per thread (atoms blockIdx.x * 256 *
-// AT + a * 256 + threadIdx.x), so each k's shared-memory loads serve AT
-// atoms; per k one 16-byte load of (k / pi).xy, one of (Re rho, Im rho, kx,
-// ky) in FP32 and two scalars.  Every atom sums its k terms in k order with
-// the same operations whatever U and AT, so the shapes give identical forces.
-template <int U, int AT>
-__global__ void __launch_bounds__(256) k_sk_force_mixed(SkDev d, const double *__restrict__ f_src,
-                                                        double *__restrict__ f_dst, SysDev s, CellGrid g,
-                                                        double *vpart) {
+// Force pass, AT atoms per thread and tile (atoms tile * 256 * AT + a * 256 +
+// threadIdx.x), tiles over a grid of resident blocks.  One sine per pair:
+// Im rho cos(k.x) - Re rho sin(k.x) = -|rho| sin(pi (u - u_rho)), with the
+// phase of rho(k) in half turns u_rho set off the phase sum's start and |rho|
+// multiplied into k, both formed once per block.  k-vectors go in pairs, with
+// the sums over the even and the odd k kept apart and added at the end, so the
+// forces do not depend on U, AT or the grid.
+// Bound by dispatch as the value pass (16 instructions a pair, 27 cycles).
+// 1,048,576 atoms x 96 k: 119 us before (sine and cosine, 3 more FP64
+// additions), 82 now; FP64 at 108,000 x 24: 16 us, 14 now.
+template <bool FP64, int U, int AT>
+__global__ void __launch_bounds__(256, FP64 ? 2 : 4)
+    k_sk_force(SkDev d, const double *__restrict__ f_src, double *__restrict__ f_dst, SysDev s, CellGrid g,
+               double *vpart) {
     pdl_entry();
     __shared__ double smem[6 * 32];
-    extern __shared__ double4 skf_raw[];   // K double2, K float4, K double, K float (44 K bytes)
-    double2 *kxy = reinterpret_cast<double2 *>(skf_raw);
-    float4 *rk = reinterpret_cast<float4 *>(kxy + d.K);
-    double *kz = reinterpret_cast<double *>(rk + d.K);
-    float *kzf = reinterpret_cast<float *>(kz + d.K);
-    for (int q = threadIdx.x; q < d.K; q += blockDim.x) {
-        kxy[q] = make_double2(d.k[3 * q] * kInvPi, d.k[3 * q + 1] * kInvPi);
-        kz[q] = d.k[3 * q + 2] * kInvPi;
-        rk[q] = make_float4((float)d.rho[2 * q], (float)d.rho[2 * q + 1], (float)d.k[3 * q], (float)d.k[3 * q + 1]);
-        kzf[q] = (float)d.k[3 * q + 2];
-    }
-    __syncthreads();
+    extern __shared__ double2 skf_raw[];   // per pair of k: 4 double2; 1 double2 (FP64) or 3 float2
+    const int np = (d.K + 1) / 2;
+    double2 *kp = skf_raw, *wd = kp + 4 * np;
+    float2 *wf = reinterpret_cast<float2 *>(wd);
     const double a = d.coef[0];
-    double x[AT], y[AT], z[AT];
-    float fx[AT], fy[AT], fz[AT];
-    bool on[AT];
-#pragma unroll
-    for (int t = 0; t < AT; ++t) {
-        const int i = (blockIdx.x * AT + t) * blockDim.x + threadIdx.x;
-        on[t] = i < d.nown && (!d.mask || (d.mask[i] & d.groupbit));
-        x[t] = on[t] ? d.x[3 * i] : 0.0;
-        y[t] = on[t] ? d.x[3 * i + 1] : 0.0;
-        z[t] = on[t] ? d.x[3 * i + 2] : 0.0;
-        fx[t] = fy[t] = fz[t] = 0.f;
+    for (int q = threadIdx.x; q < 2 * np; q += blockDim.x) {
+        const bool real = q < d.K;   // an odd K is filled up with a zero vector
+        const double re = real ? d.rho[2 * q] : 0.0, im = real ? d.rho[2 * q + 1] : 0.0;
+        const double amp = -sqrt(re * re + im * im), ph = atan2(im, re) * kInvPi;
+        double *kd = reinterpret_cast<double *>(kp) + q / 2 * 8 + q % 2;
+        for (int c = 0; c < 3; ++c) {
+            const double kc = real ? d.k[3 * q + c] : 0.0;
+            kd[2 * c] = kc * kInvPi;
+            if (!FP64) reinterpret_cast<float *>(wf)[q / 2 * 6 + 2 * c + q % 2] = (float)(amp * kc);
+        }
+        if (FP64) reinterpret_cast<double *>(wd)[q] = amp * kPi;   // on k / pi
+        kd[6] = FP64 ? -ph : kTurnBase - ph;
     }
-    bool any = false;
+    const double reach = FP64 ? 0.0 : kTurnMax / fmax(sk_kmax(d, smem), 1e-300);
+    __syncthreads();
+    for (int tile = blockIdx.x; tile * 256 * AT < d.n; tile += gridDim.x) {
+        using R2 = typename std::conditional<FP64, double2, float2>::type;
+        double x[AT], y[AT], z[AT];
+        R2 fx[AT], fy[AT], fz[AT];
+        bool on[AT], far[AT], any = false, any_far = false;
 #pragma unroll
-    for (int t = 0; t < AT; ++t) any = any || on[t];
-    if (any) {
+        for (int t = 0; t < AT; ++t) {
+            const int i = (tile * AT + t) * 256 + threadIdx.x;
+            on[t] = i < d.nown && (!d.mask || (d.mask[i] & d.groupbit));
+            x[t] = on[t] ? d.x[3 * i] : 0.0;
+            y[t] = on[t] ? d.x[3 * i + 1] : 0.0;
+            z[t] = on[t] ? d.x[3 * i + 2] : 0.0;
+            fx[t].x = fy[t].x = fz[t].x = fx[t].y = fy[t].y = fz[t].y = 0;
+            far[t] = !FP64 && !(fabs(x[t]) + fabs(y[t]) + fabs(z[t]) < reach);
+            any = any || on[t];
+            any_far = any_far || far[t];
+        }
+        auto add_pair = [&](int q, int t, bool is_far) {
+            const double2 kx = kp[4 * q], ky = kp[4 * q + 1], kz = kp[4 * q + 2], base = kp[4 * q + 3];
+            double ua = fma(kz.x, z[t], fma(ky.x, y[t], fma(kx.x, x[t], base.x)));
+            double ub = fma(kz.y, z[t], fma(ky.y, y[t], fma(kx.y, x[t], base.y)));
+            if constexpr (FP64) {
+                double sa, sb, c;
+                halfturn_sincos_f64<false>(ua, sa, c);
+                halfturn_sincos_f64<false>(ub, sb, c);
+                sa *= wd[q].x;
+                sb *= wd[q].y;
+                fx[t] = make_double2(fma(sa, kx.x, fx[t].x), fma(sb, kx.y, fx[t].y));
+                fy[t] = make_double2(fma(sa, ky.x, fy[t].x), fma(sb, ky.y, fy[t].y));
+                fz[t] = make_double2(fma(sa, kz.x, fz[t].x), fma(sb, kz.y, fz[t].y));
+            } else {
+                float2 s0, c0;
+                unsigned ga, gb;
+                if (!is_far) {
+                    turn_sin2(ua, ub, s0);
+                    ga = turn_sign(ua);
+                    gb = turn_sign(ub);
+                } else {
+                    // the phase without the base, its sum rounded as the phase is
+                    ua = fma(kz.x, z[t], fma(ky.x, y[t], kx.x * x[t])) + (base.x - kTurnBase);
+                    ub = fma(kz.y, z[t], fma(ky.y, y[t], kx.y * x[t])) + (base.y - kTurnBase);
+                    ga = halfturn_sincos_f32_parts(ua, s0.x, c0.x);
+                    gb = halfturn_sincos_f32_parts(ub, s0.y, c0.y);
+                }
+                // the sign (-1)^n on the sine: exact
+                s0.x = __uint_as_float(__float_as_uint(s0.x) ^ ga);
+                s0.y = __uint_as_float(__float_as_uint(s0.y) ^ gb);
+                fx[t] = __ffma2_rn(s0, wf[3 * q], fx[t]);
+                fy[t] = __ffma2_rn(s0, wf[3 * q + 1], fy[t]);
+                fz[t] = __ffma2_rn(s0, wf[3 * q + 2], fz[t]);
+            }
+        };
+        if (any && !any_far) {
 #pragma unroll U
-        for (int q = 0; q < d.K; ++q) {
-            const double2 kq = kxy[q];
-            const double kzq = kz[q];
-            const float4 r = rk[q];
-            const float kzq_f = kzf[q];
+            for (int q = 0; q < np; ++q)
 #pragma unroll
-            for (int t = 0; t < AT; ++t) {
-                const double u = kq.x * x[t] + kq.y * y[t] + kzq * z[t];
-                float s0, c0;
-                const unsigned sgn = halfturn_sincos_f32_parts(u, s0, c0);
-                // Im rho cos - Re rho sin, with the sign (-1)^n applied after
-                // (exact: rounding is symmetric in the sign)
-                const float w = __uint_as_float(__float_as_uint(fmaf(r.y, c0, -r.x * s0)) ^ sgn);
-                fx[t] = fmaf(w, r.z, fx[t]);
-                fy[t] = fmaf(w, r.w, fy[t]);
-                fz[t] = fmaf(w, kzq_f, fz[t]);
+                for (int t = 0; t < AT; ++t) add_pair(q, t, false);
+        } else if (any) {
+            for (int q = 0; q < np; ++q)
+#pragma unroll
+                for (int t = 0; t < AT; ++t) add_pair(q, t, far[t]);
+        }
+#pragma unroll
+        for (int t = 0; t < AT; ++t) {
+            const int vb = tile * AT + t, i = vb * 256 + threadIdx.x;
+            double vir[6] = {0, 0, 0, 0, 0, 0};
+            if (i < d.n)
+                sk_apply(d, s, g, i, on[t] ? -a * ((double)fx[t].x + (double)fx[t].y) : 0.0,
+                         on[t] ? -a * ((double)fy[t].x + (double)fy[t].y) : 0.0,
+                         on[t] ? -a * ((double)fz[t].x + (double)fz[t].y) : 0.0, f_src, f_dst, vpart != nullptr, vir);
+            // one virial partial per 256 atoms, as the other units write
+            if (vpart && vb * 256 < d.n) {
+                block_sum<6>(vir, smem);
+                if (threadIdx.x == 0)
+                    for (int c = 0; c < 6; ++c) vpart[vb * 8 + c] = vir[c];
+                __syncthreads();
             }
         }
-    }
-    double vir[6] = {0, 0, 0, 0, 0, 0};
-#pragma unroll
-    for (int t = 0; t < AT; ++t) {
-        const int i = (blockIdx.x * AT + t) * blockDim.x + threadIdx.x;
-        if (i >= d.n) continue;
-        const double gx = on[t] ? -a * (double)fx[t] : 0.0, gy = on[t] ? -a * (double)fy[t] : 0.0,
-                     gz = on[t] ? -a * (double)fz[t] : 0.0;
-        f_dst[3 * i] = f_src[3 * i] + gx;
-        f_dst[3 * i + 1] = f_src[3 * i + 1] + gy;
-        f_dst[3 * i + 2] = f_src[3 * i + 2] + gz;
-        if (vpart) {
-            double ux = d.x[3 * i], uy = d.x[3 * i + 1], uz = d.x[3 * i + 2];
-            if (s.image) {
-                int ix, iy, iz;
-                unpack_image(s.image[i], ix, iy, iz);
-                ux += ix * g.L[0];
-                uy += iy * g.L[1];
-                uz += iz * g.L[2];
-            }
-            vir[0] += gx * ux; vir[1] += gy * uy; vir[2] += gz * uz;
-            vir[3] += gx * uy; vir[4] += gx * uz; vir[5] += gy * uz;
-        }
-    }
-    if (vpart) {
-        block_sum<6>(vir, smem);
-        if (threadIdx.x == 0)
-            for (int t = 0; t < 6; ++t) vpart[blockIdx.x * 8 + t] = vir[t];
     }
 }
 
@@ -405,35 +502,36 @@ template void launch_debye_forces<float>(const DebyeDev<float> &, const double *
 template void launch_debye_forces<double>(const DebyeDev<double> &, const double *, double *, const SysDev &,
                                           const CellGrid &, double *, DevStatus *, cudaStream_t);
 
+// Blocks of the value pass: 64 atoms each give a small system the whole GPU.
 int sk_blocks(int n) {
-    int b = (n + 255) / 256;
+    const int b = (n + 63) / 64;
     return b < kSkBlocks ? (b < 1 ? 1 : b) : kSkBlocks;
 }
 
-template <int QV> static void launch_sk_partial_q(const SkDev &d, size_t sm, cudaStream_t st) {
-    if (d.fp64) launch_k(k_sk_partial<true, QV>, d.nblocks, 256, sm, st, d);
-    else launch_k(k_sk_partial<false, QV>, d.nblocks, 256, sm, st, d);
+template <int U> static void launch_sk_partial_u(const SkDev &d, cudaStream_t st) {
+    const int per = (d.nown + d.nblocks - 1) / d.nblocks;
+    if (d.fp64) launch_k(k_sk_partial<true, U>, d.nblocks, 256, 0, st, d, per);
+    else launch_k(k_sk_partial<false, U>, d.nblocks, 256, 0, st, d, per);
 }
 
 template <int U>
 static void launch_sk_force_u(const SkDev &d, const double *f_src, double *f_dst, const SysDev &s, const CellGrid &g,
                               double *vpart, size_t sm, int nb, cudaStream_t st) {
     if (d.fp64) {
-        launch_k(k_sk_force<U>, nb, 256, sm, st, d, f_src, f_dst, s, g, vpart);
-    } else if (vpart) {   // one atom per thread: one virial partial per 256 atoms, as the other units write
-        launch_k(k_sk_force_mixed<U, 1>, nb, 256, sm, st, d, f_src, f_dst, s, g, vpart);
+        launch_k(k_sk_force<true, U, 1>, std::min(nb, kSkBlocks / 2), 256, sm, st, d, f_src, f_dst, s, g, vpart);
+    } else if (nb <= kSkBlocks) {   // one atom a thread until the resident blocks are full
+        launch_k(k_sk_force<false, U, 1>, nb, 256, sm, st, d, f_src, f_dst, s, g, vpart);
     } else {
-        launch_k(k_sk_force_mixed<U, 2>, (d.n + 511) / 512, 256, sm, st, d, f_src, f_dst, s, g, vpart);
+        launch_k(k_sk_force<false, U, 2>, std::min((nb + 1) / 2, kSkBlocks), 256, sm, st, d, f_src, f_dst, s, g, vpart);
     }
 }
 
 void launch_sk_values(const SkDev &d, cudaStream_t st) {
-    const size_t sm = sizeof(double) * 3 * (size_t)d.K;
-    if (d.qv == 4) launch_sk_partial_q<4>(d, sm, st);
-    else if (d.qv == 16) launch_sk_partial_q<16>(d, sm, st);
-    else launch_sk_partial_q<8>(d, sm, st);
+    if (d.qv == 4) launch_sk_partial_u<2>(d, st);
+    else if (d.qv == 16) launch_sk_partial_u<8>(d, st);
+    else launch_sk_partial_u<4>(d, st);
     prof_mark("sk_partial", st);
-    launch_k(k_sk_reduce, 2 * d.K + 1, 256, 0, st, d);
+    launch_k(k_sk_reduce, (2 * d.K + 8) / 8, 256, 0, st, d);
     prof_mark("sk_reduce", st);
 }
 
@@ -441,7 +539,8 @@ void launch_sk_forces(const SkDev &d, const double *f_src, double *f_dst, const 
                       double *vpart, cudaStream_t st) {
     if (d.n == 0) return;
     const int nb = (d.n + 255) / 256;
-    const size_t sm = sizeof(double) * 3 * (size_t)d.K + (d.fp64 ? sizeof(double) * 2 : sizeof(float) * 5) * (size_t)d.K;
+    // per pair of k: 4 double2, then 1 double2 or 3 float2 (40,960 and 45,056 bytes at 1,024 k)
+    const size_t sm = (size_t)((d.K + 1) / 2) * (4 * sizeof(double2) + (d.fp64 ? sizeof(double2) : 3 * sizeof(float2)));
     if (d.qf == 1) launch_sk_force_u<1>(d, f_src, f_dst, s, g, vpart, sm, nb, st);
     else if (d.qf == 4) launch_sk_force_u<4>(d, f_src, f_dst, s, g, vpart, sm, nb, st);
     else launch_sk_force_u<2>(d, f_src, f_dst, s, g, vpart, sm, nb, st);

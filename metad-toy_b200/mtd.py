@@ -356,7 +356,7 @@ class Metad:
         self._check(lib().mtd_set_tuning_all(self._h, a))
 
     def sk_tiles(self):
-        """S(k) shapes: (k-vectors per value pass, unroll depth of the force pass)."""
+        """S(k) shapes: (phases in flight per thread of the value pass, unroll depth of the force pass)."""
         a, b = C.c_int(), C.c_int()
         self._check(lib().mtd_sk_tiles(self._h, C.byref(a), C.byref(b)))
         return a.value, b.value
