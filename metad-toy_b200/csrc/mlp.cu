@@ -7,8 +7,9 @@
 // Kernels
 //   hillsum_batch     exact FP64 V and dV/ds for a batch of points (hillsum.cu)
 //   k_hillsum_point   exact FP64 V and dV/ds at one point, hills spread over the grid
-//   k_mlp_tile        128 points per CTA: layer 1 and 3 on CUDA cores, the 128 x 128
-//                     layer and its two backward contractions on tcgen05 (TMEM accumulators)
+//   k_mlp_eval        V and dV/ds of 128-point tiles: layers 1 and 3 on CUDA cores, the
+//                     128 x 128 layer and its backward contraction on tcgen05 (TMEM accumulators)
+//   k_mlp_train       one 128-point tile's parameter gradients: three tcgen05 contractions
 //   k_mlp_adam        sums the per-tile gradients in tile order, Adam step, BF16 copies
 //   k_mlp_point       V_theta and dV_theta/ds at one point (CUDA cores, one block)
 //
@@ -45,10 +46,7 @@ constexpr int ow3 = ob2 + kH;
 constexpr int ob3 = ow3 + kH;
 constexpr int kNP = ob3 + 1;            // 17,281 parameters
 constexpr int kNPpad = (kNP + 3) / 4 * 4;
-constexpr int kTileSmem = 6 * 32768 + (4 * kH + 3 * kH) * 4 + 64;   // operand tiles + small weights
 constexpr int kWaitTries = 1 << 20;     // bounded mbarrier waits (default limit)
-
-enum { MODE_FWD = 0, MODE_GRAD_S = 1, MODE_TRAIN = 2 };
 
 struct MlpDev {
     int D;
@@ -56,261 +54,483 @@ struct MlpDev {
     const __nv_bfloat16 *W2, *W2t;             // [n][k] and [k][n]
 };
 
+// sigmoid(z): exp by the SFU and the reciprocal by the SFU with one Newton
+// step (1 + exp(-z) is capped so that the step stays finite; z * s is then
+// z * 1e-30 where it was z * 0).
+__device__ __forceinline__ float sigmoid(float z) {
+    const float a = fminf(1.0f + __expf(-z), 1e30f);
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a));
+    return fmaf(r, fmaf(-a, r, 1.0f), r);
+}
 __device__ __forceinline__ float silu(float z, float &dsilu) {
-    const float s = 1.0f / (1.0f + __expf(-z));
+    const float s = sigmoid(z);
     dsilu = s * (1.0f + z * (1.0f - s));
     return z * s;
 }
 
-// Sum over the 128 rows of a CTA of Q per-row values, Q <= 96: rows write a
-// [128][Q+1] FP32 tile, then thread q sums column q in row order.
-__device__ __forceinline__ void rows_sum(float *scratch, const float *vals, int Q, float *out) {
-    const int m = threadIdx.x;
-    for (int q = 0; q < Q; ++q) scratch[m * (Q + 1) + q] = vals[q];
-    __syncthreads();
-    if (m < Q) {
-        float s = 0.0f;
-        for (int r = 0; r < kH; ++r) s += scratch[r * (Q + 1) + m];
-        out[m] = s;
-    }
-    __syncthreads();
+// Barrier `id` of 128 threads; the second form also votes.
+__device__ __forceinline__ void wg_sync(int id) {
+    asm volatile("barrier.cta.sync %0, 128;" ::"r"(id) : "memory");
+    __syncwarp();
+}
+__device__ __forceinline__ bool wg_all(int id, bool v) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %2, 0;\n\t"
+        "barrier.cta.red.and.pred q, %1, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}\n"
+        : "=r"(r)
+        : "r"(id), "r"((uint32_t)v)
+        : "memory");
+    __syncwarp();
+    return r != 0;
 }
 
-// A bounded wait that runs out (in any thread: the block votes) ends the
-// tile: it issues no further MMA, reads no TMEM and overlays no operand the
-// tensor core may still be reading; it waits once more (same limit) for the
-// batch in flight, releases its TMEM, sets *err and returns.  stall != 0 is
-// the check of that path: after the first batch has completed, every thread
-// waits on the barrier's next phase, which no commit will complete.
-template <int MODE>
-__global__ void __launch_bounds__(128, 1)
-    k_mlp_tile(MlpDev p, int npts, const float *__restrict__ x, const float *__restrict__ t, float *y_out,
-               float *ds_out, float *part, float *loss_part, float grad_scale, int *err, int tries, int stall) {
-    extern __shared__ __align__(1024) unsigned char sm[];
-    unsigned char *sA = sm;                   // h1        rows m, K k
-    unsigned char *sBf = sm + 32768;          // W2        rows n, K k
-    unsigned char *sBt = sm + 2 * 32768;      // W2^T      rows k, K n
-    unsigned char *sG = sm + 3 * 32768;       // dL/dz2    rows m, K n
-    unsigned char *sGt = sm + 4 * 32768;      // dL/dz2^T  rows n, K m
-    unsigned char *sHt = sm + 5 * 32768;      // h1^T      rows k, K m
-    float *sW1 = reinterpret_cast<float *>(sm + 6 * 32768);
-    float *sb1 = sW1 + 4 * kH, *sb2 = sb1 + kH, *sw3 = sb2 + kH;
-    float *scratch = reinterpret_cast<float *>(sm);   // reused once the operands are consumed
-    __shared__ uint64_t mbar;
-    __shared__ uint32_t tbase;
-    __shared__ float cols[96];
-    const int m = threadIdx.x, warp = m >> 5;
-    const int row = blockIdx.x * kH + m;
-    const bool valid = row < npts;
+// Where a batch's points come from and its results go: network units (x, y,
+// ds: rows of kIn floats) or the caller's doubles (pts, V, dV: rows of D),
+// normalised and scaled here.
+struct MlpIo {
+    const float *x;
+    float *y, *ds;
+    const double *pts;
+    double *V, *dV;
+    double lo[kIn], sc[kIn], vscale;
+};
 
-    if (m == 0) mbar_init(&mbar, 1);
-    if (warp == 0) tmem_alloc(&tbase, 512);
-    tc_fence_before();
-    // weights: W2 and W2^T rows as 16-byte vectors into the operand layout
-    {
-        const uint4 *w2 = reinterpret_cast<const uint4 *>(p.W2 + (size_t)m * kH);
-        const uint4 *w2t = reinterpret_cast<const uint4 *>(p.W2t + (size_t)m * kH);
-#pragma unroll 4
-        for (int c = 0; c < kH / 8; ++c) {
-            *reinterpret_cast<uint4 *>(sBf + umma_off(m, 8 * c, kH)) = w2[c];
-            *reinterpret_cast<uint4 *>(sBt + umma_off(m, 8 * c, kH)) = w2t[c];
-        }
-        for (int i = 0; i < kIn; ++i) sW1[m * kIn + i] = p.W1[m * kIn + i];
-        sb1[m] = p.b1[m];
-        sb2[m] = p.b2[m];
-        sw3[m] = p.w3[m];
+__device__ __forceinline__ void mlp_input(const MlpIo &io, int D, int row, bool valid, float (&u)[kIn]) {
+#pragma unroll
+    for (int i = 0; i < kIn; ++i) {
+        u[i] = 0.f;
+        if (valid && i < D)
+            u[i] = io.pts ? (float)(io.sc[i] * (io.pts[(size_t)row * D + i] - io.lo[i]) - 1.0)
+                          : io.x[(size_t)row * kIn + i];
     }
-    __syncthreads();
-    float u[kIn] = {0.f, 0.f, 0.f, 0.f};
-    if (valid)
-        for (int i = 0; i < p.D; ++i) u[i] = x[(size_t)row * kIn + i];
-    // layer 1 -> h1 (BF16) in the A layout, and h1^T for the weight gradient
-    for (int c = 0; c < kH / 8; ++c) {
+}
+
+// Shared memory of both tile kernels: W2, W2^T (32 KB each, operand layout),
+// the small weights (W1 as float4 rows, b1, b2, w3), then the kernel's own.
+constexpr int kSmW = 2 * 32768, kSmSmall = (4 + 3) * kH * 4;
+
+__device__ __forceinline__ void load_weights(const MlpDev &p, unsigned char *sm, bool back) {
+    // 16-byte vectors, eight rows by four K chunks a warp: 64 contiguous bytes
+    // of each row, and eight lanes fill one 128-byte core matrix (a row's chunks
+    // side by side in a warp hit one bank group)
+#pragma unroll 4
+    for (int e = threadIdx.x; e < kH * kH / 8; e += blockDim.x) {
+        const int r = (e >> 7) * 8 + (e & 7), c = (e >> 3) & 15;
+        const uint4 v = reinterpret_cast<const uint4 *>(p.W2)[r * (kH / 8) + c];
+        const uint4 vt = back ? reinterpret_cast<const uint4 *>(p.W2t)[r * (kH / 8) + c] : v;
+        *reinterpret_cast<uint4 *>(sm + umma_off(r, 8 * c, kH)) = v;
+        if (back) *reinterpret_cast<uint4 *>(sm + 32768 + umma_off(r, 8 * c, kH)) = vt;
+    }
+    float *w = reinterpret_cast<float *>(sm + kSmW);
+    for (int e = threadIdx.x; e < kH * kIn; e += blockDim.x) w[e] = p.W1[e];
+    for (int e = threadIdx.x; e < kH; e += blockDim.x) {
+        w[4 * kH + e] = p.b1[e];
+        w[5 * kH + e] = p.b2[e];
+        w[6 * kH + e] = p.w3[e];
+    }
+}
+
+__device__ __forceinline__ float layer1(const float4 *sW1, const float *sb1, int j, const float (&u)[kIn]) {
+    const float4 w = sW1[j];
+    return fmaf(w.w, u[3], fmaf(w.z, u[2], fmaf(w.y, u[1], fmaf(w.x, u[0], sb1[j]))));
+}
+
+// Columns [c0, c0 + n) of h1 = silu(z1) of this thread's row, in BF16, into the
+// A operand.
+__device__ __forceinline__ void write_h1(const float4 *sW1, const float *sb1, const float (&u)[kIn], int m, int c0,
+                                         int n, unsigned char *sA) {
+#pragma unroll 2
+    for (int c = c0; c < c0 + n; c += 8) {
         __align__(16) __nv_bfloat16 hb[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            const int j = 8 * c + e;
-            float z = sb1[j];
-#pragma unroll
-            for (int i = 0; i < kIn; ++i) z = fmaf(sW1[j * kIn + i], u[i], z);
-            float ds;
-            hb[e] = __float2bfloat16_rn(silu(z, ds));
-            if (MODE == MODE_TRAIN) *reinterpret_cast<__nv_bfloat16 *>(sHt + umma_off(j, m, kH)) = hb[e];
+            const float z = layer1(sW1, sb1, c + e, u);
+            hb[e] = __float2bfloat16_rn(z * sigmoid(z));
         }
-        *reinterpret_cast<uint4 *>(sA + umma_off(m, 8 * c, kH)) = *reinterpret_cast<const uint4 *>(hb);
+        *reinterpret_cast<uint4 *>(sA + umma_off(m, c, kH)) = *reinterpret_cast<const uint4 *>(hb);
     }
+}
+
+// D[128 x 128] = A B^T over K = 128, both K-major, issued by one thread.
+__device__ __forceinline__ void mma_tile(uint32_t d, const unsigned char *sA, const unsigned char *sB) {
+#pragma unroll
+    for (int kk = 0; kk < kH / 16; ++kk)
+        umma_bf16(d, umma_desc(smem_addr(sA) + kk * 2 * kH * 16, kH * 16, 128),
+                  umma_desc(smem_addr(sB) + kk * 2 * kH * 16, kH * 16, 128), umma_idesc_bf16(kH, kH), kk > 0 ? 1u : 0u);
+}
+
+// Forward pass (GRAD: and input gradient) of 128 points per tile.  Each of the
+// block's four warpgroups has its own A operand (32 KB) and 128 columns of
+// tensor memory, so that one's SiLU work runs beside another's MMA; the block
+// stays for all its tiles and loads the weights once.  CS = 1: a tile per
+// warpgroup.  CS = 4: a tile per block, each warpgroup taking 32 of the 128
+// columns of every layer (batches too small to give every warpgroup a tile).
+// Bound by the SFU and FP32 work of three SiLU evaluations per hidden unit and
+// point (the MMAs are under 5 % of it): 5.7 us per tile and SM, of which the
+// SFU's two calls a SiLU take 3.1.  V and dV/ds at 65,536 points: 198 us before
+// (one warpgroup and one tile a block, four SiLU evaluations, inputs and
+// outputs converted by kernels of their own), 31 now; up to 148 tiles 14.
+//
+// A bounded wait that runs out (in any thread: the warpgroup votes) ends the
+// warpgroup's work: it issues no further MMA, reads no TMEM and overwrites no
+// operand the tensor core may still be reading; it waits once more (same
+// limit) for the batch in flight, sets *err and meets the others at the end,
+// where the block's TMEM is released.  stall != 0 is the check of that path:
+// after its first batch has completed, every warpgroup waits on the barrier's
+// next phase, which no commit will complete.
+template <bool GRAD, int CS>
+__global__ void __launch_bounds__(512, 1)
+    k_mlp_eval(MlpDev p, int npts, MlpIo io, int *err, int tries, int stall) {
+    extern __shared__ __align__(1024) unsigned char sm[];
+    __shared__ uint64_t mbar[4];
+    __shared__ uint32_t tbase;
+    const float4 *sW1 = reinterpret_cast<const float4 *>(sm + kSmW);
+    const float *sb1 = reinterpret_cast<const float *>(sm + kSmW) + 4 * kH, *sb2 = sb1 + kH, *sw3 = sb2 + kH;
+    const int wg = threadIdx.x >> 7, m = threadIdx.x & 127, warp = threadIdx.x >> 5;
+    constexpr int NC = kH / CS;                         // columns of a thread
+    const int c0 = CS > 1 ? NC * wg : 0, who = CS > 1 ? 0 : wg;
+    unsigned char *sA = sm + kSmW + kSmSmall + who * 32768;
+    float *red = reinterpret_cast<float *>(sm + kSmW + kSmSmall + 32768);   // CS > 1: [4][1 + kIn][128]
+    if (threadIdx.x < 4) mbar_init(&mbar[threadIdx.x], 1);
+    if (warp == 0) tmem_alloc(&tbase, 512);
+    load_weights(p, sm, GRAD);
+    tc_fence_before();
     fence_async_smem();
     __syncthreads();
     tc_fence_after();
-    const uint32_t taddr = tbase;
-    const uint32_t idesc = umma_idesc_bf16(kH, kH);
-    if (m == 0) {
-        for (int kk = 0; kk < kH / 16; ++kk) {
-            const uint64_t a = umma_desc(smem_addr(sA) + kk * 2 * kH * 16, kH * 16, 128);
-            const uint64_t b = umma_desc(smem_addr(sBf) + kk * 2 * kH * 16, kH * 16, 128);
-            umma_bf16(taddr, a, b, idesc, kk > 0 ? 1u : 0u);
-        }
-        umma_commit(&mbar);
-    }
-    bool ok = mbar_wait(&mbar, 0, tries);
-    if (stall) ok = mbar_wait(&mbar, 1, tries) && ok;
-    if (!__syncthreads_and(ok)) {
-        mbar_wait(&mbar, 0, tries);
+    const uint32_t taddr = tbase + who * kH, lane_addr = taddr + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    const int ntiles = (npts + kH - 1) / kH;
+    uint32_t phase = 0;
+    bool alive = true;
+    auto sync = [&] {
+        if (CS > 1) __syncthreads();
+        else wg_sync(1 + wg);
+    };
+    auto vote = [&](bool v) { return CS > 1 ? __syncthreads_and(v) != 0 : wg_all(1 + wg, v); };
+    // operand written by this warpgroup -> one thread issues -> every thread waits
+    auto run_mma = [&](const unsigned char *sB) {
         tc_fence_before();
-        __syncthreads();
-        if (warp == 0) tmem_dealloc(taddr, 512);
-        if (m == 0) atomicExch(err, 1);
-        return;
-    }
-    tc_fence_after();
-    const uint32_t lane_addr = taddr + (static_cast<uint32_t>(warp * 32) << 16);
-    // forward epilogue: z2 = D + b2, y = w3 . silu(z2) + b3
-    float y = p.b3[0];
-    for (int c = 0; c < kH / 16; ++c) {
-        float z[16];
-        tmem_ld16(lane_addr + 16 * c, z);
+        fence_async_smem();
+        sync();
+        tc_fence_after();
+        if (CS > 1 ? threadIdx.x == 0 : m == 0) {
+            mma_tile(taddr, sA, sB);
+            umma_commit(&mbar[who]);
+        }
+        bool ok = mbar_wait(&mbar[who], phase, tries);
+        if (stall) ok = mbar_wait(&mbar[who], phase ^ 1, tries) && ok;
+        ok = vote(ok);
+        if (!ok) mbar_wait(&mbar[who], phase, tries);
+        tc_fence_after();
+        phase ^= 1;
+        return ok;
+    };
+    for (int tile = CS > 1 ? blockIdx.x : wg * gridDim.x + blockIdx.x; tile < ntiles;
+         tile += CS > 1 ? gridDim.x : 4 * gridDim.x) {
+        const int row = tile * kH + m;
+        const bool valid = row < npts;
+        float u[kIn];
+        mlp_input(io, p.D, row, valid, u);
+        write_h1(sW1, sb1, u, m, c0, NC, sA);
+        if (!(alive = run_mma(sm))) break;
+        // z2 = D + b2, y = w3 . silu(z2) + b3, dy/dz2 in BF16 over the consumed h1
+        float y = CS > 1 && wg ? 0.f : p.b3[0];
+#pragma unroll 1
+        for (int c = c0; c < c0 + NC; c += 16) {
+            float z[16];
+            tmem_ld16(lane_addr + c, z);
+            __align__(16) __nv_bfloat16 gb[16];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-            float ds;
-            y = fmaf(sw3[16 * c + e], silu(z[e] + sb2[16 * c + e], ds), y);
+            for (int e = 0; e < 16; ++e) {
+                float dsl;
+                y = fmaf(sw3[c + e], silu(z[e] + sb2[c + e], dsl), y);
+                if (GRAD) gb[e] = __float2bfloat16_rn(sw3[c + e] * dsl);
+            }
+            if (GRAD) {
+                *reinterpret_cast<uint4 *>(sA + umma_off(m, c, kH)) = reinterpret_cast<const uint4 *>(gb)[0];
+                *reinterpret_cast<uint4 *>(sA + umma_off(m, c + 8, kH)) = reinterpret_cast<const uint4 *>(gb)[1];
+            }
         }
-    }
-    if (valid && y_out) y_out[row] = y;
-    if (MODE == MODE_FWD) {
-        tc_fence_before();
-        __syncthreads();
-        if (warp == 0) tmem_dealloc(taddr, 512);
-        return;
-    }
-    float dy = 0.0f;
-    if (valid) dy = (MODE == MODE_TRAIN) ? grad_scale * (y - t[row]) : 1.0f;
-    if (MODE == MODE_TRAIN) {
-        float l = valid ? (y - t[row]) * (y - t[row]) : 0.0f;
-        for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-        if ((m & 31) == 0) cols[warp] = l;
-        __syncthreads();
-        if (m == 0) loss_part[blockIdx.x] = cols[0] + cols[1] + cols[2] + cols[3];
-        __syncthreads();
-    }
-    // dL/dz2 = dy w3 silu'(z2): BF16 into the A layout (and its transpose);
-    // b2, w3 gradients summed over rows in FP32
-    for (int c = 0; c < kH / 16; ++c) {
-        float z[16];
-        tmem_ld16(lane_addr + 16 * c, z);
-        __align__(16) __nv_bfloat16 gb[16];
-        float red[32];
+        float du[kIn] = {0.f, 0.f, 0.f, 0.f};
+        if (GRAD) {
+            if (!(alive = run_mma(sm + 32768))) break;   // dy/dh1 = dy/dz2 W2
+#pragma unroll 1
+            for (int c = c0; c < c0 + NC; c += 16) {
+                float dh[16];
+                tmem_ld16(lane_addr + c, dh);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-            const int n = 16 * c + e;
-            float dsl;
-            const float h2 = silu(z[e] + sb2[n], dsl);
-            const float g = dy * sw3[n] * dsl;
-            gb[e] = __float2bfloat16_rn(g);
-            red[e] = g;
-            red[16 + e] = dy * h2;
-            if (MODE == MODE_TRAIN) *reinterpret_cast<__nv_bfloat16 *>(sGt + umma_off(n, m, kH)) = gb[e];
+                for (int e = 0; e < 16; ++e) {
+                    const float4 w = sW1[c + e];
+                    float dsl;
+                    silu(layer1(sW1, sb1, c + e, u), dsl);
+                    const float g = dh[e] * dsl;
+                    du[0] = fmaf(g, w.x, du[0]);
+                    du[1] = fmaf(g, w.y, du[1]);
+                    du[2] = fmaf(g, w.z, du[2]);
+                    du[3] = fmaf(g, w.w, du[3]);
+                }
+            }
         }
-        *reinterpret_cast<uint4 *>(sG + umma_off(m, 16 * c, kH)) = *reinterpret_cast<const uint4 *>(gb);
-        *reinterpret_cast<uint4 *>(sG + umma_off(m, 16 * c + 8, kH)) = *reinterpret_cast<const uint4 *>(gb + 8);
-        if (MODE == MODE_TRAIN) {
-            // scratch overlays sA / sBf, free since the forward MMA completed
-            rows_sum(scratch, red, 32, cols);
-            if (m < 16) part[(size_t)blockIdx.x * kNPpad + ob2 + 16 * c + m] = cols[m];
-            else if (m < 32) part[(size_t)blockIdx.x * kNPpad + ow3 + 16 * c + (m - 16)] = cols[m];
+        if (CS > 1) {   // the column groups' sums, in their order
+            red[(wg * (1 + kIn)) * kH + m] = y;
+            for (int i = 0; i < kIn; ++i) red[(wg * (1 + kIn) + 1 + i) * kH + m] = du[i];
+            __syncthreads();
+            if (wg == 0)
+                for (int q = 1; q < 4; ++q) {
+                    y += red[q * (1 + kIn) * kH + m];
+                    for (int i = 0; i < kIn; ++i) du[i] += red[(q * (1 + kIn) + 1 + i) * kH + m];
+                }
+        }
+        if (valid && (CS == 1 || wg == 0)) {
+            if (io.pts) {
+                io.V[row] = io.vscale * (double)y;
+                if (GRAD)
+#pragma unroll
+                    for (int i = 0; i < kIn; ++i)
+                        if (i < p.D) io.dV[(size_t)row * p.D + i] = io.vscale * (double)du[i] * io.sc[i];
+            } else {
+                io.y[row] = y;
+                if (GRAD) *reinterpret_cast<float4 *>(io.ds + (size_t)row * kIn) = make_float4(du[0], du[1], du[2], du[3]);
+            }
         }
     }
-    if (MODE == MODE_TRAIN) {
-        float v[1] = {dy};
-        rows_sum(scratch, v, 1, cols);
-        if (m == 0) part[(size_t)blockIdx.x * kNPpad + ob3] = cols[0];
+    if (!alive && m == 0) atomicExch(err, 1);
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tbase, 512);
+}
+
+// Sums over the 32 lanes of N values a lane (N a power of two up to 32): lanes
+// 16, 8, ... apart swap halves of their values, so lane l ends with the sum of
+// value l * N / 32.
+template <int N> __device__ __forceinline__ float lanes_sum(float (&v)[N], int lane) {
+    constexpr int P = N == 32 ? 5 : N == 16 ? 4 : 3;
+    static_assert(N == 1 << P, "N: 8, 16 or 32");
+#pragma unroll
+    for (int st = 0; st < P; ++st) {
+        const int o = 16 >> st, h = (N >> st) / 2;
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int j = 0; j < h; ++j) {
+            const float send = up ? v[j] : v[j + h], keep = up ? v[j + h] : v[j];
+            v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
     }
+    float r = v[0];
+#pragma unroll
+    for (int st = P; st < 5; ++st) r += __shfl_xor_sync(0xffffffffu, r, 16 >> st);
+    return r;
+}
+
+// One 128-point training tile per block: loss and the parameter gradients of
+// sum (y - t)^2 scaled by grad_scale, as one row of `part`.  Four warpgroups
+// take 32 columns each of every layer.  The three MMAs share two operands: h1
+// and dL/dz2, rows of points; dL/dW2 = dL/dz2^T h1 reads both transposed
+// (M-major descriptors), so no transposed copies are written (two-byte stores
+// down a column cost a bank conflict each).  Sums over a tile's points go
+// through warp butterflies (lanes_sum) and the four warps' rows in order.
+// 8,192 points (64 tiles): 72 us before (128 threads a tile; row sums through a
+// [128][97] scratch tile), 20 now; latency of one tile's serial phases.
+// Timeouts as in k_mlp_eval, the whole block together.
+constexpr int kEvalSmem = kSmW + kSmSmall + 4 * 32768;
+constexpr int kTrainRed = 7 * 4 * kH;   // [value][row warp][column]: b2, w3, b1, W1 x 4
+constexpr int kTrainSmem = kSmW + kSmSmall + 2 * 32768 + kTrainRed * 4;
+__global__ void __launch_bounds__(512, 1)
+    k_mlp_train(MlpDev p, int npts, const float *__restrict__ x, const float *__restrict__ t, float *part,
+                float *loss_part, float grad_scale, int *err, int tries, int stall) {
+    extern __shared__ __align__(1024) unsigned char sm[];
+    __shared__ uint64_t mbar;
+    __shared__ uint32_t tbase;
+    __shared__ float srow[2][4][kH], sdy[kH], sl[4], sb3[4];
+    const float4 *sW1 = reinterpret_cast<const float4 *>(sm + kSmW);
+    const float *sb1 = reinterpret_cast<const float *>(sm + kSmW) + 4 * kH, *sb2 = sb1 + kH, *sw3 = sb2 + kH;
+    unsigned char *sH = sm + kSmW + kSmSmall, *sG = sH + 32768;
+    float *red = reinterpret_cast<float *>(sG + 32768);
+    const int wg = threadIdx.x >> 7, m = threadIdx.x & 127, warp = threadIdx.x >> 5, rw = warp & 3;
+    const int lane = threadIdx.x & 31, c0 = 32 * wg, row = blockIdx.x * kH + m;
+    const bool valid = row < npts;
+    if (threadIdx.x == 0) mbar_init(&mbar, 1);
+    if (warp == 0) tmem_alloc(&tbase, 512);
+    load_weights(p, sm, true);
+    float u[kIn] = {0.f, 0.f, 0.f, 0.f};
+    if (valid) {
+        const float4 v = *reinterpret_cast<const float4 *>(x + (size_t)row * kIn);
+        u[0] = v.x;
+        u[1] = v.y;
+        u[2] = v.z;
+        u[3] = v.w;
+    }
+    __syncthreads();
+    write_h1(sW1, sb1, u, m, c0, 32, sH);
+    uint32_t phase = 0;
+    auto wait = [&] {
+        bool ok = mbar_wait(&mbar, phase, tries);
+        if (stall) ok = mbar_wait(&mbar, phase ^ 1, tries) && ok;
+        ok = __syncthreads_and(ok) != 0;
+        if (!ok) mbar_wait(&mbar, phase, tries);
+        tc_fence_after();
+        phase ^= 1;
+        return ok;
+    };
+    tc_fence_before();
     fence_async_smem();
     __syncthreads();
     tc_fence_after();
-    if (m == 0) {
-        for (int kk = 0; kk < kH / 16; ++kk) {   // dL/dh1 = dL/dz2 . W2  -> columns 128..255
-            const uint64_t a = umma_desc(smem_addr(sG) + kk * 2 * kH * 16, kH * 16, 128);
-            const uint64_t b = umma_desc(smem_addr(sBt) + kk * 2 * kH * 16, kH * 16, 128);
-            umma_bf16(taddr + kH, a, b, idesc, kk > 0 ? 1u : 0u);
-        }
-        if (MODE == MODE_TRAIN) {
-            for (int kk = 0; kk < kH / 16; ++kk) {   // dL/dW2 = dL/dz2^T . h1  -> columns 256..383
-                const uint64_t a = umma_desc(smem_addr(sGt) + kk * 2 * kH * 16, kH * 16, 128);
-                const uint64_t b = umma_desc(smem_addr(sHt) + kk * 2 * kH * 16, kH * 16, 128);
-                umma_bf16(taddr + 2 * kH, a, b, idesc, kk > 0 ? 1u : 0u);
-            }
-        }
+    const uint32_t taddr = tbase, lane_addr = taddr + (static_cast<uint32_t>(rw * 32) << 16);
+    if (threadIdx.x == 0) {
+        mma_tile(taddr, sH, sm);
         umma_commit(&mbar);
     }
-    if (!__syncthreads_and(mbar_wait(&mbar, 1, tries))) {
-        mbar_wait(&mbar, 1, tries);
-        tc_fence_before();
+    bool ok = wait();
+    if (ok) {
+        // forward: this column group's part of y; w3 silu'(z2) and silu(z2) wait for dy
+        float wd[32], h2[32];
+        float y = wg ? 0.f : p.b3[0];
+#pragma unroll
+        for (int c = 0; c < 32; c += 16) {
+            float z[16];
+            tmem_ld16(lane_addr + c0 + c, z);
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+                const int n = c0 + c + e;
+                float dsl;
+                h2[c + e] = silu(z[e] + sb2[n], dsl);
+                y = fmaf(sw3[n], h2[c + e], y);
+                wd[c + e] = dsl;
+            }
+        }
+        srow[0][wg][m] = y;
         __syncthreads();
-        if (warp == 0) tmem_dealloc(taddr, 512);
-        if (m == 0) atomicExch(err, 1);
-        return;
-    }
-    tc_fence_after();
-    // layer 1 backward: dL/dz1 = dL/dh1 silu'(z1); input gradient and W1, b1 gradients
-    float dsu[kIn] = {0.f, 0.f, 0.f, 0.f};
-    for (int c = 0; c < kH / 16; ++c) {
-        float dh[16];
-        tmem_ld16(lane_addr + kH + 16 * c, dh);
-        float red[80];
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-            const int j = 16 * c + e;
-            float z = sb1[j];
-#pragma unroll
-            for (int i = 0; i < kIn; ++i) z = fmaf(sW1[j * kIn + i], u[i], z);
-            float dsl;
-            silu(z, dsl);
-            const float g = dh[e] * dsl;
-#pragma unroll
-            for (int i = 0; i < kIn; ++i) {
-                dsu[i] = fmaf(g, sW1[j * kIn + i], dsu[i]);
-                red[16 + 16 * i + e] = g * u[i];
+        if (wg == 0) {
+            y = srow[0][0][m] + srow[0][1][m] + srow[0][2][m] + srow[0][3][m];
+            const float d = valid ? y - t[row] : 0.0f;
+            sdy[m] = grad_scale * d;
+            float l = d * d, g = grad_scale * d;
+            for (int o = 16; o > 0; o >>= 1) {
+                l += __shfl_xor_sync(0xffffffffu, l, o);
+                g += __shfl_xor_sync(0xffffffffu, g, o);
             }
-            red[e] = g;
-        }
-        if (MODE == MODE_TRAIN) {
-            rows_sum(scratch, red, 80, cols);
-            if (m < 16) part[(size_t)blockIdx.x * kNPpad + ob1 + 16 * c + m] = cols[m];
-            else if (m < 80) {
-                const int i = (m - 16) >> 4, e = (m - 16) & 15;
-                part[(size_t)blockIdx.x * kNPpad + oW1 + (16 * c + e) * kIn + i] = cols[m];
+            if (lane == 0) {
+                sl[rw] = l;
+                sb3[rw] = g;
             }
         }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            loss_part[blockIdx.x] = sl[0] + sl[1] + sl[2] + sl[3];
+            part[(size_t)blockIdx.x * kNPpad + ob3] = sb3[0] + sb3[1] + sb3[2] + sb3[3];
+        }
+        const float dy = sdy[m];
+        // dL/dz2 = dy w3 silu'(z2) in BF16; b2 and w3 gradients summed in FP32
+#pragma unroll
+        for (int e = 0; e < 32; ++e) {
+            wd[e] = dy * sw3[c0 + e] * wd[e];
+            h2[e] = dy * h2[e];
+        }
+#pragma unroll
+        for (int c = 0; c < 32; c += 8) {
+            __align__(16) __nv_bfloat16 gb[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) gb[e] = __float2bfloat16_rn(wd[c + e]);
+            *reinterpret_cast<uint4 *>(sG + umma_off(m, c0 + c, kH)) = *reinterpret_cast<const uint4 *>(gb);
+        }
+        red[(0 * 4 + rw) * kH + c0 + lane] = lanes_sum<32>(wd, lane);
+        red[(1 * 4 + rw) * kH + c0 + lane] = lanes_sum<32>(h2, lane);
+        tc_fence_before();
+        fence_async_smem();
+        __syncthreads();
+        tc_fence_after();
+        if (threadIdx.x == 0) {
+            mma_tile(taddr + kH, sG, sm + 32768);   // dL/dh1 = dL/dz2 W2
+#pragma unroll
+            for (int kk = 0; kk < kH / 16; ++kk)    // dL/dW2 = dL/dz2^T h1, K = the tile's points
+                umma_bf16(taddr + 2 * kH, umma_desc(smem_addr(sG) + kk * 256, 128, kH * 16),
+                          umma_desc(smem_addr(sH) + kk * 256, 128, kH * 16),
+                          umma_idesc_bf16(kH, kH) | kIdescTransA | kIdescTransB, kk > 0 ? 1u : 0u);
+            umma_commit(&mbar);
+        }
+        ok = wait();
     }
-    if (MODE == MODE_GRAD_S && valid && ds_out)
-        for (int i = 0; i < kIn; ++i) ds_out[(size_t)row * kIn + i] = dsu[i];
-    if (MODE == MODE_TRAIN) {   // row n of the W2 gradient
-        float *dst = part + (size_t)blockIdx.x * kNPpad + oW2 + (size_t)m * kH;
-        for (int c = 0; c < kH / 16; ++c) {
+    if (ok) {
+        // layer 1: dL/dz1 = dL/dh1 silu'(z1), eight columns at a time
+#pragma unroll 1
+        for (int c = c0; c < c0 + 32; c += 8) {
+            float dh[8], g[8], q[8];
+            tmem_ld8(lane_addr + kH + c, dh);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                float dsl;
+                silu(layer1(sW1, sb1, c + e, u), dsl);
+                g[e] = dh[e] * dsl;
+            }
+#pragma unroll
+            for (int v = 0; v < 1 + kIn; ++v) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) q[e] = v ? g[e] * u[v ? v - 1 : 0] : g[e];
+                const float sum = lanes_sum<8>(q, lane);
+                if ((lane & 3) == 0) red[((2 + v) * 4 + rw) * kH + c + (lane >> 2)] = sum;
+            }
+        }
+        // rows of the W2 gradient: this thread's row n = m, 32 columns
+        float *dst = part + (size_t)blockIdx.x * kNPpad + oW2 + (size_t)m * kH + c0;
+#pragma unroll
+        for (int c = 0; c < 32; c += 16) {
             float g[16];
-            tmem_ld16(lane_addr + 2 * kH + 16 * c, g);
+            tmem_ld16(lane_addr + 2 * kH + c0 + c, g);
 #pragma unroll
-            for (int e = 0; e < 16; ++e) dst[16 * c + e] = g[e];
+            for (int e = 0; e < 16; e += 4)
+                *reinterpret_cast<float4 *>(dst + c + e) = make_float4(g[e], g[e + 1], g[e + 2], g[e + 3]);
         }
+        __syncthreads();
+        for (int e = threadIdx.x; e < 7 * kH; e += blockDim.x) {
+            const int v = e / kH, n = e % kH;
+            const float *r = red + (size_t)v * 4 * kH + n;
+            const float s = r[0] + r[kH] + r[2 * kH] + r[3 * kH];
+            const int at = v == 0 ? ob2 + n : v == 1 ? ow3 + n : v == 2 ? ob1 + n : oW1 + n * kIn + (v - 3);
+            part[(size_t)blockIdx.x * kNPpad + at] = s;
+        }
+    } else if (threadIdx.x == 0) {
+        atomicExch(err, 1);
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(taddr, 512);
+    if (warp == 0) tmem_dealloc(tbase, 512);
 }
 
 __device__ __forceinline__ float bf16_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
-// Adam on the FP32 masters with the gradient summed over tiles in tile order;
-// refreshes the forward copies (BF16 W1, W2, W2^T, w3; FP32 biases).
+// Parameter q of a block of 256: 64 parameters by 4 groups of tiles (tiles g,
+// g + 4, ...), whose sums are added in order; true on the thread that goes on.
+constexpr int kSumQ = 64, kSumBlocks = (kNP + kSumQ - 1) / kSumQ;
+__device__ __forceinline__ bool tile_sum(int ntiles, const float *__restrict__ part, int &q, float &g) {
+    __shared__ float sums[4][kSumQ];
+    const int grp = threadIdx.x / kSumQ, at = threadIdx.x % kSumQ;
+    q = blockIdx.x * kSumQ + at;
+    float s = 0.0f;
+    if (q < kNP) {
+#pragma unroll 4
+        for (int t = grp; t < ntiles; t += 4) s += part[(size_t)t * kNPpad + q];
+    }
+    sums[grp][at] = s;
+    __syncthreads();
+    g = sums[0][at] + sums[1][at] + sums[2][at] + sums[3][at];
+    return grp == 0 && q < kNP;
+}
+
+// Adam on the FP32 masters with the gradient summed over tiles in a fixed
+// order; refreshes the forward copies (BF16 W1, W2, W2^T, w3; FP32 biases).
 __global__ void k_mlp_adam(int ntiles, const float *__restrict__ part, float *master, float *mom, float *vel,
                            float lr, float b1c, float b2c, float *W1, float *b1, __nv_bfloat16 *W2,
                            __nv_bfloat16 *W2t, float *b2, float *w3, float *b3, int update) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= kNP) return;
+    int q;
+    float g;
+    if (!tile_sum(ntiles, part, q, g)) return;
     float w = master[q];
     if (update) {
-        float g = 0.0f;
-        for (int t = 0; t < ntiles; ++t) g += part[(size_t)t * kNPpad + q];
         const float m1 = 0.9f * mom[q] + 0.1f * g;
         const float v1 = 0.999f * vel[q] + 0.001f * g * g;
         mom[q] = m1;
@@ -331,38 +551,15 @@ __global__ void k_mlp_adam(int ntiles, const float *__restrict__ part, float *ma
 
 // Gradient summed over tiles without an update (for checks).
 __global__ void k_mlp_gradsum(int ntiles, const float *__restrict__ part, float *g) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= kNP) return;
-    float s = 0.0f;
-    for (int t = 0; t < ntiles; ++t) s += part[(size_t)t * kNPpad + q];
-    g[q] = s;
+    int q;
+    float s;
+    if (tile_sum(ntiles, part, q, s)) g[q] = s;
 }
 
 // Hills packed as in hillsum.h.  A hill farther than sqrt(80) sigma from the
 // point contributes below h e^-40 (4e-18 h) and is skipped; its gradient term
 // is smaller still.
 constexpr double kExpCut = 40.0;
-
-// Caller points (rows of D doubles) to the network's normalised FP32 inputs.
-__global__ void k_nb_inputs(int D, int npts, const double *__restrict__ pts, double lo0, double lo1, double lo2,
-                            double lo3, double sc0, double sc1, double sc2, double sc3, float *x) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= npts) return;
-    const double lo[kIn] = {lo0, lo1, lo2, lo3}, sc[kIn] = {sc0, sc1, sc2, sc3};
-#pragma unroll
-    for (int k = 0; k < kIn; ++k) x[(size_t)i * kIn + k] = k < D ? (float)(sc[k] * (pts[(size_t)i * D + k] - lo[k]) - 1.0) : 0.f;
-}
-
-// Network outputs to V = vscale y and dV/ds = vscale dy/du du/ds (FP64, rows of D).
-__global__ void k_nb_outputs(int D, int npts, const float *__restrict__ y, const float *__restrict__ ds,
-                             double vscale, double sc0, double sc1, double sc2, double sc3, double *V, double *dV) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= npts) return;
-    const double sc[kIn] = {sc0, sc1, sc2, sc3};
-    V[i] = vscale * (double)y[i];
-    if (dV)
-        for (int k = 0; k < D; ++k) dV[(size_t)i * D + k] = vscale * (double)ds[(size_t)i * kIn + k] * sc[k];
-}
 
 // One point, hills spread over blocks; block partials reduced in block order by the last block.
 constexpr int kPointBlocks = 80;
@@ -501,9 +698,6 @@ struct mtd_nnbias {
     int adam_t = 0;
     int *d_err = nullptr;
     double *d_pt = nullptr, *d_ppart = nullptr, *d_pout = nullptr;
-    // device batch evaluation scratch (grown on demand)
-    float *d_bx = nullptr, *d_by = nullptr, *d_bds = nullptr;
-    int cap_b = 0;
     unsigned int *d_ticket = nullptr;
     // training pool
     int ntrain = 0;
@@ -549,12 +743,14 @@ MlpDev nb_dev(const mtd_nnbias *b) {
 mtd_status nb_tile_attr(mtd_nnbias *b) {
     std::lock_guard<std::mutex> lock(g_attr_mutex);
     if (b->device >= 0 && b->device < 64 && g_attr_done[b->device]) return MTD_OK;
-    NB_CU(cudaFuncSetAttribute(k_mlp_tile<MODE_FWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem),
-          "smem attribute");
-    NB_CU(cudaFuncSetAttribute(k_mlp_tile<MODE_GRAD_S>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem),
-          "smem attribute");
-    NB_CU(cudaFuncSetAttribute(k_mlp_tile<MODE_TRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmem),
-          "smem attribute");
+    const auto set = [](auto *k, int bytes) {
+        return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    };
+    NB_CU(set(k_mlp_eval<false, 1>, kEvalSmem), "smem attribute");
+    NB_CU(set(k_mlp_eval<true, 1>, kEvalSmem), "smem attribute");
+    NB_CU(set(k_mlp_eval<false, 4>, kEvalSmem), "smem attribute");
+    NB_CU(set(k_mlp_eval<true, 4>, kEvalSmem), "smem attribute");
+    NB_CU(set(k_mlp_train, kTrainSmem), "smem attribute");
     if (b->device >= 0 && b->device < 64) g_attr_done[b->device] = true;
     return MTD_OK;
 }
@@ -577,7 +773,7 @@ void nb_normalise(const mtd_nnbias *b, const double *s, float *u) {
 }
 
 mtd_status nb_refresh_forward(mtd_nnbias *b) {
-    k_mlp_adam<<<(kNP + 255) / 256, 256, 0, b->st>>>(0, b->d_part, b->d_master, b->d_mom, b->d_vel, 0.f, 1.f, 1.f,
+    k_mlp_adam<<<kSumBlocks, 256, 0, b->st>>>(0, b->d_part, b->d_master, b->d_mom, b->d_vel, 0.f, 1.f, 1.f,
                                                      b->d_W1, b->d_b1, b->d_W2, b->d_W2t, b->d_b2, b->d_w3,
                                                      b->d_b3, 0);
     NB_CU(cudaGetLastError(), "forward copies");
@@ -666,18 +862,26 @@ void nb_sample(const mtd_nnbias *b, int npts, unsigned long long seed, std::vect
     }
 }
 
+// A tile per block while every tile has an SM to itself (14.4 us, 16.5 with a
+// tile per warpgroup), beyond that a tile per warpgroup (200 tiles: 20.7 us
+// against 22.6 with two rounds of blocks; 1,184 tiles: 53 against 66).
+void nb_launch_eval(const mtd_nnbias *b, int npts, const MlpIo &io, bool grad, cudaStream_t st) {
+    const int ntiles = (npts + kH - 1) / kH;
+    const bool whole = ntiles <= 148;
+    const int grid = std::min(ntiles, 148);
+    const auto k = whole ? (grad ? k_mlp_eval<true, 4> : k_mlp_eval<false, 4>)
+                         : (grad ? k_mlp_eval<true, 1> : k_mlp_eval<false, 1>);
+    k<<<grid, 512, kEvalSmem, st>>>(nb_dev(b), npts, io, b->d_err, b->wait_tries, b->wait_stall);
+}
+
 mtd_status nb_forward_batch(mtd_nnbias *b, int npts, const float *d_x, float *d_y, float *d_ds) {
     mtd_status s = nb_tile_attr(b);
     if (s != MTD_OK) return s;
-    const int ntiles = (npts + kH - 1) / kH;
-    if (d_ds)
-        k_mlp_tile<MODE_GRAD_S><<<ntiles, 128, kTileSmem, b->st>>>(nb_dev(b), npts, d_x, nullptr, d_y, d_ds,
-                                                                   nullptr, nullptr, 0.f, b->d_err, b->wait_tries,
-                                                                   b->wait_stall);
-    else
-        k_mlp_tile<MODE_FWD><<<ntiles, 128, kTileSmem, b->st>>>(nb_dev(b), npts, d_x, nullptr, d_y, nullptr, nullptr,
-                                                                nullptr, 0.f, b->d_err, b->wait_tries,
-                                                                b->wait_stall);
+    MlpIo io{};
+    io.x = d_x;
+    io.y = d_y;
+    io.ds = d_ds;
+    nb_launch_eval(b, npts, io, d_ds != nullptr, b->st);
     NB_CU(cudaGetLastError(), "MLP forward");
     return MTD_OK;
 }
@@ -753,7 +957,7 @@ void mtd_nnbias_destroy(mtd_nnbias *b) {
     if (b->st) cudaStreamSynchronize(b->st);
     void *ptrs[] = {b->d_hills, b->d_master, b->d_mom, b->d_vel, b->d_W1, b->d_b1, b->d_b2, b->d_w3, b->d_b3,
                     b->d_W2, b->d_W2t, b->d_part, b->d_loss, b->d_err, b->d_pt, b->d_pout, b->d_ppart,
-                    b->d_ticket, b->d_xt, b->d_tt, b->d_bx, b->d_by, b->d_bds, b->d_hs};
+                    b->d_ticket, b->d_xt, b->d_tt, b->d_hs};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (b->hs_ev) cudaEventDestroy(b->hs_ev);
@@ -853,10 +1057,9 @@ mtd_status mtd_nnbias_loss_grad(mtd_nnbias *b, int npts, const double *pts, cons
     NB_CU(cudaMalloc(&d_g, sizeof(float) * kNPpad), "gradient");
     cudaMemcpyAsync(d_x, x.data(), sizeof(float) * x.size(), cudaMemcpyHostToDevice, b->st);
     cudaMemcpyAsync(d_t, t.data(), sizeof(float) * npts, cudaMemcpyHostToDevice, b->st);
-    k_mlp_tile<MODE_TRAIN><<<ntiles, 128, kTileSmem, b->st>>>(nb_dev(b), npts, d_x, d_t, nullptr, nullptr, b->d_part,
-                                                              b->d_loss, 2.0f / npts, b->d_err, b->wait_tries,
-                                                              b->wait_stall);
-    k_mlp_gradsum<<<(kNP + 255) / 256, 256, 0, b->st>>>(ntiles, b->d_part, d_g);
+    k_mlp_train<<<ntiles, 512, kTrainSmem, b->st>>>(nb_dev(b), npts, d_x, d_t, b->d_part, b->d_loss, 2.0f / npts,
+                                                    b->d_err, b->wait_tries, b->wait_stall);
+    k_mlp_gradsum<<<kSumBlocks, 256, 0, b->st>>>(ntiles, b->d_part, d_g);
     std::vector<float> lp(ntiles);
     cudaMemcpyAsync(grad, d_g, sizeof(float) * kNP, cudaMemcpyDeviceToHost, b->st);
     cudaMemcpyAsync(lp.data(), b->d_loss, sizeof(float) * ntiles, cudaMemcpyDeviceToHost, b->st);
@@ -946,10 +1149,10 @@ mtd_status mtd_nnbias_fit(mtd_nnbias *b, int ntrain, int iters, int batch, doubl
         const float b1c = 1.0f - std::pow(0.9f, (float)b->adam_t), b2c = 1.0f - std::pow(0.999f, (float)b->adam_t);
         const float lr_t = (float)(lr * (it < iters / 2 ? 1.0 : 0.5 * (1.0 + std::cos(M_PI * (it - iters / 2) /
                                                                                    std::max(1, iters - iters / 2)))));
-        k_mlp_tile<MODE_TRAIN><<<ntiles, 128, kTileSmem, b->st>>>(
-            nb_dev(b), nb, b->d_xt + (size_t)bi * batch * kIn, b->d_tt + (size_t)bi * batch, nullptr, nullptr,
-            b->d_part, b->d_loss, 2.0f / nb, b->d_err, b->wait_tries, b->wait_stall);
-        k_mlp_adam<<<(kNP + 255) / 256, 256, 0, b->st>>>(ntiles, b->d_part, b->d_master, b->d_mom, b->d_vel,
+        k_mlp_train<<<ntiles, 512, kTrainSmem, b->st>>>(nb_dev(b), nb, b->d_xt + (size_t)bi * batch * kIn,
+                                                        b->d_tt + (size_t)bi * batch, b->d_part, b->d_loss, 2.0f / nb,
+                                                        b->d_err, b->wait_tries, b->wait_stall);
+        k_mlp_adam<<<kSumBlocks, 256, 0, b->st>>>(ntiles, b->d_part, b->d_master, b->d_mom, b->d_vel,
                                                          std::max(lr_t, (float)(lr * 0.02)), b1c, b2c, b->d_W1,
                                                          b->d_b1, b->d_W2, b->d_W2t, b->d_b2, b->d_w3, b->d_b3, 1);
     }
@@ -1004,7 +1207,6 @@ mtd_status mtd_nnbias_eval_device(mtd_nnbias *b, int npts, const double *d_pts, 
     if (npts == 0) return MTD_OK;
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : b->st;
     const bool nn = use_nn > 0 || (use_nn < 0 && b->validated);
-    const int nb = (npts + 255) / 256;
     if (!nn) {
         if (b->nh == 0) {
             NB_CU(cudaMemsetAsync(d_V, 0, sizeof(double) * npts, st), "bias");
@@ -1014,33 +1216,18 @@ mtd_status mtd_nnbias_eval_device(mtd_nnbias *b, int npts, const double *d_pts, 
         NB_CU(nb_hillsum(b, npts, d_pts, b->D, d_V, d_dV, b->D, st), "exact hill sum");
         return MTD_OK;
     }
-    if (npts > b->cap_b) {
-        cudaFree(b->d_bx);
-        cudaFree(b->d_by);
-        cudaFree(b->d_bds);
-        b->d_bx = b->d_by = b->d_bds = nullptr;
-        b->cap_b = 0;
-        NB_CU(cudaMalloc(&b->d_bx, sizeof(float) * (size_t)npts * kIn), "points");
-        NB_CU(cudaMalloc(&b->d_by, sizeof(float) * (size_t)npts), "values");
-        NB_CU(cudaMalloc(&b->d_bds, sizeof(float) * (size_t)npts * kIn), "gradients");
-        b->cap_b = npts;
-    }
-    double sc[kIn];
-    for (int k = 0; k < kIn; ++k) sc[k] = 2.0 / (b->hi[k] - b->lo[k]);
-    k_nb_inputs<<<nb, 256, 0, st>>>(b->D, npts, d_pts, b->lo[0], b->lo[1], b->lo[2], b->lo[3], sc[0], sc[1], sc[2],
-                                    sc[3], b->d_bx);
     mtd_status s = nb_tile_attr(b);
     if (s != MTD_OK) return s;
-    const int ntiles = (npts + kH - 1) / kH;
-    if (d_dV)
-        k_mlp_tile<MODE_GRAD_S><<<ntiles, 128, kTileSmem, st>>>(nb_dev(b), npts, b->d_bx, nullptr, b->d_by, b->d_bds,
-                                                                nullptr, nullptr, 0.f, b->d_err, b->wait_tries,
-                                                                b->wait_stall);
-    else
-        k_mlp_tile<MODE_FWD><<<ntiles, 128, kTileSmem, st>>>(nb_dev(b), npts, b->d_bx, nullptr, b->d_by, nullptr,
-                                                             nullptr, nullptr, 0.f, b->d_err, b->wait_tries,
-                                                             b->wait_stall);
-    k_nb_outputs<<<nb, 256, 0, st>>>(b->D, npts, b->d_by, b->d_bds, b->vscale, sc[0], sc[1], sc[2], sc[3], d_V, d_dV);
+    MlpIo io{};
+    io.pts = d_pts;
+    io.V = d_V;
+    io.dV = d_dV;
+    io.vscale = b->vscale;
+    for (int k = 0; k < b->D; ++k) {
+        io.lo[k] = b->lo[k];
+        io.sc[k] = 2.0 / (b->hi[k] - b->lo[k]);
+    }
+    nb_launch_eval(b, npts, io, d_dV != nullptr, st);
     NB_CU(cudaGetLastError(), "network");
     return MTD_OK;
 }

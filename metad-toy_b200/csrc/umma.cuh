@@ -35,6 +35,12 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int M, int N) {
            (static_cast<uint32_t>(M >> 4) << 24);
 }
 
+// Operands read transposed (M- or N-major): the same 8 x 16-byte core matrices
+// then hold 8 K-rows of 8 consecutive M (N), with K groups `lbo` and M (N)
+// groups `sbo` apart.  A tile stored as above with rows k and columns m is
+// A^T for umma_desc(addr, 128, R * 16), the next K = 16 at + 256 bytes.
+constexpr uint32_t kIdescTransA = 1u << 15, kIdescTransB = 1u << 16;
+
 // Byte offset of element (row, k) in the operand layout above.
 __device__ __forceinline__ uint32_t umma_off(int row, int k, int rows) {
     return static_cast<uint32_t>((k >> 3) * rows * 16 + (row >> 3) * 128 + (row & 7) * 16 + (k & 7) * 2);
@@ -107,6 +113,17 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// 8 columns.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 
 }  // namespace mtd
