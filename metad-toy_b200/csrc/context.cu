@@ -148,6 +148,7 @@ NeighSpec neigh_spec(const Env &e) {
     } else {
         ns.kind = NK_RANGE;
     }
+    ns.accept = (float)(2.0 * e.eps + 1e-5);
     ns.lo2 = (float)(eff * (1.0 - 2e-5) - 1e-4);
     ns.hi2 = (float)(ns.kind == NK_SWITCH ? ns.rc2 * (1.0 + 2e-5) + 1e-4 : eff * (1.0 + 2e-5) + 1e-4);
     return ns;
@@ -848,8 +849,7 @@ mtd_status enqueue_values(mtd_ctx *c, int n, const double *x, const int *mask, c
             for (Env &e : c->envs) {
                 NeighSpec ns = neigh_spec(e);
                 ns.variant = c->tune_nbr;
-                launch_neighbors(g, s, ns, env_dev(e), c->d_status, c->st);
-                c->launches += ns.cap > 0 ? 2 : 1;
+                c->launches += launch_neighbors(g, s, ns, env_dev(e), c->d_status, c->st);
             }
             c->skin_valid = false;
         }

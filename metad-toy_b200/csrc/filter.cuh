@@ -1,8 +1,9 @@
 // filter.cuh -- the exact neighbour decision shared by the per-step neighbour
 // search and the skin-list filter.
 //
-// A candidate is decided by its FP32 cell-relative r^2 unless that lies
-// within the guard band [lo2, hi2] around the bound; inside the band the FP64
+// A candidate is decided by its FP32 cell-relative r^2 (and the FP32 value of a
+// smooth switch) unless that lies within the guard band [lo2, hi2] around the
+// bound (or near eps); inside the band the FP64
 // test on raw coordinates decides with the FP64 oracle's operations in the
 // same order, so every neighbour set equals the FP64 criterion exactly.
 #pragma once
@@ -62,7 +63,12 @@ template <int KIND>
 __device__ __forceinline__ bool decide(const GeoD &gd, const NeighSpec &ns, const double *xs, int k, int j,
                                        float r2f) {
     if (r2f > ns.hi2) return false;
-    if (KIND != NK_SWITCH && r2f < ns.lo2 && r2f > 1e-6f) return true;
+    if (r2f < ns.lo2 && r2f > 1e-6f) {
+        // a smooth switch well above eps: ns.accept leaves room for a relative
+        // error of its FP32 value of one half, where 1e-4 is usual (the FP64
+        // test, an exponential a pair, decided every listed pair before)
+        if (KIND != NK_SWITCH || sw_f<float>(ns.sw, sqrtf(r2f)) > ns.accept) return true;
+    }
     return exact_decide<KIND>(exact_spec(gd, ns), xs, k, j);
 }
 

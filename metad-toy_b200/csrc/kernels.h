@@ -126,6 +126,7 @@ struct NeighSpec {
     double eps;
     SwParams sw;
     float lo2, hi2;     // FP32 accept-below / reject-above
+    float accept;       // NK_SWITCH: an FP32 switch value above this is above eps
     int cap;            // STEINH Q cutoff_Natoms, 0 = none
     int variant;        // kernel shape of the fast path (0, 1, 2: see launch_neighbors); same lists
 };
@@ -182,14 +183,34 @@ void launch_k(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t sm
     cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// The same as clusters of `cluster` blocks.
+template <typename... KArgs, typename... Args>
+void launch_k_cluster(void (*kernel)(KArgs...), unsigned grid, unsigned cluster, unsigned block, cudaStream_t st,
+                      Args &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = pdl_on() ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 // ------------------------------------------------------------------ neighbours
 // Cell list (counting sort by cell).  The cell counts must be zero on entry:
 // they are zeroed when allocated and again by the scatter pass after use.
 // Returns the number of kernels launched.
 int launch_build_cells(const CellGrid &g, SysDev &s, cudaStream_t st);
 // Neighbour lists from the cell list (ns.kind NK_CAND: skin-list candidates;
-// for a cap, the cap selection follows unless ns.kind is NK_CAND).
-void launch_neighbors(const CellGrid &g, const SysDev &s, const NeighSpec &ns, NeighDev nd, DevStatus *status,
+// for a cap, the cap selection follows unless ns.kind is NK_CAND).  Returns the
+// number of kernels launched.
+int launch_neighbors(const CellGrid &g, const SysDev &s, const NeighSpec &ns, NeighDev nd, DevStatus *status,
                       cudaStream_t st);
 void launch_select_cap(const CellGrid &g, const SysDev &s, const NeighSpec &ns, NeighDev nd, cudaStream_t st);
 // Skin lists: the per-step repack and rebuild decision (force: the kept

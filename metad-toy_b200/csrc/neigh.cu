@@ -24,11 +24,16 @@
 // src/core/neigh_hub.cu:191-222).
 #include "persist.cuh"
 
+#include <cooperative_groups.h>
 #include <math_constants.h>
+
+#include <atomic>
 
 namespace mtd {
 
 namespace {
+
+namespace cg = cooperative_groups;
 
 
 // The rebuild kernels return at once while the skin gate is closed (the
@@ -148,6 +153,48 @@ __global__ void k_place(CellGrid g, SysDev s) {
     place_body(g, s, blockIdx.x);
 }
 
+// The whole cell list in one launch of one cluster (16 SMs), its phases apart
+// by cluster barriers instead of launches: bin, scan (a chunk of cells per
+// block, the blocks' totals read from each other's shared memory; the counts
+// are zeroed for the next build as they are read), scatter, place.  The same
+// per-atom work and the same order as the five kernels.  A small system's
+// kernels are all latency: 4,000 atoms 33 us (five kernels, event intervals)
+// and 17 now, 32,000 atoms 40 and 23, 61,000 atoms 34 and 34 on a tenth of
+// the SMs and with four launches fewer; beyond 65,536 the five kernels.
+constexpr int kClusterBlocks = 16, kClusterAtoms = 4;   // atoms per thread
+__global__ void __launch_bounds__(kScanBlock) k_cells_cluster(CellGrid g, SysDev s) {
+    pdl_entry();
+    __shared__ int sum;
+    if (gate_closed(s.skin)) return;
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = cl.block_rank();
+    for (int v = rank; v * kScanBlock < s.n; v += kClusterBlocks) bin_body(g, s, v);
+    cl.sync();
+    const int per = (g.ncell + kClusterBlocks * kScanBlock - 1) / (kClusterBlocks * kScanBlock);
+    const int c0 = (rank * kScanBlock + threadIdx.x) * per, c1 = min(c0 + per, g.ncell);
+    int mine = 0;
+    for (int c = c0; c < c1; ++c) mine += s.count[c];
+    int total;
+    int at = block_excl_scan(mine, total);
+    if (threadIdx.x == 0) sum = total;
+    cl.sync();
+    for (int r = 0; r < rank; ++r) at += *cl.map_shared_rank(&sum, r);
+    for (int c = c0; c < c1; ++c) {
+        const int v = s.count[c];
+        s.count[c] = 0;
+        s.start[c] = at;
+        at += v;
+    }
+    if (rank == kClusterBlocks - 1 && threadIdx.x == kScanBlock - 1) s.start[g.ncell] = s.n;
+    cl.sync();   // also: no block leaves while another reads its total
+    for (int v = rank; v * kScanBlock < s.n; v += kClusterBlocks) {
+        const int i = v * kScanBlock + threadIdx.x;
+        if (i < s.n) s.arrival[s.start[s.cellof[i]] + s.slot[i]] = i;
+    }
+    cl.sync();
+    for (int v = rank; v * kScanBlock < s.n; v += kClusterBlocks) place_body(g, s, v);
+}
+
 template <int KIND>
 __global__ void __launch_bounds__(kBlock) k_neighbors(CellGrid g, SysDev s, NeighSpec ns, NeighDev nd,
                                                       DevStatus *status) {
@@ -200,14 +247,7 @@ __global__ void __launch_bounds__(kBlock) k_neighbors(CellGrid g, SysDev s, Neig
                     float dx, dy, dz;
                     disp_f(gf, a, b, dx, dy, dz);
                     const float r2f = dx * dx + dy * dy + dz * dz;
-                    if (r2f > ns.hi2) continue;
-                    bool in;
-                    if (KIND != NK_SWITCH && r2f < ns.lo2 && r2f > 1e-6f) {
-                        in = true;
-                    } else {
-                        in = exact_decide<KIND>(exact_spec(gd, ns), s.xs, k, j);
-                    }
-                    if (!in) continue;
+                    if (!decide<KIND>(gd, ns, s.xs, k, j, r2f)) continue;
                     if (cnt < nd.M) nd.list[(size_t)cnt * s.npad + k] = j;
                     ++cnt;
                 }
@@ -219,6 +259,8 @@ __global__ void __launch_bounds__(kBlock) k_neighbors(CellGrid g, SysDev s, Neig
 }
 
 
+constexpr int kMaxCapList = 64;
+
 // Fast path, valid when every periodic dimension has at least three cells
 // (neighbors_fast_body).
 template <int KIND>
@@ -227,6 +269,170 @@ __global__ void __launch_bounds__(kBlock) k_neighbors_fast(CellGrid g, SysDev s,
     pdl_entry();
     if (gate_closed(s.skin)) return;
     neighbors_fast_body<KIND>(g, s, ns, nd, status, blockIdx.x);
+}
+
+// Same lists as k_neighbors_fast, one warp per atom: lanes 0..26 read the
+// stencil cells' ranges at once, the candidates of all cells are dealt to the
+// lanes in list order, and a ballot packs the survivors.  Bound by latency
+// where it is used: a thread per atom goes through some 50 (STEP) to 180
+// candidates one after another with a few warps per SM, a warp per atom
+// through two to six rounds of them (a lane per stencil cell in place of the
+// dealing measured the same for STEP and a quarter longer for switches).  A
+// smooth switch is evaluated for 32 candidates in range at a time.  With the
+// cap of STEINH Q the warp also ranks its list (k_select_cap), from shared
+// memory.
+// Event intervals, before and now: 4,000 atoms, cutoff 3.9 with the cap 58 us
+// (search 35, ranking 23) and 10; 32,000 atoms, cutoff 6.0 with the cap 101
+// and 50, without 54 and 33; 61,111 atoms, FERMI 125 and 60.
+constexpr int kWarpAtoms = kBlock / 32;
+template <int KIND, bool CAP>
+__global__ void __launch_bounds__(kBlock) k_neighbors_warp(CellGrid g, SysDev s, NeighSpec ns, NeighDev nd,
+                                                           DevStatus *status) {
+    pdl_entry();
+    __shared__ int held[CAP || KIND == NK_SWITCH ? kWarpAtoms : 1][kMaxCapList];
+    __shared__ float held_r2[KIND == NK_SWITCH ? kWarpAtoms : 1][kMaxCapList];
+    if (gate_closed(s.skin)) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = blockIdx.x * kWarpAtoms + warp;
+    if (k >= s.n) return;   // whole warps; no block-wide synchronisation below
+    const unsigned all = 0xffffffffu, below = (1u << lane) - 1;
+    const GeoD gd = geo_d(g, s.xs);
+    const float4 a = s.pf[k];
+    const int w = __float_as_int(a.w);
+    const int ox = lane / 9 - 1, oy = lane / 3 % 3 - 1, oz = lane % 3 - 1;
+    int x = (w & 1023) + ox, y = ((w >> 10) & 1023) + oy, z = (w >> 20) + oz;
+    bool cell = lane < 27;
+    if (x < 0 || x >= g.nc[0]) {
+        cell = cell && g.periodic[0];
+        x += x < 0 ? g.nc[0] : -g.nc[0];
+    }
+    if (y < 0 || y >= g.nc[1]) {
+        cell = cell && g.periodic[1];
+        y += y < 0 ? g.nc[1] : -g.nc[1];
+    }
+    if (z < 0 || z >= g.nc[2]) {
+        cell = cell && g.periodic[2];
+        z += z < 0 ? g.nc[2] : -g.nc[2];
+    }
+    int first = 0, len = 0;
+    if (cell) {
+        const int key = cell_key(g, x, y, z);
+        first = __ldg(s.start + key);
+        len = __ldg(s.start + key + 1) - first;
+    }
+    int end = len;   // candidates up to and with this lane's cell
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(all, end, o);
+        if (lane >= o) end += v;
+    }
+    const int begin = end - len, total = __shfl_sync(all, end, 31);
+    int cnt = 0, wait = 0;
+    auto keep = [&](bool in, int j) {
+        const unsigned hits = __ballot_sync(all, in);
+        const int at = cnt + __popc(hits & below);
+        if (in && at < nd.M) {
+            if (CAP) held[warp][at] = j;   // M <= kMaxCapList with a cap
+            else nd.list[(size_t)at * s.npad + k] = j;
+        }
+        cnt += __popc(hits);
+    };
+    // NK_SWITCH: the switch is evaluated for full warps of candidates in range
+    auto decide_held = [&](int n) {
+        __syncwarp();
+        const int j = lane < n ? held[warp][lane] : k;
+        const float r2f = lane < n ? held_r2[warp][lane] : 0.f;
+        keep(lane < n && decide<KIND>(gd, ns, s.xs, k, j, r2f), j);
+    };
+    for (int t0 = 0; t0 < total; t0 += 32) {
+        const int t = t0 + lane;
+        int c = 0;   // the last cell that begins at or before t
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const int v = __shfl_sync(all, begin, c + o);
+            if (c + o < 27 && v <= t) c += o;
+        }
+        const int j = __shfl_sync(all, first, c) + t - __shfl_sync(all, begin, c);
+        float r2f = INFINITY;
+        if (t < total && j != k) {
+            const float4 b = __ldg(s.pf + j);
+            const float dx = b.x + ((float)(c / 9 - 1) * g.hf[0] - a.x);
+            const float dy = b.y + ((float)(c / 3 % 3 - 1) * g.hf[1] - a.y);
+            const float dz = b.z + ((float)(c % 3 - 1) * g.hf[2] - a.z);
+            r2f = dx * dx + dy * dy + dz * dz;
+        }
+        if (KIND != NK_SWITCH) {
+            keep(r2f < INFINITY && decide<KIND>(gd, ns, s.xs, k, j, r2f), j);
+            continue;
+        }
+        // NaN fails, as in decide
+        const bool in = r2f <= ns.hi2;
+        const unsigned hits = __ballot_sync(all, in);
+        const int at = wait + __popc(hits & below);
+        if (in) {
+            held[warp][at] = j;
+            held_r2[warp][at] = r2f;
+        }
+        wait += __popc(hits);
+        if (wait >= 32) {
+            decide_held(32);
+            const int j2 = held[warp][32 + lane];
+            const float q2 = held_r2[warp][32 + lane];
+            __syncwarp();
+            held[warp][lane] = j2;
+            held_r2[warp][lane] = q2;
+            wait -= 32;
+        }
+    }
+    if (KIND == NK_SWITCH && wait > 0) decide_held(wait);
+    if (lane == 0) {
+        nd.count[k] = cnt;
+        if (cnt > nd.M) atomicMax(&status->overflow, (unsigned)cnt);
+    }
+    if (!CAP) return;
+    __syncwarp();
+    const int c = min(cnt, min(nd.M, kMaxCapList));
+    const double xk[3] = {s.xs[3 * k], s.xs[3 * k + 1], s.xs[3 * k + 2]};
+    double r2[2];
+    int id[2], jj[2], rank[2] = {0, 0};
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int t = lane + 32 * e;
+        r2[e] = CUDART_INF;
+        id[e] = 0x7fffffff;
+        jj[e] = 0;
+        if (t < c) {
+            jj[e] = held[warp][t];
+            const double xj[3] = {s.xs[3 * jj[e]], s.xs[3 * jj[e] + 1], s.xs[3 * jj[e] + 2]};
+            double d[3];
+            r2[e] = exact_disp(gd, xk, xj, d);
+            id[e] = s.perm[jj[e]];
+        }
+    }
+    for (int u = 0; u < c; ++u) {
+        const double ru = __shfl_sync(all, u < 32 ? r2[0] : r2[1], u);
+        const int iu = __shfl_sync(all, u < 32 ? id[0] : id[1], u);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) rank[e] += ru < r2[e] || (ru == r2[e] && iu < id[e]);
+    }
+    double kr2 = CUDART_INF;
+    int kid = 0x7fffffff;
+    unsigned owner = 0;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const bool mine = lane + 32 * e < c;
+        if (mine) nd.list[(size_t)(lane + 32 * e) * s.npad + k] = jj[e] | (rank[e] < ns.cap ? 1 << kFlagBit : 0);
+        const bool key = mine && c > ns.cap && rank[e] == ns.cap - 1;
+        if (key) {
+            kr2 = r2[e];
+            kid = id[e];
+        }
+        owner |= __ballot_sync(all, key);
+    }
+    if (lane == (owner ? __ffs(owner) - 1 : 0)) {
+        nd.key_r2[k] = kr2;
+        nd.key_id[k] = kid;
+        nd.nkept[k] = c < ns.cap ? c : ns.cap;
+    }
 }
 
 // Same lists as k_neighbors_fast (same cells in the same order, same tests),
@@ -316,21 +522,13 @@ __global__ void __launch_bounds__(kFlatBlock) k_neighbors_flat(CellGrid g, SysDe
         if (live) nxt = __ldg(s.pf + j);
         const float r2f = dx * dx + dy * dy + dz * dz;
         if (r2f > ns.hi2 || jj == k) continue;
-        bool in;
-        if (KIND == NK_CAND || (KIND != NK_SWITCH && r2f < ns.lo2 && r2f > 1e-6f)) {
-            in = true;
-        } else {
-            in = exact_decide<KIND>(exact_spec(gd, ns), s.xs, k, jj);
-        }
-        if (!in) continue;
+        if (KIND != NK_CAND && !decide<KIND>(gd, ns, s.xs, k, jj, r2f)) continue;
         if (cnt < nd.M) nd.list[(size_t)cnt * s.npad + k] = jj;
         ++cnt;
     }
     nd.count[k] = cnt;
     if (cnt > nd.M) atomicMax(KIND == NK_CAND ? &status->cand_overflow : &status->overflow, (unsigned)cnt);
 }
-
-constexpr int kMaxCapList = 64;
 
 // STEINH Q cap: keep the `cap` nearest by (r2, caller index), the order of the
 // reference's strict-'>' insertion with ties resolved canonically.
@@ -506,9 +704,41 @@ cudaError_t launch_rebuild(const CellGrid &g, const SysDev &s, const NeighSpec &
     return e;
 }
 
+// Whether k_cells_cluster can run on the current device (asked once).
+static bool cells_cluster_ok() {
+    static std::atomic<int> known[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    int k = known[dev].load();
+    if (k == 0) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kClusterBlocks);
+        cfg.blockDim = dim3(kScanBlock);
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = kClusterBlocks;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int fit = 0;
+        k = cudaFuncSetAttribute(k_cells_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&fit, k_cells_cluster, &cfg) == cudaSuccess && fit > 0
+                ? 1
+                : -1;
+        cudaGetLastError();
+        known[dev].store(k);
+    }
+    return k > 0;
+}
+
 int launch_build_cells(const CellGrid &g, SysDev &s, cudaStream_t st) {
     const int nb = (s.n + kBlock - 1) / kBlock;
     const SkinState *sk = s.skin;
+    if (s.n > 0 && s.n <= kClusterBlocks * kScanBlock * kClusterAtoms && cells_cluster_ok()) {
+        launch_k_cluster(k_cells_cluster, kClusterBlocks, kClusterBlocks, kScanBlock, st, g, s);
+        prof_mark("cell_list", st);
+        return 1;
+    }
     if (s.n > 0) launch_k(k_bin, nb, kBlock, 0, st, g, s);
     prof_mark("cell_bin", st);
     {
@@ -533,9 +763,16 @@ int launch_build_cells(const CellGrid &g, SysDev &s, cudaStream_t st) {
     return (s.n > 0 ? 3 : 0) + (sb <= kScanBlock ? 2 : 3);
 }
 
-void launch_neighbors(const CellGrid &g, const SysDev &s, const NeighSpec &ns, NeighDev nd, DevStatus *status,
-                      cudaStream_t st) {
-    if (s.n == 0) return;
+// One warp per atom up to 65,536 atoms, 131,072 for a smooth switch: there a
+// thread per atom has the warps to hide its loads and runs fewer instructions
+// (STEP at 64,000 atoms 38 us and 29 with a warp per atom, at 100,000 39 and
+// 41, at 200,000 68 and 74; cutoff 6.0 at 32,000 54 and 33, at 87,000 57 and
+// 76; FERMI at 64,000 110 and 62).
+constexpr int kWarpMax = 65536;
+
+int launch_neighbors(const CellGrid &g, const SysDev &s, const NeighSpec &ns, NeighDev nd, DevStatus *status,
+                     cudaStream_t st) {
+    if (s.n == 0) return 0;
     const int nb = (s.n + kBlock - 1) / kBlock;
     bool fast = true;
     for (int c = 0; c < 3; ++c)
@@ -543,7 +780,15 @@ void launch_neighbors(const CellGrid &g, const SysDev &s, const NeighSpec &ns, N
     // the fast path has three interchangeable shapes (identical lists): 256- or
     // 128-thread blocks of k_neighbors_fast, or k_neighbors_flat (autotuned)
     // skin-list candidates need the fast path (the context builds them only where it applies)
-    if (fast && ns.variant == 2 && s.n < (1 << 26)) {
+    bool capped = ns.cap > 0 && ns.kind != NK_CAND;
+    if (fast && ns.variant == 0 && ns.kind != NK_CAND && s.n <= (ns.kind == NK_SWITCH ? 2 : 1) * kWarpMax) {
+        const int wb = (s.n + kWarpAtoms - 1) / kWarpAtoms;
+        if (ns.kind == NK_RANGE && capped) launch_k(k_neighbors_warp<NK_RANGE, true>, wb, kBlock, 0, st, g, s, ns, nd, status);
+        else if (ns.kind == NK_RANGE) launch_k(k_neighbors_warp<NK_RANGE, false>, wb, kBlock, 0, st, g, s, ns, nd, status);
+        else if (ns.kind == NK_STEP) launch_k(k_neighbors_warp<NK_STEP, false>, wb, kBlock, 0, st, g, s, ns, nd, status);
+        else launch_k(k_neighbors_warp<NK_SWITCH, false>, wb, kBlock, 0, st, g, s, ns, nd, status);
+        capped = false;   // ranked by the same kernel
+    } else if (fast && ns.variant == 2 && s.n < (1 << 26)) {
         const int fb = (s.n + kFlatBlock - 1) / kFlatBlock;
         if (ns.kind == NK_RANGE) launch_k(k_neighbors_flat<NK_RANGE>, fb, kFlatBlock, 0, st, g, s, ns, nd, status);
         else if (ns.kind == NK_STEP) launch_k(k_neighbors_flat<NK_STEP>, fb, kFlatBlock, 0, st, g, s, ns, nd, status);
@@ -560,7 +805,8 @@ void launch_neighbors(const CellGrid &g, const SysDev &s, const NeighSpec &ns, N
     else if (ns.kind == NK_STEP) launch_k(k_neighbors<NK_STEP>, nb, kBlock, 0, st, g, s, ns, nd, status);
     else launch_k(k_neighbors<NK_SWITCH>, nb, kBlock, 0, st, g, s, ns, nd, status);
     prof_mark(ns.kind == NK_CAND ? "neighbor_candidates" : "neighbors", st);
-    if (ns.cap > 0 && ns.kind != NK_CAND) launch_select_cap(g, s, ns, nd, st);
+    if (capped) launch_select_cap(g, s, ns, nd, st);
+    return capped ? 2 : 1;
 }
 
 void launch_select_cap(const CellGrid &g, const SysDev &s, const NeighSpec &ns, NeighDev nd, cudaStream_t st) {

@@ -130,13 +130,7 @@ __device__ __forceinline__ void neighbors_fast_body(const CellGrid &g, const Sys
                     const float dx = b.x + sx, dy = b.y + sy, dz = b.z + sz;
                     const float r2f = dx * dx + dy * dy + dz * dz;
                     if (r2f > ns.hi2 || j == k) continue;
-                    bool in;
-                    if (KIND == NK_CAND || (KIND != NK_SWITCH && r2f < ns.lo2 && r2f > 1e-6f)) {
-                        in = true;
-                    } else {
-                        in = exact_decide<KIND>(exact_spec(gd, ns), s.xs, k, j);
-                    }
-                    if (!in) continue;
+                    if (KIND != NK_CAND && !decide<KIND>(gd, ns, s.xs, k, j, r2f)) continue;
                     if (cnt < nd.M) nd.list[(size_t)cnt * s.npad + k] = j;
                     ++cnt;
                 }
