@@ -190,10 +190,16 @@ mtd_status alloc_env(mtd_ctx *c, Env &e, int npad) {
     return MTD_OK;
 }
 
+// Atoms per block of a unit's passes, and so per row of its partial sums and
+// virial partials.
+static int unit_block(const Unit &u, int n) {
+    return u.kind == CAL_STEINH_Q || u.kind == CAL_STRU_FACTOR ? lanes_block(n) : kBlock;
+}
+
 mtd_status alloc_unit(mtd_ctx *c, Unit &u, int npad) {
     const size_t R = real_size(c);
     const int SQ = record_stride(c, u);
-    const int nb = (npad + kBlock - 1) / kBlock;
+    const int nb = std::max((npad + kBlock - 1) / kBlock, (std::min(npad, kLaneAtoms) * kLanes + kBlock - 1) / kBlock);
     void **arrs[] = {&u.q, &u.nf, &u.lq, &u.lqs, &u.e12, &u.lam, &u.g, &u.tu, &u.Q, &u.S, &u.w};
     for (void **a : arrs) dfree(*a);
     dfree(u.partials);
@@ -374,7 +380,7 @@ void build_plan(mtd_ctx *c) {
             Q.sk_n = U.skn;
         } else {
             Q.partials = U.partials;
-            Q.nparts = (c->n + kBlock - 1) / kBlock;
+            Q.nparts = (c->n + unit_block(U, c->n) - 1) / unit_block(U, c->n);
             Q.pstride = 8;
             Q.nvals = U.kind == CAL_STEINH_L ? 5 : 4;
             Q.rho = nullptr;
@@ -699,7 +705,7 @@ void run_forces(mtd_ctx *c, const SysDev &s, const CellGrid &g, const double *x,
         if (!u.used) continue;
         const double *src = first ? fin : fout;
         double *vp = virial ? c->d_vpart + (size_t)voff * 8 : nullptr;
-        const int nb = (c->n + kBlock - 1) / kBlock;
+        const int nb = (c->n + unit_block(u, c->n) - 1) / unit_block(u, c->n);
         if (u.kind == CAL_STEINH_L) {
             launch_local_forces<T>(local_dev<T>(c, u, g), src, fout, s, g, vp, c->d_status, st);
             c->launches += 2;

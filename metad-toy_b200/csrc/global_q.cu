@@ -29,20 +29,20 @@ template <int L> struct QSize {
     static constexpr int SQ = pad4(S);
 };
 
-template <int L, typename T> __global__ void __launch_bounds__(kBlock) k_global_values(GlobalDev<T> d) {
+template <int L, typename T, int G> __global__ void __launch_bounds__(kBlock) k_global_values(GlobalDev<T> d) {
     pdl_entry();
     using Z = QSize<L>;
     __shared__ double smem[4 * 32];
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = blockIdx.x * (kBlock / G) + threadIdx.x / G, sub = threadIdx.x % G;
     double part[4] = {0, 0, 0, 0};
+    T acc[Z::SQ];
+#pragma unroll
+    for (int t = 0; t < Z::SQ; ++t) acc[t] = T(0);
+    int kept = 0;
     if (k < d.n) {
         const auto a = d.geo.load(k);
         const int c = min(d.nb.count[k], d.nb.M);
-        T acc[Z::SQ];
-#pragma unroll
-        for (int t = 0; t < Z::SQ; ++t) acc[t] = T(0);
-        int kept = 0;
-        for (int t = 0; t < c; ++t) {
+        for (int t = sub; t < c; t += G) {
             const int e = d.nb.list[(size_t)t * d.npad + k];
             if (!((e >> kFlagBit) & 1)) continue;
             T dx, dy, dz;
@@ -51,6 +51,13 @@ template <int L, typename T> __global__ void __launch_bounds__(kBlock) k_global_
             ylm_accum<L, T>(dx * rinv, dy * rinv, dz * rinv, T(1), acc);
             ++kept;
         }
+    }
+    if (G > 1) {
+        kept = lanes_total<G>(kept);
+#pragma unroll
+        for (int t = 0; t < Z::S; ++t) acc[t] = lanes_total<G>(acc[t]);
+    }
+    if (k < d.n) {
         const T inv = kept > 0 ? T(1) / T(kept) : T(0);
 #pragma unroll
         for (int t = 0; t < Z::SQ; ++t) acc[t] *= inv;
@@ -59,9 +66,10 @@ template <int L, typename T> __global__ void __launch_bounds__(kBlock) k_global_
         for (int m = 1; m <= L; ++m) q2 += T(2) * (acc[2 * m] * acc[2 * m] + acc[2 * m + 1] * acc[2 * m + 1]);
         const T Q = kept > 0 ? t_sqrt<T>(q2 * T(4.0 * kPi / (2 * L + 1))) : T(0);
 #pragma unroll
-        for (int t = 0; t < Z::SQ; ++t) d.q[(size_t)k * Z::SQ + t] = acc[t];
-        d.Q[k] = Q;
-        if (d.smask[k] & d.groupbit) {
+        for (int t = 0; t < Z::SQ; ++t)
+            if (t % G == sub) d.q[(size_t)k * Z::SQ + t] = acc[t];
+        if (sub == 0) d.Q[k] = Q;
+        if (sub == 0 && (d.smask[k] & d.groupbit)) {
             part[0] = (double)Q;
             if (d.nsw > 0) part[1] = sw_f<double>(d.sw[0], (double)Q);
             if (d.nsw > 1) part[2] = sw_f<double>(d.sw[1], (double)Q);
@@ -85,28 +93,29 @@ __device__ __forceinline__ T lambda_scale(const GlobalDev<T> &d, int k, const do
     return (T)(dcv * (4.0 * kPi / (2 * L + 1)) / (Q * n));
 }
 
-template <int L, typename T>
+template <int L, typename T, int G>
 __global__ void __launch_bounds__(kBlock) k_global_force(GlobalDev<T> d, const double *__restrict__ f_src,
                                                          double *__restrict__ f_dst, SysDev s, CellGrid g,
                                                          double *vpart, DevStatus *status) {
     pdl_entry();
     using Z = QSize<L>;
     __shared__ double smem[6 * 32];
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = blockIdx.x * (kBlock / G) + threadIdx.x / G, sub = threadIdx.x % G;
     double vir[6] = {0, 0, 0, 0, 0, 0};
     const double c[3] = {d.coef[0], d.coef[1], d.coef[2]};
+    T gx = T(0), gy = T(0), gz = T(0);
+    int myid = 0;
     if (k < d.n) {
         const T ak = lambda_scale<L, T>(d, k, c);
         T la[Z::SQ];
 #pragma unroll
         for (int t = 0; t < Z::SQ; ++t) la[t] = ak * d.q[(size_t)k * Z::SQ + t] * (t >= 2 ? T(2) : T(1));
-        const int myid = d.perm[k];
+        myid = d.perm[k];
         const double xk[3] = {s.xs[3 * k], s.xs[3 * k + 1], s.xs[3 * k + 2]};
         const auto a = d.geo.load(k);
         constexpr T sgn = (L & 1) ? T(-1) : T(1);
-        T gx = T(0), gy = T(0), gz = T(0);
         const int cnt = min(d.nb.count[k], d.nb.M);
-        for (int t = 0; t < cnt; ++t) {
+        for (int t = sub; t < cnt; t += G) {
             const int e = d.nb.list[(size_t)t * d.npad + k];
             const bool kept = (e >> kFlagBit) & 1;
             const int j = e & ((1 << kFlagBit) - 1);
@@ -135,6 +144,13 @@ __global__ void __launch_bounds__(kBlock) k_global_force(GlobalDev<T> d, const d
             gy -= ay;
             gz -= az;
         }
+    }
+    if (G > 1) {
+        gx = lanes_total<G>(gx);
+        gy = lanes_total<G>(gy);
+        gz = lanes_total<G>(gz);
+    }
+    if (k < d.n && sub == 0) {
         const int i = myid;
         const double fx = -(double)gx, fy = -(double)gy, fz = -(double)gz;
         const bool own = (unsigned)i < (unsigned)d.n;   // a sorted order left by a rebuild that gave up is not trusted
@@ -145,7 +161,7 @@ __global__ void __launch_bounds__(kBlock) k_global_force(GlobalDev<T> d, const d
         }
         if (!(isfinite(fx) && isfinite(fy) && isfinite(fz))) atomicOr(&status->nan_force, 1u);
         if (vpart && own) {
-            double ux = xk[0], uy = xk[1], uz = xk[2];
+            double ux = s.xs[3 * k], uy = s.xs[3 * k + 1], uz = s.xs[3 * k + 2];
             if (s.image) {
                 int ix, iy, iz;
                 unpack_image(s.image[i], ix, iy, iz);
@@ -166,26 +182,38 @@ __global__ void __launch_bounds__(kBlock) k_global_force(GlobalDev<T> d, const d
 
 }  // namespace
 
+template <int L, typename T> static void launch_global_values_l(const GlobalDev<T> &d, cudaStream_t st) {
+    const int ab = lanes_block(d.n), nb = (d.n + ab - 1) / ab;
+    if (ab < kBlock) launch_k(k_global_values<L, T, kLanes>, nb, kBlock, 0, st, d);
+    else launch_k(k_global_values<L, T, 1>, nb, kBlock, 0, st, d);
+}
+
 template <typename T> void launch_global_values(const GlobalDev<T> &d, cudaStream_t st) {
     if (d.n == 0) return;
-    const int nb = (d.n + kBlock - 1) / kBlock;
     switch (d.L) {
-    case 3: launch_k(k_global_values<3, T>, nb, kBlock, 0, st, d); break;
-    case 4: launch_k(k_global_values<4, T>, nb, kBlock, 0, st, d); break;
-    case 6: launch_k(k_global_values<6, T>, nb, kBlock, 0, st, d); break;
+    case 3: launch_global_values_l<3>(d, st); break;
+    case 4: launch_global_values_l<4>(d, st); break;
+    case 6: launch_global_values_l<6>(d, st); break;
     }
     prof_mark("global_values", st);
+}
+
+template <int L, typename T>
+static void launch_global_forces_l(const GlobalDev<T> &d, const double *f_src, double *f_dst, const SysDev &s,
+                                   const CellGrid &g, double *vpart, DevStatus *status, cudaStream_t st) {
+    const int ab = lanes_block(d.n), nb = (d.n + ab - 1) / ab;
+    if (ab < kBlock) launch_k(k_global_force<L, T, kLanes>, nb, kBlock, 0, st, d, f_src, f_dst, s, g, vpart, status);
+    else launch_k(k_global_force<L, T, 1>, nb, kBlock, 0, st, d, f_src, f_dst, s, g, vpart, status);
 }
 
 template <typename T>
 void launch_global_forces(const GlobalDev<T> &d, const double *f_src, double *f_dst, const SysDev &s,
                           const CellGrid &g, double *vpart, DevStatus *status, cudaStream_t st) {
     if (d.n == 0) return;
-    const int nb = (d.n + kBlock - 1) / kBlock;
     switch (d.L) {
-    case 3: launch_k(k_global_force<3, T>, nb, kBlock, 0, st, d, f_src, f_dst, s, g, vpart, status); break;
-    case 4: launch_k(k_global_force<4, T>, nb, kBlock, 0, st, d, f_src, f_dst, s, g, vpart, status); break;
-    case 6: launch_k(k_global_force<6, T>, nb, kBlock, 0, st, d, f_src, f_dst, s, g, vpart, status); break;
+    case 3: launch_global_forces_l<3>(d, f_src, f_dst, s, g, vpart, status, st); break;
+    case 4: launch_global_forces_l<4>(d, f_src, f_dst, s, g, vpart, status, st); break;
+    case 6: launch_global_forces_l<6>(d, f_src, f_dst, s, g, vpart, status, st); break;
     }
     prof_mark("global_force", st);
 }

@@ -271,6 +271,20 @@ void launch_local_force_pass(const LocalDev<T> &d, const double *f_src, double *
                              const CellGrid &g, double *vpart, DevStatus *status, cudaStream_t st);
 
 // ------------------------------------------------------------------ STEINH Q
+// Lanes per atom of the STEINH Q and STRU_FACTOR passes: eight while a thread
+// per atom would leave most of the GPU without work (LANES_NOTE), each lane
+// taking every eighth neighbour.  A block then holds 32 atoms instead of 256,
+// and so do its partial sums.
+constexpr int kLaneAtoms = 65536;
+constexpr int kLanes = 8;
+inline int lanes_block(int n) { return n <= kLaneAtoms ? kBlock / kLanes : kBlock; }
+// Sum over the G lanes of an atom (G neighbouring lanes, all in the warp).
+template <int G, typename T> __device__ __forceinline__ T lanes_total(T v) {
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
 template <typename T> struct GlobalDev {
     int n, npad, SQ, L;
     int groupbit, nsw;

@@ -54,33 +54,35 @@ template <typename T> __global__ void k_chem_weights(DebyeDev<T> d) {
     d.w[k] = (T)(t >= 0 && t < d.ntab ? d.wtab[t] : 0.0);
 }
 
-template <typename T> __global__ void __launch_bounds__(kBlock) k_debye_values(DebyeDev<T> d) {
+template <typename T, int G> __global__ void __launch_bounds__(kBlock) k_debye_values(DebyeDev<T> d) {
     pdl_entry();
     __shared__ double smem[4 * 32];
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = blockIdx.x * (kBlock / G) + threadIdx.x / G, sub = threadIdx.x % G;
     double part[4] = {0, 0, 0, 0};
-    if (k < d.n) {
-        T S = T(0);
-        if (d.smask[k] & d.groupbit) {
-            const int c = min(d.nb.count[k], d.nb.M);
-            const T rc2 = (T)d.rc2, qf = (T)d.qf;
-            const auto a = d.geo.load(k);
-            const T wk = d.w ? d.w[k] : T(1);
-            for (int t = 0; t < c; ++t) {
-                const int j = d.nb.list[(size_t)t * d.npad + k];
-                T dx, dy, dz;
-                d.geo.disp(a, d.geo.load(j), dx, dy, dz);
-                T gv, dg;
-                debye_g<T>(dx * dx + dy * dy + dz * dz, rc2, qf, gv, dg);
-                S += d.w ? wk * d.w[j] * gv : gv;
-            }
-            S += T(1);
-            part[0] = (double)S;
-            part[1] = sw_f<double>(d.sw, (double)S);
-            part[2] = 1.0;
+    const bool on = k < d.n && (d.smask[k] & d.groupbit);
+    T S = T(0);
+    if (on) {
+        const int c = min(d.nb.count[k], d.nb.M);
+        const T rc2 = (T)d.rc2, qf = (T)d.qf;
+        const auto a = d.geo.load(k);
+        const T wk = d.w ? d.w[k] : T(1);
+        for (int t = sub; t < c; t += G) {
+            const int j = d.nb.list[(size_t)t * d.npad + k];
+            T dx, dy, dz;
+            d.geo.disp(a, d.geo.load(j), dx, dy, dz);
+            T gv, dg;
+            debye_g<T>(dx * dx + dy * dy + dz * dz, rc2, qf, gv, dg);
+            S += d.w ? wk * d.w[j] * gv : gv;
         }
-        d.S[k] = S;
     }
+    if (G > 1) S = lanes_total<G>(S);
+    if (on) S += T(1);
+    if (on && sub == 0) {
+        part[0] = (double)S;
+        part[1] = sw_f<double>(d.sw, (double)S);
+        part[2] = 1.0;
+    }
+    if (k < d.n && sub == 0) d.S[k] = S;
     block_sum<4>(part, smem);
     if (threadIdx.x == 0)
         for (int t = 0; t < 4; ++t) d.partials[blockIdx.x * 8 + t] = part[t];
@@ -94,23 +96,23 @@ __device__ __forceinline__ T debye_a(const DebyeDev<T> &d, int k, double c0, dou
     return (T)a;
 }
 
-template <typename T>
+template <typename T, int G>
 __global__ void __launch_bounds__(kBlock) k_debye_force(DebyeDev<T> d, const double *__restrict__ f_src,
                                                         double *__restrict__ f_dst, SysDev s, CellGrid g,
                                                         double *vpart, DevStatus *status) {
     pdl_entry();
     __shared__ double smem[6 * 32];
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = blockIdx.x * (kBlock / G) + threadIdx.x / G, sub = threadIdx.x % G;
     double vir[6] = {0, 0, 0, 0, 0, 0};
     const double c0 = d.coef[0], c1 = d.coef[1];
+    T gx = T(0), gy = T(0), gz = T(0);
     if (k < d.n) {
         const T ak = debye_a<T>(d, k, c0, c1);
         const T rc2 = (T)d.rc2, qf = (T)d.qf;
-        T gx = T(0), gy = T(0), gz = T(0);
         const int c = min(d.nb.count[k], d.nb.M);
         const auto a = d.geo.load(k);
         const T wk = d.w ? d.w[k] : T(1);
-        for (int t = 0; t < c; ++t) {
+        for (int t = sub; t < c; t += G) {
             const int j = d.nb.list[(size_t)t * d.npad + k];
             T w = ak + debye_a<T>(d, j, c0, c1);
             if (d.w) w *= wk * d.w[j];
@@ -125,6 +127,13 @@ __global__ void __launch_bounds__(kBlock) k_debye_force(DebyeDev<T> d, const dou
             gy -= f * dy;
             gz -= f * dz;
         }
+    }
+    if (G > 1) {
+        gx = lanes_total<G>(gx);
+        gy = lanes_total<G>(gy);
+        gz = lanes_total<G>(gz);
+    }
+    if (k < d.n && sub == 0) {
         const int i = d.perm[k];
         const double fx = -(double)gx, fy = -(double)gy, fz = -(double)gz;
         if ((unsigned)i < (unsigned)d.n) {   // a sorted order left by a rebuild that gave up is not trusted
@@ -485,14 +494,18 @@ __global__ void __launch_bounds__(256, FP64 ? 2 : 4)
 template <typename T> void launch_debye_values(const DebyeDev<T> &d, cudaStream_t st) {
     if (d.n == 0) return;
     if (d.w) launch_k(k_chem_weights<T>, (d.n + kBlock - 1) / kBlock, kBlock, 0, st, d);
-    launch_k(k_debye_values<T>, (d.n + kBlock - 1) / kBlock, kBlock, 0, st, d);
+    const int ab = lanes_block(d.n), nb = (d.n + ab - 1) / ab;
+    if (ab < kBlock) launch_k(k_debye_values<T, kLanes>, nb, kBlock, 0, st, d);
+    else launch_k(k_debye_values<T, 1>, nb, kBlock, 0, st, d);
     prof_mark("debye_values", st);
 }
 template <typename T>
 void launch_debye_forces(const DebyeDev<T> &d, const double *f_src, double *f_dst, const SysDev &s, const CellGrid &g,
                          double *vpart, DevStatus *status, cudaStream_t st) {
     if (d.n == 0) return;
-    launch_k(k_debye_force<T>, (d.n + kBlock - 1) / kBlock, kBlock, 0, st, d, f_src, f_dst, s, g, vpart, status);
+    const int ab = lanes_block(d.n), nb = (d.n + ab - 1) / ab;
+    if (ab < kBlock) launch_k(k_debye_force<T, kLanes>, nb, kBlock, 0, st, d, f_src, f_dst, s, g, vpart, status);
+    else launch_k(k_debye_force<T, 1>, nb, kBlock, 0, st, d, f_src, f_dst, s, g, vpart, status);
     prof_mark("debye_force", st);
 }
 template void launch_debye_values<float>(const DebyeDev<float> &, cudaStream_t);
