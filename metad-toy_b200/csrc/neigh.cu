@@ -281,9 +281,12 @@ __global__ void __launch_bounds__(kBlock) k_neighbors_fast(CellGrid g, SysDev s,
 // smooth switch is evaluated for 32 candidates in range at a time.  With the
 // cap of STEINH Q the warp also ranks its list (k_select_cap), from shared
 // memory.
-// Event intervals, before and now: 4,000 atoms, cutoff 3.9 with the cap 58 us
-// (search 35, ranking 23) and 10; 32,000 atoms, cutoff 6.0 with the cap 101
-// and 50, without 54 and 33; 61,111 atoms, FERMI 125 and 60.
+// (A candidate's cell is found by a bit mask of the cells that begin in its
+// round; a binary search by shuffles cost 30 instructions more a round, 33 us
+// against 27 at 32,000 atoms.)  Event intervals, before and now: 4,000 atoms,
+// cutoff 3.9 with the cap 58 us (search 35, ranking 23) and 10; 32,000 atoms,
+// cutoff 6.0 with the cap 101 and 37, without 54 and 27; 61,111 atoms, FERMI
+// 125 and 53.
 constexpr int kWarpAtoms = kBlock / 32;
 template <int KIND, bool CAP>
 __global__ void __launch_bounds__(kBlock) k_neighbors_warp(CellGrid g, SysDev s, NeighSpec ns, NeighDev nd,
@@ -291,6 +294,7 @@ __global__ void __launch_bounds__(kBlock) k_neighbors_warp(CellGrid g, SysDev s,
     pdl_entry();
     __shared__ int held[CAP || KIND == NK_SWITCH ? kWarpAtoms : 1][kMaxCapList];
     __shared__ float held_r2[KIND == NK_SWITCH ? kWarpAtoms : 1][kMaxCapList];
+    __shared__ float4 cells[kWarpAtoms][27];
     if (gate_closed(s.skin)) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = blockIdx.x * kWarpAtoms + warp;
     if (k >= s.n) return;   // whole warps; no block-wide synchronisation below
@@ -326,7 +330,13 @@ __global__ void __launch_bounds__(kBlock) k_neighbors_warp(CellGrid g, SysDev s,
         if (lane >= o) end += v;
     }
     const int begin = end - len, total = __shfl_sync(all, end, 31);
-    int cnt = 0, wait = 0;
+    // the non-empty cells in order: where candidate t lies (first - begin + t), the cell's shift
+    const unsigned full = __ballot_sync(all, len > 0);
+    if (len > 0)
+        cells[warp][__popc(full & below)] = make_float4(__int_as_float(first - begin), (float)ox * g.hf[0] - a.x,
+                                                        (float)oy * g.hf[1] - a.y, (float)oz * g.hf[2] - a.z);
+    __syncwarp();
+    int cnt = 0, wait = 0, opened = -1;   // opened: the last cell begun before this round
     auto keep = [&](bool in, int j) {
         const unsigned hits = __ballot_sync(all, in);
         const int at = cnt + __popc(hits & below);
@@ -345,19 +355,14 @@ __global__ void __launch_bounds__(kBlock) k_neighbors_warp(CellGrid g, SysDev s,
     };
     for (int t0 = 0; t0 < total; t0 += 32) {
         const int t = t0 + lane;
-        int c = 0;   // the last cell that begins at or before t
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const int v = __shfl_sync(all, begin, c + o);
-            if (c + o < 27 && v <= t) c += o;
-        }
-        const int j = __shfl_sync(all, first, c) + t - __shfl_sync(all, begin, c);
+        const unsigned starts = __reduce_or_sync(all, len > 0 && (unsigned)(begin - t0) < 32u ? 1u << (begin - t0) : 0u);
+        const float4 c = cells[warp][opened + __popc(starts & (below | 1u << lane))];
+        opened += __popc(starts);
+        const int j = __float_as_int(c.x) + t;
         float r2f = INFINITY;
         if (t < total && j != k) {
             const float4 b = __ldg(s.pf + j);
-            const float dx = b.x + ((float)(c / 9 - 1) * g.hf[0] - a.x);
-            const float dy = b.y + ((float)(c / 3 % 3 - 1) * g.hf[1] - a.y);
-            const float dz = b.z + ((float)(c % 3 - 1) * g.hf[2] - a.z);
+            const float dx = b.x + c.y, dy = b.y + c.z, dz = b.z + c.w;
             r2f = dx * dx + dy * dy + dz * dz;
         }
         if (KIND != NK_SWITCH) {
@@ -408,11 +413,19 @@ __global__ void __launch_bounds__(kBlock) k_neighbors_warp(CellGrid g, SysDev s,
             id[e] = s.perm[jj[e]];
         }
     }
-    for (int u = 0; u < c; ++u) {
-        const double ru = __shfl_sync(all, u < 32 ? r2[0] : r2[1], u);
-        const int iu = __shfl_sync(all, u < 32 ? id[0] : id[1], u);
+    if (c <= 32) {
+        for (int u = 0; u < c; ++u) {
+            const double ru = __shfl_sync(all, r2[0], u);
+            const int iu = __shfl_sync(all, id[0], u);
+            rank[0] += ru < r2[0] || (ru == r2[0] && iu < id[0]);
+        }
+    } else {
+        for (int u = 0; u < c; ++u) {
+            const double ru = __shfl_sync(all, u < 32 ? r2[0] : r2[1], u);
+            const int iu = __shfl_sync(all, u < 32 ? id[0] : id[1], u);
 #pragma unroll
-        for (int e = 0; e < 2; ++e) rank[e] += ru < r2[e] || (ru == r2[e] && iu < id[e]);
+            for (int e = 0; e < 2; ++e) rank[e] += ru < r2[e] || (ru == r2[e] && iu < id[e]);
+        }
     }
     double kr2 = CUDART_INF;
     int kid = 0x7fffffff;
@@ -766,8 +779,8 @@ int launch_build_cells(const CellGrid &g, SysDev &s, cudaStream_t st) {
 // One warp per atom up to 65,536 atoms, 131,072 for a smooth switch: there a
 // thread per atom has the warps to hide its loads and runs fewer instructions
 // (STEP at 64,000 atoms 38 us and 29 with a warp per atom, at 100,000 39 and
-// 41, at 200,000 68 and 74; cutoff 6.0 at 32,000 54 and 33, at 87,000 57 and
-// 76; FERMI at 64,000 110 and 62).
+// 41, at 200,000 68 and 74; cutoff 6.0 at 32,000 54 and 27, at 87,000 57 and
+// 60; FERMI at 64,000 110 and 55).
 constexpr int kWarpMax = 65536;
 
 int launch_neighbors(const CellGrid &g, const SysDev &s, const NeighSpec &ns, NeighDev nd, DevStatus *status,
