@@ -882,13 +882,10 @@ mtd_status enqueue_forces(mtd_ctx *c, long long step, const double *x, const int
     if (c->fp64) run_forces<double>(c, c->last_sys, c->last_grid, x, mask, fin, fout, virial);
     else run_forces<float>(c, c->last_sys, c->last_grid, x, mask, fin, fout, virial);
     MTD_CU(cudaGetLastError(), "kernel launch");
-    // outputs of this step into pinned host memory
+    // outputs of this step into pinned host memory, in one copy (616 bytes)
     const int slot = c->ring ? c->slot_next : 0;
     use_slot(c, slot);
-    MTD_CU(cudaMemcpyAsync(c->h_out, c->d_out, sizeof(double) * 64, cudaMemcpyDeviceToHost, c->st), "outputs");
-    MTD_CU(cudaMemcpyAsync(c->h_status, c->d_status, sizeof(DevStatus), cudaMemcpyDeviceToHost, c->st), "status");
-    MTD_CU(cudaMemcpyAsync(c->h_nhills, c->d_nhills, sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->st), "hills");
-    if (virial) MTD_CU(cudaMemcpyAsync(c->h_vir, c->d_vir, sizeof(double) * 6, cudaMemcpyDeviceToHost, c->st), "virial");
+    MTD_CU(cudaMemcpyAsync(&c->h_slots[slot], c->d_slot, sizeof(OutSlot), cudaMemcpyDeviceToHost, c->st), "outputs");
     if (c->ring) {
         MTD_CU(cudaEventRecord(c->slot_ev[slot], c->st), "outputs");
         c->fifo.push_back(PendingOut{slot, step, virial});
@@ -1181,14 +1178,15 @@ mtd_status mtd_create(int narg, const char *const *arg, const mtd_options *opt, 
     if (s == MTD_OK) {
         cudaError_t ce = cudaSuccess;
         ce = dalloc(&c->d_plan, sizeof(BiasPlan));
-        if (ce == cudaSuccess) ce = dalloc(&c->d_out, sizeof(double) * 64);
-        if (ce == cudaSuccess) ce = dalloc(&c->d_status, sizeof(DevStatus));
+        if (ce == cudaSuccess) ce = dalloc(&c->d_slot, sizeof(OutSlot));
         if (ce == cudaSuccess) ce = dalloc(&c->d_hills, sizeof(HillRec) * kHillCap);
-        if (ce == cudaSuccess) ce = dalloc(&c->d_nhills, sizeof(unsigned long long));
-        if (ce == cudaSuccess) ce = dalloc(&c->d_vir, sizeof(double) * 8);
-        if (ce == cudaSuccess) ce = cudaMemset(c->d_out, 0, sizeof(double) * 64);
-        if (ce == cudaSuccess) ce = cudaMemset(c->d_status, 0, sizeof(DevStatus));
-        if (ce == cudaSuccess) ce = cudaMemset(c->d_nhills, 0, sizeof(unsigned long long));
+        if (ce == cudaSuccess) ce = cudaMemset(c->d_slot, 0, sizeof(OutSlot));
+        if (ce == cudaSuccess) {
+            c->d_out = c->d_slot->out;
+            c->d_status = &c->d_slot->status;
+            c->d_nhills = &c->d_slot->nhills;
+            c->d_vir = c->d_slot->vir;
+        }
         if (ce == cudaSuccess) ce = cudaMallocHost((void **)&c->h_slots, sizeof(OutSlot) * kOutSlots);
         if (ce == cudaSuccess) {
             std::memset(c->h_slots, 0, sizeof(OutSlot) * kOutSlots);
@@ -1221,8 +1219,7 @@ void mtd_destroy(mtd_ctx *c) {
     dfree(c->d_x); dfree(c->d_fin); dfree(c->d_fout); dfree(c->d_mask); dfree(c->d_image);
     dfree(c->cellof); dfree(c->slot); dfree(c->perm); dfree(c->iperm); dfree(c->smask); dfree(c->arrival);
     dfree(c->xs); dfree(c->pf); dfree(c->count); dfree(c->start); dfree(c->d_vpart);
-    dfree(c->d_plan); dfree(c->d_grid); dfree(c->d_hills); dfree(c->d_nhills); dfree(c->d_out);
-    dfree(c->d_status); dfree(c->d_vir);
+    dfree(c->d_plan); dfree(c->d_grid); dfree(c->d_hills); dfree(c->d_slot);
     if (c->h_slots) cudaFreeHost(c->h_slots);
     for (int k = 0; k < kOutSlots; ++k)
         if (c->slot_ev[k]) cudaEventDestroy(c->slot_ev[k]);

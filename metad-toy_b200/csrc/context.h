@@ -142,6 +142,7 @@ struct mtd_ctx {
     double *d_grid = nullptr;
     long long grid_size = 0;
     HillRec *d_hills = nullptr;
+    OutSlot *d_slot = nullptr;           // a step's outputs on the device; the four below point into it
     unsigned long long *d_nhills = nullptr;
     double *d_out = nullptr;
     DevStatus *d_status = nullptr;
