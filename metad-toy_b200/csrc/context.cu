@@ -192,14 +192,17 @@ mtd_status alloc_env(mtd_ctx *c, Env &e, int npad) {
 
 // Atoms per block of a unit's passes, and so per row of its partial sums and
 // virial partials.
-static int unit_block(const Unit &u, int n) {
-    return u.kind == CAL_STEINH_Q || u.kind == CAL_STRU_FACTOR ? lanes_block(n) : kBlock;
+// (STEINH L of a walker keeps a thread per atom, as the one-launch step of all
+// walkers has it: the two give the same results bit for bit.)
+static int unit_block(const mtd_ctx *c, const Unit &u) {
+    if (u.kind == CAL_STRU_FACTOR) return lanes_block(c->n, kLaneAtomsSf);
+    return u.kind == CAL_STEINH_Q || c->ring ? lanes_block(c->n) : kBlock;
 }
 
 mtd_status alloc_unit(mtd_ctx *c, Unit &u, int npad) {
     const size_t R = real_size(c);
     const int SQ = record_stride(c, u);
-    const int nb = std::max((npad + kBlock - 1) / kBlock, (std::min(npad, kLaneAtoms) * kLanes + kBlock - 1) / kBlock);
+    const int nb = std::max((npad + kBlock - 1) / kBlock, (std::min(npad, kLaneAtomsSf) * kLanes + kBlock - 1) / kBlock);
     void **arrs[] = {&u.q, &u.nf, &u.lq, &u.lqs, &u.e12, &u.lam, &u.g, &u.tu, &u.Q, &u.S, &u.w};
     for (void **a : arrs) dfree(*a);
     dfree(u.partials);
@@ -380,7 +383,7 @@ void build_plan(mtd_ctx *c) {
             Q.sk_n = U.skn;
         } else {
             Q.partials = U.partials;
-            Q.nparts = (c->n + unit_block(U, c->n) - 1) / unit_block(U, c->n);
+            Q.nparts = (c->n + unit_block(c, U) - 1) / unit_block(c, U);
             Q.pstride = 8;
             Q.nvals = U.kind == CAL_STEINH_L ? 5 : 4;
             Q.rho = nullptr;
@@ -595,6 +598,7 @@ template <typename T> LocalDev<T> local_dev(mtd_ctx *c, Unit &u, const CellGrid 
     d.lam = (T *)u.lam; d.g = (T *)u.g; d.tu = (T *)u.tu; d.partials = u.partials; d.coef = u.coef;
     d.qblock = c->tune_q;
     d.lblock = c->tune_l;
+    d.lanes = unit_block(c, u) < kBlock;
     d.qsplit = c->tune_qsplit;
     return d;
 }
@@ -705,7 +709,7 @@ void run_forces(mtd_ctx *c, const SysDev &s, const CellGrid &g, const double *x,
         if (!u.used) continue;
         const double *src = first ? fin : fout;
         double *vp = virial ? c->d_vpart + (size_t)voff * 8 : nullptr;
-        const int nb = (c->n + unit_block(u, c->n) - 1) / unit_block(u, c->n);
+        const int nb = (c->n + unit_block(c, u) - 1) / unit_block(c, u);
         if (u.kind == CAL_STEINH_L) {
             launch_local_forces<T>(local_dev<T>(c, u, g), src, fout, s, g, vp, c->d_status, st);
             c->launches += 2;

@@ -229,6 +229,26 @@ int rebuild_blocks();
 cudaError_t launch_rebuild(const CellGrid &g, const SysDev &s, const NeighSpec &ns, NeighDev cd, DevStatus *status,
                            GridBar *bar, int limit, int stall, cudaStream_t st);
 
+// Lanes per atom of the STEINH L, STEINH Q and STRU_FACTOR passes: eight while a
+// thread per atom would leave most of the GPU without work (16,384 atoms are 64
+// blocks), each lane taking every eighth neighbour.  A block then holds 32
+// atoms instead of 256, and so do its partial sums.  The lines lie where three
+// contexts stepped in turn are as fast either way (us a step, lanes and thread
+// per atom; a step alone gains up to twice the atoms): local Q4 + Q6 in mixed
+// precision 20.9 and 26.4 at 4,000, 32.7 and 34.1 at 16,000, 52.9 and 46.5 at
+// 32,000 (FERMI 28.9 and 52.4, 56.0 and 68.8, 96.5 and 93.7); Q4 with cutoff 6
+// 25.9 and 37.4 at 6,900, 42.6 and 45.8 at 16,384, 72.9 and 60.8 at 32,000;
+// Debye 29.3 and 40.5 at 16,384, 49.0 and 49.4 at 32,000, 85 and 79 at 62,500.
+constexpr int kLaneAtoms = 16384, kLaneAtomsSf = 32768;
+constexpr int kLanes = 8;
+inline int lanes_block(int n, int most = kLaneAtoms) { return n <= most ? kBlock / kLanes : kBlock; }
+// Sum over the G lanes of an atom (G neighbouring lanes, all in the warp).
+template <int G, typename T> __device__ __forceinline__ T lanes_total(T v) {
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
 // ------------------------------------------------------------------ STEINH L
 template <typename T> struct LocalDev {
     int n, npad, SQ;
@@ -243,6 +263,7 @@ template <typename T> struct LocalDev {
     double *partials;           // [nblocks][8]: S1A S0A S1B S0B N
     const double *coef;         // c1A c2A c1B c2B (written by the bias kernel)
     int qblock, lblock;         // threads per block of the q and lambda passes (0: kBlock); same results
+    int lanes;                  // kLanes lanes per atom instead of one thread
     // skin lists: the q pass first filters this unit's candidates into nb (filter != 0),
     // in one loop with the sum (qsplit 0) or in a filter loop before it (qsplit 1)
     int filter, qsplit;
@@ -271,23 +292,6 @@ void launch_local_force_pass(const LocalDev<T> &d, const double *f_src, double *
                              const CellGrid &g, double *vpart, DevStatus *status, cudaStream_t st);
 
 // ------------------------------------------------------------------ STEINH Q
-// Lanes per atom of the STEINH Q and STRU_FACTOR passes: eight while a thread
-// per atom would leave most of the GPU without work (65,536 atoms are 256
-// blocks, 14 warps an SM), each lane taking every eighth neighbour.  A block
-// then holds 32 atoms instead of 256, and so do its partial sums.  Event
-// intervals at 32,000 atoms: Q4 values 22.7 us and 15.6 with the lanes, forces
-// 47 and 41, Debye values 26.6 and 13.7, forces 42 and 22; at 4,000 (Q6, FP64)
-// 16.6 and 9.7, 37 and 14.
-constexpr int kLaneAtoms = 65536;
-constexpr int kLanes = 8;
-inline int lanes_block(int n) { return n <= kLaneAtoms ? kBlock / kLanes : kBlock; }
-// Sum over the G lanes of an atom (G neighbouring lanes, all in the warp).
-template <int G, typename T> __device__ __forceinline__ T lanes_total(T v) {
-#pragma unroll
-    for (int o = 1; o < G; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 template <typename T> struct GlobalDev {
     int n, npad, SQ, L;
     int groupbit, nsw;

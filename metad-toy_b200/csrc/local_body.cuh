@@ -341,7 +341,7 @@ __device__ __forceinline__ void add_g(T *acc, const T *lq, T w, T s) {
 }
 
 // A CV switch whose derivative is identically zero (e2 = 0 for every atom).
-__device__ __forceinline__ bool sw_flat(const SwParams &p) { return p.type == SW_LINE || p.type == SW_STEP; }
+__host__ __device__ __forceinline__ bool sw_flat(const SwParams &p) { return p.type == SW_LINE || p.type == SW_STEP; }
 
 // Pass 3 for a step pair switch and flat CV switches: with e2 = 0 the weight
 // of an order is c1 e1, so lam_k = c1 / NF_k * (e1_k LQ_k + sum_j s_kj e1_j
@@ -475,6 +475,85 @@ __device__ __forceinline__ void local_lambda_body(const LocalDev<T> &d, int bid,
     store_rec(d.lam + (size_t)k * S::SQ, lam);
 }
 
+// dCV/dx of sorted atom k, less its sign: the terms of neighbours t0, t0 + dt, ....
+template <int LA, int LB, typename T, bool STEP>
+__device__ __forceinline__ void local_force_sum(const LocalDev<T> &d, int k, int t0, int dt, T &gx, T &gy, T &gz) {
+    using S = LSet<LA, LB, T>;
+    constexpr bool DSIG = !STEP;
+    T la[S::SQ];
+    load_rec(d.lam + (size_t)k * S::SQ, la);
+    T qa[S::SQ], ga[S::SQ];
+    T tua[4] = {T(0), T(0), T(0), T(0)};
+    if constexpr (DSIG) {
+        load_rec(d.q + (size_t)k * S::SQ, qa);
+        load_rec(d.g + (size_t)k * S::SQ, ga);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) tua[t] = d.tu[4 * k + t];
+    }
+    const auto a = d.geo.load(k);
+    const int c = min(d.nb.count[k], d.nb.M);
+    constexpr T sgnA = (LA & 1) ? T(-1) : T(1);
+    constexpr T sgnB = (LB & 1) ? T(-1) : T(1);
+    // each neighbour's index is loaded an iteration ahead, so its record
+    // load waits on one memory latency instead of two
+    int jn = t0 < c ? nb_index(d.nb, d.npad, t0, k) : 0;
+    for (int t = t0; t < c; t += dt) {
+        const int j = jn;
+        if (t + dt < c) jn = nb_index(d.nb, d.npad, t + dt, k);
+        T ux, uy, uz, rinv, sg, dsg;
+        pair_geom<T, STEP>(d, a, j, ux, uy, uz, rinv, sg, dsg);
+        T lj[S::SQ];
+        load_rec32(d.lam + (size_t)j * S::SQ, lj);
+        T Lm[S::SQ];
+#pragma unroll
+        for (int q = 0; q < S::SA; ++q) Lm[q] = la[q] + sgnA * lj[q];
+#pragma unroll
+        for (int q = S::SA; q < S::SQ; ++q) Lm[q] = la[q] + sgnB * lj[q];
+        T ax, ay, az;
+        const T sA = ylm_dot_grad<LA, T>(ux, uy, uz, rinv, Lm, ax, ay, az);
+        gx -= sg * ax;
+        gy -= sg * ay;
+        gz -= sg * az;
+        T sB = T(0);
+        if constexpr (LB > 0) {
+            T bx, by, bz;
+            sB = ylm_dot_grad<LB, T>(ux, uy, uz, rinv, Lm + S::SA, bx, by, bz);
+            gx -= sg * bx;
+            gy -= sg * by;
+            gz -= sg * bz;
+        }
+        if constexpr (DSIG) {
+            if (dsg != T(0)) {
+                T qj[S::SQ], gj[S::SQ];
+                load_rec(d.q + (size_t)j * S::SQ, qj);
+                load_rec(d.g + (size_t)j * S::SQ, gj);
+                T cross = sA + sB - tua[0] - tua[1] - tua[2] - tua[3] - d.tu[4 * j] - d.tu[4 * j + 1] -
+                          d.tu[4 * j + 2] - d.tu[4 * j + 3];
+#pragma unroll
+                for (int q = 0; q < S::SA + S::SB; ++q) cross += ga[q] * qj[q] + gj[q] * qa[q];
+                gx -= dsg * cross * ux;
+                gy -= dsg * cross * uy;
+                gz -= dsg * cross * uz;
+            }
+        }
+    }
+}
+
+// Virial terms of a force on sorted atom k, caller index i (unwrapped coordinates).
+__device__ __forceinline__ void force_virial(const SysDev &s, const CellGrid &g, int k, int i, double fx, double fy,
+                                             double fz, double (&vir)[6]) {
+    double ux = s.xs[3 * k], uy = s.xs[3 * k + 1], uz = s.xs[3 * k + 2];
+    if (s.image) {
+        int ix, iy, iz;
+        unpack_image(s.image[i], ix, iy, iz);
+        ux += ix * g.L[0];
+        uy += iy * g.L[1];
+        uz += iz * g.L[2];
+    }
+    vir[0] = fx * ux; vir[1] = fy * uy; vir[2] = fz * uz;
+    vir[3] = fx * uy; vir[4] = fx * uz; vir[5] = fy * uz;
+}
+
 // Pass 4: gather forces, f_dst = f_src - dV/dx, plus the virial block partials.
 // One thread per sorted slot, or (d.iperm set) per caller index of d.i0 ..
 // d.i1 - 1, so a caller-order range of f is complete when its launch is.
@@ -483,7 +562,6 @@ __device__ __forceinline__ void local_force_body(const LocalDev<T> &d, const dou
                                                  double *__restrict__ f_dst, const SysDev &s, const CellGrid &g,
                                                  double *vpart, DevStatus *status, int bid) {
     using S = LSet<LA, LB, T>;
-    constexpr bool DSIG = !STEP;
     __shared__ double smem[6 * 32];
     // caller order: the block's stretch of f (3 x blockDim doubles, which
     // may be host memory over the host link) is read into shared memory and
@@ -507,64 +585,8 @@ __device__ __forceinline__ void local_force_body(const LocalDev<T> &d, const dou
     }
     double vir[6] = {0, 0, 0, 0, 0, 0};
     if (valid) {
-        T la[S::SQ];
-        load_rec(d.lam + (size_t)k * S::SQ, la);
-        T qa[S::SQ], ga[S::SQ];
-        T tua[4] = {T(0), T(0), T(0), T(0)};
-        if constexpr (DSIG) {
-            load_rec(d.q + (size_t)k * S::SQ, qa);
-            load_rec(d.g + (size_t)k * S::SQ, ga);
-#pragma unroll
-            for (int t = 0; t < 4; ++t) tua[t] = d.tu[4 * k + t];
-        }
-        const auto a = d.geo.load(k);
         T gx = T(0), gy = T(0), gz = T(0);
-        const int c = min(d.nb.count[k], d.nb.M);
-        constexpr T sgnA = (LA & 1) ? T(-1) : T(1);
-        constexpr T sgnB = (LB & 1) ? T(-1) : T(1);
-        // each neighbour's index is loaded an iteration ahead, so its record
-        // load waits on one memory latency instead of two
-        int jn = c > 0 ? nb_index(d.nb, d.npad, 0, k) : 0;
-        for (int t = 0; t < c; ++t) {
-            const int j = jn;
-            if (t + 1 < c) jn = nb_index(d.nb, d.npad, t + 1, k);
-            T ux, uy, uz, rinv, sg, dsg;
-            pair_geom<T, STEP>(d, a, j, ux, uy, uz, rinv, sg, dsg);
-            T lj[S::SQ];
-            load_rec32(d.lam + (size_t)j * S::SQ, lj);
-            T Lm[S::SQ];
-#pragma unroll
-            for (int q = 0; q < S::SA; ++q) Lm[q] = la[q] + sgnA * lj[q];
-#pragma unroll
-            for (int q = S::SA; q < S::SQ; ++q) Lm[q] = la[q] + sgnB * lj[q];
-            T ax, ay, az;
-            const T sA = ylm_dot_grad<LA, T>(ux, uy, uz, rinv, Lm, ax, ay, az);
-            gx -= sg * ax;
-            gy -= sg * ay;
-            gz -= sg * az;
-            T sB = T(0);
-            if constexpr (LB > 0) {
-                T bx, by, bz;
-                sB = ylm_dot_grad<LB, T>(ux, uy, uz, rinv, Lm + S::SA, bx, by, bz);
-                gx -= sg * bx;
-                gy -= sg * by;
-                gz -= sg * bz;
-            }
-            if constexpr (DSIG) {
-                if (dsg != T(0)) {
-                    T qj[S::SQ], gj[S::SQ];
-                    load_rec(d.q + (size_t)j * S::SQ, qj);
-                    load_rec(d.g + (size_t)j * S::SQ, gj);
-                    T cross = sA + sB - tua[0] - tua[1] - tua[2] - tua[3] - d.tu[4 * j] - d.tu[4 * j + 1] -
-                              d.tu[4 * j + 2] - d.tu[4 * j + 3];
-#pragma unroll
-                    for (int q = 0; q < S::SA + S::SB; ++q) cross += ga[q] * qj[q] + gj[q] * qa[q];
-                    gx -= dsg * cross * ux;
-                    gy -= dsg * cross * uy;
-                    gz -= dsg * cross * uz;
-                }
-            }
-        }
+        local_force_sum<LA, LB, T, STEP>(d, k, 0, 1, gx, gy, gz);
         const int i = CALLER ? ic : d.perm[k];
         const double fx = -(double)gx, fy = -(double)gy, fz = -(double)gz;   // delta f = -dV/dx
         if constexpr (CALLER) {
@@ -578,16 +600,7 @@ __device__ __forceinline__ void local_force_body(const LocalDev<T> &d, const dou
         }
         if (!(isfinite(fx) && isfinite(fy) && isfinite(fz))) atomicOr(&status->nan_force, 1u);
         if (vpart && (unsigned)i < (unsigned)d.n) {
-            double ux_ = s.xs[3 * k], uy_ = s.xs[3 * k + 1], uz_ = s.xs[3 * k + 2];
-            if (s.image) {
-                int ix, iy, iz;
-                unpack_image(s.image[i], ix, iy, iz);
-                ux_ += ix * g.L[0];
-                uy_ += iy * g.L[1];
-                uz_ += iz * g.L[2];
-            }
-            vir[0] = fx * ux_; vir[1] = fy * uy_; vir[2] = fz * uz_;
-            vir[3] = fx * uy_; vir[4] = fx * uz_; vir[5] = fy * uz_;
+            force_virial(s, g, k, i, fx, fy, fz, vir);
         }
     }
     if constexpr (CALLER) {

@@ -20,21 +20,24 @@
 // (Q4 and Q6 of one neighbour environment) are fused in one pass.  With a STEP
 // switch sigma = 1 and sigma' = 0 on every listed pair, so the LQ and lambda
 // passes need neighbour indices only.
-#include "local_body.cuh"
+#include "local_lanes.cuh"
 
 namespace mtd {
 
 namespace {
 
-// The passes as kernels (local_body.cuh).
+// The passes as kernels (local_body.cuh).  FP64 records and smooth switches
+// need more than the 64 registers of four blocks an SM: held to them, the
+// spills cost FERMI forces 98 us against 70 at 61,111 atoms, FP64 LQ at 100,000
+// atoms 61 against 45 (two blocks).
 template <int LA, int LB, typename T, bool STEP, bool FILTER, bool MERGED = true>
-__global__ void __launch_bounds__(kBlock, 4) k_local_q(LocalDev<T> d) {
+__global__ void __launch_bounds__(kBlock, sizeof(T) == 8 && STEP ? 2 : 4) k_local_q(LocalDev<T> d) {
     pdl_entry();
     local_q_body<LA, LB, T, STEP, FILTER, MERGED>(d, blockIdx.x);
 }
 
 template <int LA, int LB, typename T, bool STEP>
-__global__ void __launch_bounds__(kBlock, 4) k_local_lq(LocalDev<T> d) {
+__global__ void __launch_bounds__(kBlock, sizeof(T) == 8 ? 2 : 4) k_local_lq(LocalDev<T> d) {
     pdl_entry();
     local_lq_body<LA, LB, T, STEP>(d, blockIdx.x);
 }
@@ -45,14 +48,81 @@ __global__ void __launch_bounds__(kBlock) k_local_lambda(LocalDev<T> d) {
 }
 
 template <int LA, int LB, typename T, bool STEP, bool CALLER = false>
-__global__ void __launch_bounds__(kBlock, CALLER ? 2 : 4) k_local_force(LocalDev<T> d, const double *__restrict__ f_src,
+__global__ void __launch_bounds__(kBlock, CALLER || !STEP || sizeof(T) == 8 ? 2 : 4) k_local_force(LocalDev<T> d, const double *__restrict__ f_src,
                                                         double *__restrict__ f_dst, SysDev s, CellGrid g,
                                                         double *vpart, DevStatus *status) {
     pdl_entry();
     local_force_body<LA, LB, T, STEP, CALLER>(d, f_src, f_dst, s, g, vpart, status, blockIdx.x);
 }
 
+// The same with kLanes lanes per atom (local_lanes.cuh).
+template <int LA, int LB, typename T, bool STEP> __global__ void __launch_bounds__(kBlock) k_lanes_q(LocalDev<T> d) {
+    pdl_entry();
+    local_q_lanes<LA, LB, T, STEP>(d);
+}
+template <int LA, int LB, typename T, bool STEP> __global__ void __launch_bounds__(kBlock) k_lanes_lq(LocalDev<T> d) {
+    pdl_entry();
+    local_lq_lanes<LA, LB, T, STEP>(d);
+}
+template <int LA, int LB, typename T, bool STEP, bool FLAT>
+__global__ void __launch_bounds__(kBlock) k_lanes_lambda(LocalDev<T> d) {
+    local_lambda_lanes<LA, LB, T, STEP, FLAT>(d);   // places the wait
+}
+template <int LA, int LB, typename T, bool STEP, bool CALLER>
+__global__ void __launch_bounds__(kBlock, 2) k_lanes_force(LocalDev<T> d, const double *__restrict__ f_src,
+                                                           double *__restrict__ f_dst, SysDev s, CellGrid g,
+                                                           double *vpart, DevStatus *status) {
+    pdl_entry();
+    local_force_lanes<LA, LB, T, STEP, CALLER>(d, f_src, f_dst, s, g, vpart, status);
+}
+
+template <int LA, int LB, typename T, bool STEP> void run_values_lanes(const LocalDev<T> &d, cudaStream_t st) {
+    constexpr int ab = kBlock / kLanes;
+    const int nb = (d.n + ab - 1) / ab;
+    const int qb = d.qblock > 0 ? d.qblock : kBlock, qg = (d.n + qb - 1) / qb;
+    // skin lists: the filter stays with a thread per atom
+    if (d.filter && d.qsplit) launch_k(k_local_q<LA, LB, T, STEP, true, false>, qg, qb, 0, st, d);
+    else if (d.filter) launch_k(k_local_q<LA, LB, T, STEP, true>, qg, qb, 0, st, d);
+    else launch_k(k_lanes_q<LA, LB, T, STEP>, nb, kBlock, 0, st, d);
+    prof_mark("local_q", st);
+    launch_k(k_lanes_lq<LA, LB, T, STEP>, nb, kBlock, 0, st, d);
+    prof_mark("local_lq", st);
+}
+
+template <int LA, int LB, typename T> void run_lambda_lanes(const LocalDev<T> &d, cudaStream_t st) {
+    constexpr int ab = kBlock / kLanes;
+    const int nb = (d.n + ab - 1) / ab;
+    if (d.sw_r.type != SW_STEP) launch_k(k_lanes_lambda<LA, LB, T, false, false>, nb, kBlock, 0, st, d);
+    else if (sw_flat(d.sw_cvA) && (LB == 0 || sw_flat(d.sw_cvB)))
+        launch_k(k_lanes_lambda<LA, LB, T, true, true>, nb, kBlock, 0, st, d);
+    else launch_k(k_lanes_lambda<LA, LB, T, true, false>, nb, kBlock, 0, st, d);
+    prof_mark("local_lambda", st);
+}
+
+template <int LA, int LB, typename T>
+void run_force_lanes(const LocalDev<T> &d, const double *f_src, double *f_dst, const SysDev &s, const CellGrid &g,
+                     double *vpart, DevStatus *status, cudaStream_t st) {
+    constexpr int ab = kBlock / kLanes;
+    const int cnt = d.iperm ? d.i1 - d.i0 : d.n, nb = (cnt + ab - 1) / ab;
+    if (cnt <= 0) return;
+    const bool step = d.sw_r.type == SW_STEP;
+    if (d.iperm) {
+        if (step) launch_k(k_lanes_force<LA, LB, T, true, true>, nb, kBlock, 0, st, d, f_src, f_dst, s, g, vpart, status);
+        else launch_k(k_lanes_force<LA, LB, T, false, true>, nb, kBlock, 0, st, d, f_src, f_dst, s, g, vpart, status);
+    } else if (step) {
+        launch_k(k_lanes_force<LA, LB, T, true, false>, nb, kBlock, 0, st, d, f_src, f_dst, s, g, vpart, status);
+    } else {
+        launch_k(k_lanes_force<LA, LB, T, false, false>, nb, kBlock, 0, st, d, f_src, f_dst, s, g, vpart, status);
+    }
+    prof_mark("local_force", st);
+}
+
 template <int LA, int LB, typename T> void run_values(const LocalDev<T> &d, cudaStream_t st) {
+    if (d.lanes) {
+        if (d.sw_r.type == SW_STEP) run_values_lanes<LA, LB, T, true>(d, st);
+        else run_values_lanes<LA, LB, T, false>(d, st);
+        return;
+    }
     const int nb = (d.n + kBlock - 1) / kBlock;
     const int qb = d.qblock > 0 ? d.qblock : kBlock, qg = (d.n + qb - 1) / qb;   // no block reduction in q
     if (d.sw_r.type == SW_STEP) {
@@ -73,6 +143,7 @@ template <int LA, int LB, typename T> void run_values(const LocalDev<T> &d, cuda
 }
 
 template <int LA, int LB, typename T> void run_lambda(const LocalDev<T> &d, cudaStream_t st) {
+    if (d.lanes) return run_lambda_lanes<LA, LB, T>(d, st);
     const int lb = d.lblock > 0 ? d.lblock : kBlock, lg = (d.n + lb - 1) / lb;
     if (d.sw_r.type == SW_STEP) launch_k(k_local_lambda<LA, LB, T, true>, lg, lb, 0, st, d);
     else launch_k(k_local_lambda<LA, LB, T, false>, lg, lb, 0, st, d);
@@ -82,6 +153,7 @@ template <int LA, int LB, typename T> void run_lambda(const LocalDev<T> &d, cuda
 template <int LA, int LB, typename T>
 void run_force_pass(const LocalDev<T> &d, const double *f_src, double *f_dst, const SysDev &s, const CellGrid &g,
                     double *vpart, DevStatus *status, cudaStream_t st) {
+    if (d.lanes) return run_force_lanes<LA, LB, T>(d, f_src, f_dst, s, g, vpart, status, st);
     const int cnt = d.iperm ? d.i1 - d.i0 : d.n;
     if (cnt <= 0) return;
     const int nb = (cnt + kBlock - 1) / kBlock;
@@ -101,19 +173,8 @@ void run_force_pass(const LocalDev<T> &d, const double *f_src, double *f_dst, co
 template <int LA, int LB, typename T>
 void run_forces(const LocalDev<T> &d, const double *f_src, double *f_dst, const SysDev &s, const CellGrid &g,
                 double *vpart, DevStatus *status, cudaStream_t st) {
-    const int nb = (d.n + kBlock - 1) / kBlock;
-    const int lb = d.lblock > 0 ? d.lblock : kBlock, lg = (d.n + lb - 1) / lb;   // no block reduction in lambda
-    if (d.sw_r.type == SW_STEP) {
-        launch_k(k_local_lambda<LA, LB, T, true>, lg, lb, 0, st, d);
-        prof_mark("local_lambda", st);
-        launch_k(k_local_force<LA, LB, T, true>, nb, kBlock, 0, st, d, f_src, f_dst, s, g, vpart, status);
-        prof_mark("local_force", st);
-    } else {
-        launch_k(k_local_lambda<LA, LB, T, false>, lg, lb, 0, st, d);
-        prof_mark("local_lambda", st);
-        launch_k(k_local_force<LA, LB, T, false>, nb, kBlock, 0, st, d, f_src, f_dst, s, g, vpart, status);
-        prof_mark("local_force", st);
-    }
+    run_lambda<LA, LB, T>(d, st);
+    run_force_pass<LA, LB, T>(d, f_src, f_dst, s, g, vpart, status, st);
 }
 
 }  // namespace
