@@ -339,9 +339,16 @@ template <int N> __device__ __forceinline__ float lanes_sum(float (&v)[N], int l
 constexpr int kEvalSmem = kSmW + kSmSmall + 4 * 32768;
 constexpr int kTrainRed = 7 * 4 * kH;   // [value][row warp][column]: b2, w3, b1, W1 x 4
 constexpr int kTrainSmem = kSmW + kSmSmall + 2 * 32768 + kTrainRed * 4;
+// A training batch: network units (x rows of kIn, t), or the caller's doubles
+// (pts rows of D, tgt), normalised here by the operations of nb_normalise.
+struct MlpBatch {
+    const float *x, *t;
+    const double *pts, *tgt;
+    double lo[kIn], span[kIn], vscale;
+};
 __global__ void __launch_bounds__(512, 1)
-    k_mlp_train(MlpDev p, int npts, const float *__restrict__ x, const float *__restrict__ t, float *part,
-                float *loss_part, float grad_scale, int *err, int tries, int stall) {
+    k_mlp_train(MlpDev p, int npts, MlpBatch in, float *part, float *loss_part, float grad_scale, int *err, int tries,
+                int stall) {
     extern __shared__ __align__(1024) unsigned char sm[];
     __shared__ uint64_t mbar;
     __shared__ uint32_t tbase;
@@ -357,8 +364,13 @@ __global__ void __launch_bounds__(512, 1)
     if (warp == 0) tmem_alloc(&tbase, 512);
     load_weights(p, sm, true);
     float u[kIn] = {0.f, 0.f, 0.f, 0.f};
-    if (valid) {
-        const float4 v = *reinterpret_cast<const float4 *>(x + (size_t)row * kIn);
+    if (valid && in.pts) {
+#pragma unroll
+        for (int i = 0; i < kIn; ++i)
+            if (i < p.D)
+                u[i] = (float)(2.0 * (in.pts[(size_t)row * p.D + i] - in.lo[i]) / in.span[i] - 1.0);
+    } else if (valid) {
+        const float4 v = *reinterpret_cast<const float4 *>(in.x + (size_t)row * kIn);
         u[0] = v.x;
         u[1] = v.y;
         u[2] = v.z;
@@ -407,7 +419,8 @@ __global__ void __launch_bounds__(512, 1)
         __syncthreads();
         if (wg == 0) {
             y = srow[0][0][m] + srow[0][1][m] + srow[0][2][m] + srow[0][3][m];
-            const float d = valid ? y - t[row] : 0.0f;
+            const float target = !valid ? y : in.pts ? (float)(in.tgt[row] / in.vscale) : in.t[row];
+            const float d = y - target;
             sdy[m] = grad_scale * d;
             float l = d * d, g = grad_scale * d;
             for (int o = 16; o > 0; o >>= 1) {
@@ -549,8 +562,12 @@ __global__ void k_mlp_adam(int ntiles, const float *__restrict__ part, float *ma
     else b3[0] = w;
 }
 
-// Gradient summed over tiles without an update (for checks).
-__global__ void k_mlp_gradsum(int ntiles, const float *__restrict__ part, float *g) {
+// Gradient summed over tiles without an update (for checks), followed by the
+// timeout flag and the tiles' losses, so that one copy brings all of it.
+__global__ void k_mlp_gradsum(int ntiles, const float *__restrict__ part, const float *__restrict__ loss,
+                              const int *__restrict__ err, float *g) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t <= ntiles; t += gridDim.x * blockDim.x)
+        g[kNPpad + t] = t ? loss[t - 1] : __int_as_float(*err);
     int q;
     float s;
     if (tile_sum(ntiles, part, q, s)) g[q] = s;
@@ -699,6 +716,8 @@ struct mtd_nnbias {
     int *d_err = nullptr;
     double *d_pt = nullptr, *d_ppart = nullptr, *d_pout = nullptr;
     unsigned int *d_ticket = nullptr;
+    float *h_stage = nullptr, *d_stage = nullptr;   // nb_ensure_stage
+    size_t cap_stage = 0;
     // training pool
     int ntrain = 0;
     float *d_xt = nullptr, *d_tt = nullptr;
@@ -752,6 +771,20 @@ mtd_status nb_tile_attr(mtd_nnbias *b) {
     NB_CU(set(k_mlp_eval<true, 4>, kEvalSmem), "smem attribute");
     NB_CU(set(k_mlp_train, kTrainSmem), "smem attribute");
     if (b->device >= 0 && b->device < 64) g_attr_done[b->device] = true;
+    return MTD_OK;
+}
+
+// Pinned and device staging of mtd_nnbias_loss_grad: `n` floats each way.
+mtd_status nb_ensure_stage(mtd_nnbias *b, size_t n) {
+    n = (n + 3) / 4 * 4;
+    if (n <= b->cap_stage) return MTD_OK;
+    cudaFreeHost(b->h_stage);
+    cudaFree(b->d_stage);
+    b->h_stage = b->d_stage = nullptr;
+    b->cap_stage = 0;
+    NB_CU(cudaMallocHost(&b->h_stage, sizeof(float) * n), "staging");
+    NB_CU(cudaMalloc(&b->d_stage, sizeof(float) * 2 * n), "staging");
+    b->cap_stage = n;
     return MTD_OK;
 }
 
@@ -957,9 +990,10 @@ void mtd_nnbias_destroy(mtd_nnbias *b) {
     if (b->st) cudaStreamSynchronize(b->st);
     void *ptrs[] = {b->d_hills, b->d_master, b->d_mom, b->d_vel, b->d_W1, b->d_b1, b->d_b2, b->d_w3, b->d_b3,
                     b->d_W2, b->d_W2t, b->d_part, b->d_loss, b->d_err, b->d_pt, b->d_pout, b->d_ppart,
-                    b->d_ticket, b->d_xt, b->d_tt, b->d_hs};
+                    b->d_ticket, b->d_xt, b->d_tt, b->d_hs, b->d_stage};
     for (void *p : ptrs)
         if (p) cudaFree(p);
+    if (b->h_stage) cudaFreeHost(b->h_stage);
     if (b->hs_ev) cudaEventDestroy(b->hs_ev);
     if (b->st) cudaStreamDestroy(b->st);
     delete b;
@@ -1041,36 +1075,42 @@ mtd_status mtd_nnbias_eval(mtd_nnbias *b, int npts, const double *pts, double *V
 mtd_status mtd_nnbias_loss_grad(mtd_nnbias *b, int npts, const double *pts, const double *targets, double vscale,
                                 float *grad, double *loss) {
     if (!b || npts <= 0 || !pts || !targets || !grad || !(vscale > 0)) return MTD_ERR_INVALID_ARG;
-    std::vector<float> x((size_t)npts * kIn), t(npts);
-    for (int i = 0; i < npts; ++i) {
-        nb_normalise(b, pts + (size_t)i * b->D, x.data() + (size_t)i * kIn);
-        t[i] = (float)(targets[i] / vscale);
-    }
     const int ntiles = (npts + kH - 1) / kH;
     mtd_status s = nb_ensure_tiles(b, ntiles);
     if (s != MTD_OK) return s;
     s = nb_tile_attr(b);
     if (s != MTD_OK) return s;
-    float *d_x = nullptr, *d_t = nullptr, *d_g = nullptr;
-    NB_CU(cudaMalloc(&d_x, sizeof(float) * x.size()), "points");
-    NB_CU(cudaMalloc(&d_t, sizeof(float) * npts), "targets");
-    NB_CU(cudaMalloc(&d_g, sizeof(float) * kNPpad), "gradient");
-    cudaMemcpyAsync(d_x, x.data(), sizeof(float) * x.size(), cudaMemcpyHostToDevice, b->st);
-    cudaMemcpyAsync(d_t, t.data(), sizeof(float) * npts, cudaMemcpyHostToDevice, b->st);
-    k_mlp_train<<<ntiles, 512, kTrainSmem, b->st>>>(nb_dev(b), npts, d_x, d_t, b->d_part, b->d_loss, 2.0f / npts,
-                                                    b->d_err, b->wait_tries, b->wait_stall);
-    k_mlp_gradsum<<<kSumBlocks, 256, 0, b->st>>>(ntiles, b->d_part, d_g);
-    std::vector<float> lp(ntiles);
-    cudaMemcpyAsync(grad, d_g, sizeof(float) * kNP, cudaMemcpyDeviceToHost, b->st);
-    cudaMemcpyAsync(lp.data(), b->d_loss, sizeof(float) * ntiles, cudaMemcpyDeviceToHost, b->st);
-    s = nb_check_err(b);
-    cudaFree(d_x);
-    cudaFree(d_t);
-    cudaFree(d_g);
+    // points and targets go over as they are, through pinned memory (the
+    // divisions of their normalisation took the host 40 us at 8,192 points),
+    // and the results come back in one copy
+    const size_t np = (size_t)npts * b->D, nin = 2 * (np + npts), nout = (size_t)kNPpad + 1 + ntiles;
+    s = nb_ensure_stage(b, std::max(nin, nout));
     if (s != MTD_OK) return s;
+    std::memcpy(b->h_stage, pts, sizeof(double) * np);
+    std::memcpy(b->h_stage + 2 * np, targets, sizeof(double) * npts);
+    float *d_g = b->d_stage + b->cap_stage;
+    NB_CU(cudaMemcpyAsync(b->d_stage, b->h_stage, sizeof(float) * nin, cudaMemcpyHostToDevice, b->st), "points");
+    MlpBatch in{};
+    in.pts = reinterpret_cast<const double *>(b->d_stage);
+    in.tgt = in.pts + np;
+    in.vscale = vscale;
+    for (int k = 0; k < b->D; ++k) {
+        in.lo[k] = b->lo[k];
+        in.span[k] = b->hi[k] - b->lo[k];
+    }
+    k_mlp_train<<<ntiles, 512, kTrainSmem, b->st>>>(nb_dev(b), npts, in, b->d_part, b->d_loss, 2.0f / npts, b->d_err,
+                                                    b->wait_tries, b->wait_stall);
+    k_mlp_gradsum<<<kSumBlocks, 256, 0, b->st>>>(ntiles, b->d_part, b->d_loss, b->d_err, d_g);
+    NB_CU(cudaGetLastError(), "gradient");
+    NB_CU(cudaMemcpyAsync(b->h_stage, d_g, sizeof(float) * nout, cudaMemcpyDeviceToHost, b->st), "gradient");
+    NB_CU(cudaStreamSynchronize(b->st), "gradient");
+    int timeout;
+    std::memcpy(&timeout, b->h_stage + kNPpad, sizeof timeout);
+    if (timeout) return nb_check_err(b);   // clears the flag
+    std::memcpy(grad, b->h_stage, sizeof(float) * kNP);
     if (loss) {
         double l = 0.0;
-        for (float v : lp) l += v;
+        for (int v = 0; v < ntiles; ++v) l += b->h_stage[kNPpad + 1 + v];
         *loss = l / npts;
     }
     return MTD_OK;
@@ -1149,9 +1189,11 @@ mtd_status mtd_nnbias_fit(mtd_nnbias *b, int ntrain, int iters, int batch, doubl
         const float b1c = 1.0f - std::pow(0.9f, (float)b->adam_t), b2c = 1.0f - std::pow(0.999f, (float)b->adam_t);
         const float lr_t = (float)(lr * (it < iters / 2 ? 1.0 : 0.5 * (1.0 + std::cos(M_PI * (it - iters / 2) /
                                                                                    std::max(1, iters - iters / 2)))));
-        k_mlp_train<<<ntiles, 512, kTrainSmem, b->st>>>(nb_dev(b), nb, b->d_xt + (size_t)bi * batch * kIn,
-                                                        b->d_tt + (size_t)bi * batch, b->d_part, b->d_loss, 2.0f / nb,
-                                                        b->d_err, b->wait_tries, b->wait_stall);
+        MlpBatch in{};
+        in.x = b->d_xt + (size_t)bi * batch * kIn;
+        in.t = b->d_tt + (size_t)bi * batch;
+        k_mlp_train<<<ntiles, 512, kTrainSmem, b->st>>>(nb_dev(b), nb, in, b->d_part, b->d_loss, 2.0f / nb, b->d_err,
+                                                        b->wait_tries, b->wait_stall);
         k_mlp_adam<<<kSumBlocks, 256, 0, b->st>>>(ntiles, b->d_part, b->d_master, b->d_mom, b->d_vel,
                                                          std::max(lr_t, (float)(lr * 0.02)), b1c, b2c, b->d_W1,
                                                          b->d_b1, b->d_W2, b->d_W2t, b->d_b2, b->d_w3, b->d_b3, 1);
