@@ -470,6 +470,7 @@ struct WalkStepArgs {
     const int *pa, *pc;         // prefix sums of WalkDesc::nb and ::nchunk over the walkers (nwalk + 1)
     const BiasPlan *const *plans;
     const long long *step;      // the step number (pinned host memory)
+    long long *step_dev;        // its copy in device memory, made by the launch
     WalkState *ws;
     GridBar *bar;
     int limit;                  // barrier polls before a wait gives up

@@ -53,14 +53,16 @@ template <int LA, int LB, typename T, bool STEP>
 __global__ void __launch_bounds__(kWalkBlock, 3) k_walk_step(const WalkDesc<T> *__restrict__ wd, WalkStepArgs a) {
     constexpr int KIND = STEP ? NK_STEP : NK_SWITCH;
     __shared__ int pa[kWalkPersistMax + 1], pc[kWalkPersistMax + 1];
-    // the step number lives in pinned host memory: one read per block over
-    // the host link, every later read from shared memory
+    // the step number lives in pinned host memory: one block reads it over the
+    // host link and passes it on in device memory, past the barriers before
+    // the bias phases (a read by each of the 444 blocks, one after another on
+    // the link, held the first phase up for 395 of the step's 1,520 us)
     __shared__ long long s_step;
     for (int t = threadIdx.x; t <= a.nwalk; t += blockDim.x) {
         pa[t] = a.pa[t];
         pc[t] = a.pc[t];
     }
-    if (threadIdx.x == 0) s_step = *(volatile const long long *)a.step;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *(volatile long long *)a.step_dev = *(volatile const long long *)a.step;
     __syncthreads();
     const int nw = a.nwalk;
     const int G = gridDim.x;
@@ -124,6 +126,8 @@ __global__ void __launch_bounds__(kWalkBlock, 3) k_walk_step(const WalkDesc<T> *
     }
     if (!grid_barrier(a.bar, a.limit, false)) return;
     // bias: every walker's CVs, the deposit in walker order, coefficients
+    if (threadIdx.x == 0) s_step = *(volatile const long long *)a.step_dev;
+    __syncthreads();
     for (int w = blockIdx.x; w < nw; w += G) walk_phase_cvs(a.plans, w, &s_step, a.ws);
     if (!grid_barrier(a.bar, a.limit, false)) return;
     // one block deposits: spreading the bins over every block measured slower here

@@ -187,6 +187,7 @@ mtd_status walkers_persist_step(mtd_walkers *W, const int *n, const double *cons
     a.pc = W->d_pre + nw + 1;
     a.plans = W->d_plans;
     a.step = W->h_step;   // pinned: the launch reads the step the host set
+    a.step_dev = W->d_step;
     a.ws = W->d_ws;
     a.bar = W->d_bar;
     a.limit = W->wait_limit;
