@@ -196,7 +196,8 @@ mtd_status alloc_env(mtd_ctx *c, Env &e, int npad) {
 // walkers has it: the two give the same results bit for bit.)
 static int unit_block(const mtd_ctx *c, const Unit &u) {
     if (u.kind == CAL_STRU_FACTOR) return lanes_block(c->n, kLaneAtomsSf);
-    return u.kind == CAL_STEINH_Q || c->ring ? lanes_block(c->n) : kBlock;
+    if (u.kind == CAL_STEINH_Q) return lanes_block(c->n, c->host_call ? kLaneAtomsHost : kLaneAtoms);
+    return c->ring ? lanes_block(c->n) : kBlock;
 }
 
 mtd_status alloc_unit(mtd_ctx *c, Unit &u, int npad) {
@@ -253,9 +254,10 @@ mtd_status ensure_capacity(mtd_ctx *c, int n) {
     const int npad = ((n + kBlock - 1) / kBlock) * kBlock + kBlock;
     c->n = n;
     c->npad = npad;
-    if (n != c->n_plan) {   // the bias kernel reads ceil(n / block) partials per unit
+    if (n != c->n_plan || c->host_call != c->host_plan) {   // the bias kernel reads ceil(n / block) partials per unit
         c->plan_dirty = true;
         c->n_plan = n;
+        c->host_plan = c->host_call;
     }
     if (npad > c->cap_n) {
         const int cap = npad + npad / 4;
@@ -611,6 +613,7 @@ template <typename T> GlobalDev<T> global_dev(mtd_ctx *c, Unit &u, const CellGri
     d.smask = c->smask; d.perm = c->perm; d.geo = make_geo<T>(g, c->pf, c->xs); d.exact = geo_d(g, c->xs);
     d.nb = env_dev(c->envs[u.env]);
     d.q = (T *)u.q; d.Q = (T *)u.Q; d.partials = u.partials; d.coef = u.coef;
+    d.lanes = unit_block(c, u) < kBlock;
     return d;
 }
 
@@ -1341,6 +1344,13 @@ mtd_status mtd_init(mtd_ctx *c) {
 }
 
 namespace {
+// Marks a call that waits for its step (unit_block).
+struct HostCall {
+    mtd_ctx *c;
+    explicit HostCall(mtd_ctx *ctx) : c(ctx) { c->host_call = true; }
+    ~HostCall() { c->host_call = false; }
+};
+
 // The part of mtd_post_force after x (and mask) are on the device: f upload
 // beside the CV passes, the step with its overflow retries, f download.
 mtd_status step_uploaded(mtd_ctx *c, int64_t step, int n, bool has_mask, const int *image, double *f,
@@ -1436,6 +1446,7 @@ mtd_status mtd_post_force(mtd_ctx *c, int64_t step, int n, const double *x, cons
         mtd_status s = mtd_init(c);
         if (s != MTD_OK) return s;
     }
+    const HostCall host_call(c);
     mtd_status s = ensure_capacity(c, n);
     if (s != MTD_OK) return s;
     const size_t b3 = sizeof(double) * 3 * (size_t)n;
@@ -1458,6 +1469,7 @@ mtd_status mtd_set_positions_f64(mtd_ctx *c, const double *x, const int *type, c
         mtd_status s = mtd_init(c);
         if (s != MTD_OK) return s;
     }
+    const HostCall host_call(c);
     mtd_status s = ensure_capacity(c, n);
     if (s != MTD_OK) return s;
     if (type && mtd_needs_types(c)) {
@@ -1480,6 +1492,7 @@ mtd_status mtd_step(mtd_ctx *c, int64_t step, double *f_inout, double *cv_out, d
     if (c->staged_n > 0 && !f_inout) return MTD_ERR_INVALID_ARG;
     const int n = c->staged_n;
     c->staged_n = -1;
+    const HostCall host_call(c);
     mtd_status s = ensure_capacity(c, n);
     if (s != MTD_OK) return s;
     s = step_uploaded(c, step, n, c->staged_mask, nullptr, f_inout, virial_out);

@@ -139,6 +139,7 @@ struct mtd_ctx {
     BiasPlan plan{};
     BiasPlan *d_plan = nullptr;
     bool plan_dirty = true;
+    bool host_call = false, host_plan = false;   // inside a call that waits for its step (host arrays); the plan's
     double *d_grid = nullptr;
     long long grid_size = 0;
     HillRec *d_hills = nullptr;

@@ -183,8 +183,8 @@ __global__ void __launch_bounds__(kBlock) k_global_force(GlobalDev<T> d, const d
 }  // namespace
 
 template <int L, typename T> static void launch_global_values_l(const GlobalDev<T> &d, cudaStream_t st) {
-    const int ab = lanes_block(d.n), nb = (d.n + ab - 1) / ab;
-    if (ab < kBlock) launch_k(k_global_values<L, T, kLanes>, nb, kBlock, 0, st, d);
+    const int ab = d.lanes ? kBlock / kLanes : kBlock, nb = (d.n + ab - 1) / ab;
+    if (d.lanes) launch_k(k_global_values<L, T, kLanes>, nb, kBlock, 0, st, d);
     else launch_k(k_global_values<L, T, 1>, nb, kBlock, 0, st, d);
 }
 
@@ -201,8 +201,8 @@ template <typename T> void launch_global_values(const GlobalDev<T> &d, cudaStrea
 template <int L, typename T>
 static void launch_global_forces_l(const GlobalDev<T> &d, const double *f_src, double *f_dst, const SysDev &s,
                                    const CellGrid &g, double *vpart, DevStatus *status, cudaStream_t st) {
-    const int ab = lanes_block(d.n), nb = (d.n + ab - 1) / ab;
-    if (ab < kBlock) launch_k(k_global_force<L, T, kLanes>, nb, kBlock, 0, st, d, f_src, f_dst, s, g, vpart, status);
+    const int ab = d.lanes ? kBlock / kLanes : kBlock, nb = (d.n + ab - 1) / ab;
+    if (d.lanes) launch_k(k_global_force<L, T, kLanes>, nb, kBlock, 0, st, d, f_src, f_dst, s, g, vpart, status);
     else launch_k(k_global_force<L, T, 1>, nb, kBlock, 0, st, d, f_src, f_dst, s, g, vpart, status);
 }
 

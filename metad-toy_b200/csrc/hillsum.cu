@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(256) k_hs_count(Cells c, int D, int npts, cons
 #pragma unroll
         for (int e = 0; e < 4; ++e) r[e] = src[e];
         r[2].y *= 1.4426950408889634074 * kTab;   // 32 log2(e) / (2 sigma^2)
+        if (!isfinite(r[3].x)) r[3].y = 0.0;      // a width whose 1 / sigma^2 overflows reaches no point
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e) rows[((size_t)e * ng + g) * 32 + lane] = r[e];   // past nh: a cut of 0

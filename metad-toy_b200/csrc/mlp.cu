@@ -697,11 +697,10 @@ struct mtd_nnbias {
     double lo[kIn] = {0, 0, 0, 0}, hi[kIn] = {1, 1, 1, 1};
     double vscale = 1.0;
     cudaStream_t st = nullptr;
-    // scratch of the batched hill sum (grown on demand), the stream of its
-    // last user and an event behind that use: a call on another stream waits
+    // scratch of the batched hill sum (grown on demand) and an event behind its
+    // last use: a call on another stream waits for it
     void *d_hs = nullptr;
     size_t cap_hs = 0;
-    cudaStream_t hs_st = nullptr;
     cudaEvent_t hs_ev = nullptr;
     std::string err;
     std::vector<double> hills;   // packed, 8 doubles per hill
@@ -833,15 +832,14 @@ cudaError_t nb_hillsum(mtd_nnbias *b, int npts, const double *pts, int ps, doubl
         if ((e = cudaMalloc(&b->d_hs, need + need / 4)) != cudaSuccess) return e;
         b->cap_hs = need + need / 4;
         scratch = b->d_hs;
-    } else if (st != b->hs_st) {
-        if ((e = cudaStreamWaitEvent(st, b->hs_ev, 0)) != cudaSuccess) return e;
+    } else if ((e = cudaStreamWaitEvent(st, b->hs_ev, 0)) != cudaSuccess) {
+        return e;
     }
     e = hillsum_batch(b->D, b->lo, b->hi, npts, pts, ps, b->nh, b->d_hills, V, dV, gs, scratch, st);
     if (cap != cudaStreamCaptureStatusNone) {
         const cudaError_t ef = cudaFreeAsync(scratch, st);
         return e != cudaSuccess ? e : ef;
     }
-    b->hs_st = st;
     const cudaError_t er = cudaEventRecord(b->hs_ev, st);
     return e != cudaSuccess ? e : er;
 }

@@ -161,7 +161,8 @@ __global__ void k_place(CellGrid g, SysDev s) {
 // kernels are all latency: 4,000 atoms 33 us (five kernels, event intervals)
 // and 17 now, 32,000 atoms 40 and 23, 61,000 atoms 34 and 34 on a tenth of
 // the SMs and with four launches fewer; beyond 65,536 the five kernels.
-constexpr int kClusterBlocks = 16, kClusterAtoms = 4;   // atoms per thread
+// (A sparse system's empty cells, beyond 16 a thread, are left to them too.)
+constexpr int kClusterBlocks = 16, kClusterAtoms = 4, kClusterCells = 16;   // per thread
 __global__ void __launch_bounds__(kScanBlock) k_cells_cluster(CellGrid g, SysDev s) {
     pdl_entry();
     __shared__ int sum;
@@ -747,7 +748,8 @@ static bool cells_cluster_ok() {
 int launch_build_cells(const CellGrid &g, SysDev &s, cudaStream_t st) {
     const int nb = (s.n + kBlock - 1) / kBlock;
     const SkinState *sk = s.skin;
-    if (s.n > 0 && s.n <= kClusterBlocks * kScanBlock * kClusterAtoms && cells_cluster_ok()) {
+    constexpr int kThreads = kClusterBlocks * kScanBlock;
+    if (s.n > 0 && s.n <= kThreads * kClusterAtoms && g.ncell <= kThreads * kClusterCells && cells_cluster_ok()) {
         launch_k_cluster(k_cells_cluster, kClusterBlocks, kClusterBlocks, kScanBlock, st, g, s);
         prof_mark("cell_list", st);
         return 1;

@@ -71,8 +71,9 @@ def test_points_and_hills_that_are_not_finite_count_nothing():
     c, h, s = _hills(70, 4, 3, True)
     p = np.array([c[5], c[40], c[5], c[69]]) + 0.001
     p[1, 2], p[2, 0] = np.nan, np.inf
-    c2 = np.insert(c, [10, 50], [[np.nan] * 4, [np.inf, 0, 0, 0]], axis=0)
-    h2, s2 = np.insert(h, [10, 50], 1.0), np.insert(s, [10, 50], 0.02)
+    # and a hill on a point whose 1 / sigma^2 overflows
+    c2 = np.insert(c, [10, 50, 60], [[np.nan] * 4, [np.inf, 0, 0, 0], p[0]], axis=0)
+    h2, s2 = np.insert(h, [10, 50, 60], 1.0), np.insert(s, [10, 50, 60], [0.02, 0.02, 1e-155])
     out = []
     for args in ((c, h, s), (c2, h2, s2)):
         nb = mtd.NNBias(systems.CV4_LO, systems.CV4_HI)

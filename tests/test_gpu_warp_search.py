@@ -5,7 +5,7 @@ forces bit for bit; and against a brute-force count at small sizes.
 
 Atom counts at the edges of the warps' blocks (8 atoms), of the cluster's
 threads (1,024 and 65,536 atoms) and of the rule for the warp shape; open and
-periodic boxes, a dense system with more than 32 neighbours, caps that bind.
+periodic boxes, sparse ones on both sides of the cluster's 262,144 cells, a dense system with more than 32 neighbours, caps that bind.
 """
 import numpy as np
 import pytest
@@ -43,6 +43,7 @@ def _run(kind, x, L, per, variant, M, precision):
 @pytest.mark.parametrize("n,kind,per,rho", [(1, "STEP", (1, 1, 1), 0.02), (7, "Q", (0, 1, 0), 0.02),
                                             (9, "SF", (1, 1, 1), 0.02), (1023, "Q", (1, 1, 1), 0.13),
                                             (1025, "FERMI", (0, 0, 0), 0.05), (1024, "STEP", (1, 0, 1), 0.15),
+                                            (1000, "STEP", (1, 1, 1), 1.25e-4), (1000, "STEP", (1, 1, 1), 1.5e-5),
                                             (4000, "Q", (1, 1, 1), 0.03), (65536, "FERMI", (1, 1, 1), 0.03),
                                             (65537, "SF", (1, 1, 1), 0.03), (131073, "Q", (1, 1, 1), 0.03)])
 @pytest.mark.parametrize("precision", ["mixed", "fp64"])
