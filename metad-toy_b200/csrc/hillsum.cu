@@ -194,7 +194,7 @@ __device__ __forceinline__ double gap2(double plo, double phi, double lo, double
     return d * d;
 }
 
-// A block's warps share 64 points and split the hills, and so do the blocks of
+// A block's warps share 32 points and split the hills, and so do the blocks of
 // a cluster: split q of Q takes groups q, q + Q, ...; the splits' sums are
 // added in split order.  (Warps with points of their own finish apart, by their
 // share of the hills: 2.5 warps per issue waited at the block's end.)

@@ -697,11 +697,13 @@ struct mtd_nnbias {
     double lo[kIn] = {0, 0, 0, 0}, hi[kIn] = {1, 1, 1, 1};
     double vscale = 1.0;
     cudaStream_t st = nullptr;
-    // scratch of the batched hill sum (grown on demand) and an event behind its
-    // last use: a call on another stream waits for it
+    // scratch of the batched hill sum (grown on demand), an event behind its
+    // last use (a call on another stream waits for it), and a lock over the wait,
+    // the launches and the event (calls of several threads)
     void *d_hs = nullptr;
     size_t cap_hs = 0;
     cudaEvent_t hs_ev = nullptr;
+    std::mutex hs_mu;
     std::string err;
     std::vector<double> hills;   // packed, 8 doubles per hill
     double *d_hills = nullptr;
@@ -821,16 +823,24 @@ cudaError_t nb_hillsum(mtd_nnbias *b, int npts, const double *pts, int ps, doubl
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     cudaError_t e = cudaStreamIsCapturing(st, &cap);
     if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(b->hs_mu);
     void *scratch = b->d_hs;
     if (cap != cudaStreamCaptureStatusNone) {
         if ((e = cudaMallocAsync(&scratch, need, st)) != cudaSuccess) return e;
     } else if (need > b->cap_hs) {
-        if ((e = cudaEventSynchronize(b->hs_ev)) != cudaSuccess) return e;
-        cudaFree(b->d_hs);
-        b->d_hs = nullptr;
-        b->cap_hs = 0;
-        if ((e = cudaMalloc(&b->d_hs, need + need / 4)) != cudaSuccess) return e;
-        b->cap_hs = need + need / 4;
+        // another thread's capture on another stream is no reason to refuse these
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        if ((e = cudaThreadExchangeStreamCaptureMode(&mode)) != cudaSuccess) return e;
+        e = cudaEventSynchronize(b->hs_ev);
+        if (e == cudaSuccess) {
+            cudaFree(b->d_hs);
+            b->d_hs = nullptr;
+            b->cap_hs = 0;
+            e = cudaMalloc(&b->d_hs, need + need / 4);
+            if (e == cudaSuccess) b->cap_hs = need + need / 4;
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) return e;
         scratch = b->d_hs;
     } else if ((e = cudaStreamWaitEvent(st, b->hs_ev, 0)) != cudaSuccess) {
         return e;

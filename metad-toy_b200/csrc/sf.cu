@@ -8,8 +8,9 @@
 // STRU_FACTOR_K (no reference counterpart): rho_k = sum_j exp(i k.x_j) over the
 // group, S(k) = |rho_k|^2/N, CV = mean_k S(k),
 //   dCV/dx_j = 2/(N K) sum_k k (-Re rho_k sin(k.x_j) + Im rho_k cos(k.x_j)).
-// Phases are formed in FP64 and reduced to [-pi, pi] before an FP32 sincos;
-// the sums over atoms are FP64 block partials reduced in a fixed order.
+// Phases are formed in FP64 in half turns and reduced before the FP32 (or FP64)
+// polynomials; the sums over atoms are FP64 block partials reduced in a fixed
+// order.
 #include "kernels.h"
 
 #include <algorithm>

@@ -111,3 +111,40 @@ def test_batch_replays_from_a_captured_graph():
         assert np.array_equal(d_v.cpu().numpy(), V) and np.array_equal(d_g.cpu().numpy(), dV)
     del g
     nb.close()
+
+
+def test_two_threads_on_two_streams_share_one_object():
+    import threading
+
+    import torch
+
+    c, h, s = _hills(2000, 4, 9, True)
+    nb = mtd.NNBias(systems.CV4_LO, systems.CV4_HI)
+    nb.add_hills(c, h, s)
+    rng = np.random.default_rng(2)
+    sizes = [(700, 9000), (8000, 300)]
+    pts = [[systems.CV4_LO + (systems.CV4_HI - systems.CV4_LO) * rng.random((n, 4)) for n in ns] for ns in sizes]
+    dev = [[torch.from_numpy(p).cuda() for p in ps] for ps in pts]
+    out = [[[torch.zeros(n, dtype=torch.float64, device="cuda"), torch.zeros((n, 4), dtype=torch.float64,
+                                                                             device="cuda")] for n in ns]
+           for ns in sizes]
+    streams = [torch.cuda.Stream() for _ in sizes]
+    torch.cuda.synchronize()
+
+    def run(w):
+        for _ in range(20):
+            for n, p, (v, g) in zip(sizes[w], dev[w], out[w]):
+                nb.eval_device(n, p.data_ptr(), v.data_ptr(), g.data_ptr(), use_nn=0,
+                               stream=streams[w].cuda_stream)
+
+    ts = [threading.Thread(target=run, args=(w,)) for w in range(2)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    torch.cuda.synchronize()
+    for w in range(2):
+        for p, (v, g) in zip(pts[w], out[w]):
+            V, dV = nb.exact(p)
+            assert np.array_equal(v.cpu().numpy(), V) and np.array_equal(g.cpu().numpy(), dV)
+    nb.close()
