@@ -718,7 +718,9 @@ struct mtd_nnbias {
     double *d_pt = nullptr, *d_ppart = nullptr, *d_pout = nullptr;
     unsigned int *d_ticket = nullptr;
     float *h_stage = nullptr, *d_stage = nullptr;   // nb_ensure_stage
-    size_t cap_stage = 0;
+    size_t cap_hstage = 0, cap_stage = 0;
+    static constexpr int kStages = 4;
+    cudaEvent_t stage_ev[kStages] = {};   // behind the last copy of each piece of h_stage
     // training pool
     int ntrain = 0;
     float *d_xt = nullptr, *d_tt = nullptr;
@@ -775,17 +777,44 @@ mtd_status nb_tile_attr(mtd_nnbias *b) {
     return MTD_OK;
 }
 
-// Pinned and device staging of mtd_nnbias_loss_grad: `n` floats each way.
-mtd_status nb_ensure_stage(mtd_nnbias *b, size_t n) {
-    n = (n + 3) / 4 * 4;
-    if (n <= b->cap_stage) return MTD_OK;
-    cudaFreeHost(b->h_stage);
-    cudaFree(b->d_stage);
-    b->h_stage = b->d_stage = nullptr;
-    b->cap_stage = 0;
-    NB_CU(cudaMallocHost(&b->h_stage, sizeof(float) * n), "staging");
-    NB_CU(cudaMalloc(&b->d_stage, sizeof(float) * 2 * n), "staging");
-    b->cap_stage = n;
+// Staging of mtd_nnbias_loss_grad: device memory for `nin` floats in and `nout`
+// out, and pinned memory of kStages pieces that the inputs cross in turn (at
+// least `nout`: the results come back whole).  Pinned memory for a whole batch
+// grew with the batch, and a first call took 2,000-3,800 us at 30,000 points
+// where this takes about 1,000: new pinned memory costs more than the copies.
+constexpr size_t kStage = 16384;   // floats, 64 KB
+mtd_status nb_ensure_stage(mtd_nnbias *b, size_t nin, size_t nout) {
+    const size_t nh = std::max(b->kStages * kStage, nout), nd = (nin + 3) / 4 * 4 + nout;
+    if (nh > b->cap_hstage) {
+        cudaFreeHost(b->h_stage);
+        b->h_stage = nullptr;
+        b->cap_hstage = 0;
+        NB_CU(cudaMallocHost(&b->h_stage, sizeof(float) * nh), "staging");
+        b->cap_hstage = nh;
+    }
+    if (nd > b->cap_stage) {
+        cudaFree(b->d_stage);
+        b->d_stage = nullptr;
+        b->cap_stage = 0;
+        NB_CU(cudaMalloc(&b->d_stage, sizeof(float) * nd), "staging");
+        b->cap_stage = nd;
+    }
+    return MTD_OK;
+}
+
+// n doubles of the caller to the device through the pieces of h_stage; `used`
+// counts those of this call so far.
+mtd_status nb_stage_in(mtd_nnbias *b, float *dst, const double *src, size_t n, int &used) {
+    constexpr size_t kPiece = kStage / 2;
+    for (size_t at = 0; at < n; at += kPiece, ++used) {
+        const size_t m = std::min(kPiece, n - at);
+        const int q = used % b->kStages;
+        if (used >= b->kStages) NB_CU(cudaEventSynchronize(b->stage_ev[q]), "staging");
+        std::memcpy(b->h_stage + q * kStage, src + at, sizeof(double) * m);
+        NB_CU(cudaMemcpyAsync(dst + 2 * at, b->h_stage + q * kStage, sizeof(double) * m, cudaMemcpyHostToDevice,
+                              b->st), "points");
+        NB_CU(cudaEventRecord(b->stage_ev[q], b->st), "staging");
+    }
     return MTD_OK;
 }
 
@@ -959,6 +988,7 @@ mtd_status mtd_nnbias_create(int D, const double *lo, const double *hi, unsigned
     NB_CU(cudaGetDevice(&b->device), "device");
     NB_CU(cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking), "stream");
     NB_CU(cudaEventCreateWithFlags(&b->hs_ev, cudaEventDisableTiming), "event");
+    for (cudaEvent_t &ev : b->stage_ev) NB_CU(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "event");
     NB_CU(cudaMalloc(&b->d_master, sizeof(float) * kNPpad), "params");
     NB_CU(cudaMalloc(&b->d_mom, sizeof(float) * kNPpad), "params");
     NB_CU(cudaMalloc(&b->d_vel, sizeof(float) * kNPpad), "params");
@@ -1002,6 +1032,8 @@ void mtd_nnbias_destroy(mtd_nnbias *b) {
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (b->h_stage) cudaFreeHost(b->h_stage);
+    for (cudaEvent_t ev : b->stage_ev)
+        if (ev) cudaEventDestroy(ev);
     if (b->hs_ev) cudaEventDestroy(b->hs_ev);
     if (b->st) cudaStreamDestroy(b->st);
     delete b;
@@ -1088,16 +1120,17 @@ mtd_status mtd_nnbias_loss_grad(mtd_nnbias *b, int npts, const double *pts, cons
     if (s != MTD_OK) return s;
     s = nb_tile_attr(b);
     if (s != MTD_OK) return s;
-    // points and targets go over as they are, through pinned memory (the
-    // divisions of their normalisation took the host 40 us at 8,192 points),
-    // and the results come back in one copy
+    // points and targets go over as they are, through pinned memory in pieces
+    // (the divisions of their normalisation took the host 40 us at 8,192
+    // points), and the results come back in one copy
     const size_t np = (size_t)npts * b->D, nin = 2 * (np + npts), nout = (size_t)kNPpad + 1 + ntiles;
-    s = nb_ensure_stage(b, std::max(nin, nout));
+    s = nb_ensure_stage(b, nin, nout);
     if (s != MTD_OK) return s;
-    std::memcpy(b->h_stage, pts, sizeof(double) * np);
-    std::memcpy(b->h_stage + 2 * np, targets, sizeof(double) * npts);
-    float *d_g = b->d_stage + b->cap_stage;
-    NB_CU(cudaMemcpyAsync(b->d_stage, b->h_stage, sizeof(float) * nin, cudaMemcpyHostToDevice, b->st), "points");
+    int used = 0;
+    s = nb_stage_in(b, b->d_stage, pts, np, used);
+    if (s == MTD_OK) s = nb_stage_in(b, b->d_stage + 2 * np, targets, npts, used);
+    if (s != MTD_OK) return s;
+    float *d_g = b->d_stage + (nin + 3) / 4 * 4;
     MlpBatch in{};
     in.pts = reinterpret_cast<const double *>(b->d_stage);
     in.tgt = in.pts + np;

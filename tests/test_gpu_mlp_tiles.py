@@ -63,3 +63,24 @@ def test_training_gradient_of_partial_tiles(npts):
                  (MO.O_W3, MO.O_B3), (MO.O_B3, MO.NP)]:
         assert _block_rel(g, go, a, b) < 2e-2, (a, b, _block_rel(g, go, a, b))
     nb.close()
+
+
+@pytest.mark.parametrize("D,npts", [(4, 2048), (4, 4097), (3, 9001)])
+def test_training_gradient_of_points_in_pieces(D, npts):
+    # the points cross in pieces of 8,192 doubles; the loss is a sum over all of
+    # them (1e-6: FP32 tile sums of equal terms, added in FP64), whatever the call before left
+    w = _random_params(13)
+    nb = mtd.NNBias(systems.CV4_LO[:D], systems.CV4_HI[:D])
+    nb.set_params(w, 1.0)
+    rng = np.random.default_rng(npts)
+    p = systems.CV4_LO[:D] + (systems.CV4_HI - systems.CV4_LO)[:D] * rng.random((npts, D))
+    t = np.sin(3 * p[:, 0]) + p[:, 1] * p[:, -1]
+    nb.loss_grad(p[::-1].copy(), t, 1.0)
+    g, loss = nb.loss_grad(p, t, 1.0)
+    part = [nb.loss_grad(p[a:a + 128], t[a:a + 128], 1.0) for a in range(0, npts, 128)]
+    n = [len(p[a:a + 128]) for a in range(0, npts, 128)]
+    lo = sum(k * l for k, (_, l) in zip(n, part)) / npts
+    assert abs(loss - lo) <= 1e-6 * lo
+    go = sum(k * x.astype(np.float64) for k, (x, _) in zip(n, part)) / npts
+    assert np.abs(g - go).max() <= 2e-2 * np.abs(go).max()
+    nb.close()
