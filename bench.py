@@ -439,14 +439,11 @@ def run_secondary(args, local):
 
 
 # Operations per (atom, k) pair of the S(k) passes, counted in the kernels'
-# source (an FMA counts 2): FP64 -- the phase k.x (6) and its reduction to a
-# quarter turn (5); FP32 -- the sin / cos polynomials (22), then the value
-# pass accumulates cos and sin (2) and the force pass projects on rho(k) and
-# k (9).
-# per (atom, k): FP64 phase (k / pi).x (5) and half-turn reduction (3 adds);
-# FP32 z^2, sin(pi z) (4 FMA + 1 mul), cos(pi z) (5 FMA), then the signed
-# accumulation (2 FMA) or the force weight and gradient (1 mul + 1 FMA + 3 FMA)
-SK_FLOP_PER_PAIR = {"sk_partial": {"fp64": 8, "fp32": 24}, "sk_force": {"fp64": 8, "fp32": 29}}
+# source (an FMA counts 2): FP64 -- the based phase (k / pi).x (3 FMA); FP32 --
+# the scaling of the remainder and its square (2), sin(pi z) (4 FMA + 1 mul),
+# then the value pass's cos(pi z) (5 FMA) and signed accumulation (2 FMA), or
+# the force pass's gradient (3 FMA)
+SK_FLOP_PER_PAIR = {"sk_partial": {"fp64": 6, "fp32": 25}, "sk_force": {"fp64": 6, "fp32": 17}}
 
 
 def sk_roofline(kernels, n, nk, clocks):
