@@ -294,7 +294,7 @@ mtd_status ensure_capacity(mtd_ctx *c, int n) {
         c->skin_valid = false;
         for (Env &e : c->envs) {
             if (e.M == 0) e.M = estimate_M(c, e.rc, n);
-            if (e.kind == ENV_Q && e.M > 64) e.M = 64;
+            if (e.kind == ENV_Q) e.M = std::min(e.M, kMaxCapList);
             mtd_status s = alloc_env(c, e, cap);
             if (s != MTD_OK) return s;
             if (skin) {
@@ -332,9 +332,11 @@ mtd_status ensure_cells(mtd_ctx *c, int ncell) {
 mtd_status grow_lists(mtd_ctx *c, unsigned need, unsigned cand_need) {
     for (Env &e : c->envs) {
         if (need > 0 && e.M < (int)need) {
-            if (e.kind == ENV_Q && need > 64)
+            if (e.kind == ENV_Q && need > kMaxCapList)
                 return fail(c, MTD_ERR_UNSUPPORTED, "STEINH Q: more than 64 atoms within cutoff_r");
             e.M = (((int)need + 8) + 3) & ~3;
+            // the cap ranks at most kMaxCapList entries: more of them have to overflow again
+            if (e.kind == ENV_Q) e.M = std::min(e.M, kMaxCapList);
             const mtd_status s = alloc_env(c, e, c->cap_n);
             if (s != MTD_OK) return s;
         }

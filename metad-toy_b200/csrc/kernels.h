@@ -131,6 +131,9 @@ struct NeighSpec {
     int variant;        // kernel shape of the fast path (0, 1, 2: see launch_neighbors); same lists
 };
 
+// Entries of a list that the cap of STEINH Q ranks, and so the longest such list.
+constexpr int kMaxCapList = 64;
+
 struct NeighDev {
     int *list;          // [M][npad] sorted neighbour indices (bit kFlagBit: kept by the centre's cap)
     int *count;         // [npad] neighbours found (may exceed M: overflow)

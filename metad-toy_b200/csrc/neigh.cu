@@ -260,8 +260,6 @@ __global__ void __launch_bounds__(kBlock) k_neighbors(CellGrid g, SysDev s, Neig
 }
 
 
-constexpr int kMaxCapList = 64;
-
 // Fast path, valid when every periodic dimension has at least three cells
 // (neighbors_fast_body).
 template <int KIND>
@@ -338,13 +336,12 @@ __global__ void __launch_bounds__(kBlock) k_neighbors_warp(CellGrid g, SysDev s,
                                                         (float)oy * g.hf[1] - a.y, (float)oz * g.hf[2] - a.z);
     __syncwarp();
     int cnt = 0, wait = 0, opened = -1;   // opened: the last cell begun before this round
+    const int most = min(nd.M, kMaxCapList);   // entries of a capped list; more are an overflow
     auto keep = [&](bool in, int j) {
         const unsigned hits = __ballot_sync(all, in);
         const int at = cnt + __popc(hits & below);
-        if (in && at < nd.M) {
-            if (CAP) held[warp][at] = j;   // M <= kMaxCapList with a cap
-            else nd.list[(size_t)at * s.npad + k] = j;
-        }
+        if (CAP && in && at < most) held[warp][at] = j;
+        if (!CAP && in && at < nd.M) nd.list[(size_t)at * s.npad + k] = j;
         cnt += __popc(hits);
     };
     // NK_SWITCH: the switch is evaluated for full warps of candidates in range
@@ -392,11 +389,11 @@ __global__ void __launch_bounds__(kBlock) k_neighbors_warp(CellGrid g, SysDev s,
     if (KIND == NK_SWITCH && wait > 0) decide_held(wait);
     if (lane == 0) {
         nd.count[k] = cnt;
-        if (cnt > nd.M) atomicMax(&status->overflow, (unsigned)cnt);
+        if (cnt > (CAP ? most : nd.M)) atomicMax(&status->overflow, (unsigned)cnt);
     }
     if (!CAP) return;
     __syncwarp();
-    const int c = min(cnt, min(nd.M, kMaxCapList));
+    const int c = min(cnt, most);
     const double xk[3] = {s.xs[3 * k], s.xs[3 * k + 1], s.xs[3 * k + 2]};
     double r2[2];
     int id[2], jj[2], rank[2] = {0, 0};
