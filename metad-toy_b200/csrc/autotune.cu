@@ -28,7 +28,7 @@ mtd_status autotune_idle(mtd_ctx *c, int n, const double *d_x, const int *d_mask
             s = fail(c, MTD_ERR_NEIGH_OVERFLOW, "neighbour list capacity exceeded");
             break;
         }
-        s = grow_lists(c, hs.overflow, hs.cand_overflow);
+        s = grow_lists(c, hs.overflow, hs.cand_overflow, hs.cap_overflow);
         if (s != MTD_OK) break;
     }
     if (s != MTD_OK) {

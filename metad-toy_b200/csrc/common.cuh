@@ -120,7 +120,8 @@ struct DevStatus {
     unsigned int timeout;         // a bounded wait gave up
     unsigned int bad_pos;         // an atom position was not finite (NaN or Inf)
     unsigned int cand_overflow;   // max skin-list candidate count seen when above capacity
-    unsigned int pad[3];
+    unsigned int cap_overflow;    // the part of `overflow` that capped lists (STEINH Q) saw
+    unsigned int pad[2];
 };
 
 // First statement of every step kernel: wait until the previous kernel of the

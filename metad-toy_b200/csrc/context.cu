@@ -329,8 +329,9 @@ mtd_status ensure_cells(mtd_ctx *c, int ncell) {
     return MTD_OK;
 }
 
-mtd_status grow_lists(mtd_ctx *c, unsigned need, unsigned cand_need) {
+mtd_status grow_lists(mtd_ctx *c, unsigned need_all, unsigned cand_need, unsigned cap_need) {
     for (Env &e : c->envs) {
+        const unsigned need = e.kind == ENV_Q ? cap_need : need_all;
         if (need > 0 && e.M < (int)need) {
             if (e.kind == ENV_Q && need > kMaxCapList)
                 return fail(c, MTD_ERR_UNSUPPORTED, "STEINH Q: more than 64 atoms within cutoff_r");
@@ -1012,6 +1013,7 @@ mtd_status drain(mtd_ctx *c, bool block) {
         if (c->h_status->overflow || c->h_status->cand_overflow) {
             c->overflow_seen = std::max(c->overflow_seen, c->h_status->overflow);
             c->overflow_cand_seen = std::max(c->overflow_cand_seen, c->h_status->cand_overflow);
+            c->overflow_cap_seen = std::max(c->overflow_cap_seen, c->h_status->cap_overflow);
             continue;
         }
         c->pending = true;
@@ -1408,7 +1410,7 @@ mtd_status step_uploaded(mtd_ctx *c, int64_t step, int n, bool has_mask, const i
         if (c->h_status->overflow == 0 && c->h_status->cand_overflow == 0) break;
         c->fifo.pop_back();   // the failed attempt is not collected
         // neighbour capacity too small: grow and run the step again
-        s = grow_lists(c, c->h_status->overflow, c->h_status->cand_overflow);
+        s = grow_lists(c, c->h_status->overflow, c->h_status->cand_overflow, c->h_status->cap_overflow);
         if (s != MTD_OK) return s;
         if (attempt == 3) return fail(c, MTD_ERR_NEIGH_OVERFLOW, "neighbour list capacity exceeded");
     }
@@ -1535,10 +1537,9 @@ mtd_status mtd_sync(mtd_ctx *c) {
     const mtd_status sd = drain(c, true);
     if (sd != MTD_OK) return sd;
     if (c->overflow_seen || c->overflow_cand_seen) {
-        const unsigned need = c->overflow_seen, cneed = c->overflow_cand_seen;
-        c->overflow_seen = 0;
-        c->overflow_cand_seen = 0;
-        const mtd_status sg = grow_lists(c, need, cneed);
+        const unsigned need = c->overflow_seen, cneed = c->overflow_cand_seen, qneed = c->overflow_cap_seen;
+        c->overflow_seen = c->overflow_cand_seen = c->overflow_cap_seen = 0;
+        const mtd_status sg = grow_lists(c, need, cneed, qneed);
         if (sg != MTD_OK) return sg;
         cudaMemset(c->d_status, 0, sizeof(DevStatus));
         c->h_status->overflow = 0;

@@ -242,6 +242,7 @@ struct mtd_ctx {
     std::vector<char> env_fused;         // skin lists: environment filtered inside its STEINH L unit's q pass
     bool skin_reset_pending = false;     // the step's first fused q pass closes the skin gate
     unsigned overflow_cand_seen = 0;     // largest candidate count of an overflowed step drained since mtd_sync
+    unsigned overflow_cap_seen = 0;      // the same of the capped lists
 };
 
 namespace mtd {
@@ -266,7 +267,9 @@ CellGrid make_grid(const mtd_ctx *c, double extra = 0.0);
 bool skin_grid(const mtd_ctx *c, CellGrid &g);
 // Grows the lists a step reported too small: exact lists to hold `need`
 // neighbours, skin candidate lists `cand_need` (which forces a rebuild).
-mtd_status grow_lists(mtd_ctx *c, unsigned need, unsigned cand_need);
+// Grows the lists that were too small: `need` of the uncapped lists, `cap_need`
+// of the capped ones (DevStatus::cap_overflow), `cand_need` of the candidates.
+mtd_status grow_lists(mtd_ctx *c, unsigned need, unsigned cand_need, unsigned cap_need);
 NeighSpec neigh_spec(const Env &e);
 SkDev sk_dev(mtd_ctx *c, Unit &u, const double *x, const int *mask);
 int estimate_M(const mtd_ctx *c, double rc, int n);

@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(kBlock) k_neighbors(CellGrid g, SysDev s, Neig
         }
     }
     nd.count[k] = cnt;
-    if (cnt > nd.M) atomicMax(&status->overflow, (unsigned)cnt);
+    if (cnt > nd.M) note_overflow(status, ns, cnt);
 }
 
 
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(kBlock) k_neighbors_warp(CellGrid g, SysDev s,
     if (KIND == NK_SWITCH && wait > 0) decide_held(wait);
     if (lane == 0) {
         nd.count[k] = cnt;
-        if (cnt > (CAP ? most : nd.M)) atomicMax(&status->overflow, (unsigned)cnt);
+        if (cnt > (CAP ? most : nd.M)) note_overflow(status, ns, cnt);
     }
     if (!CAP) return;
     __syncwarp();
@@ -538,7 +538,10 @@ __global__ void __launch_bounds__(kFlatBlock) k_neighbors_flat(CellGrid g, SysDe
         ++cnt;
     }
     nd.count[k] = cnt;
-    if (cnt > nd.M) atomicMax(KIND == NK_CAND ? &status->cand_overflow : &status->overflow, (unsigned)cnt);
+    if (cnt > nd.M) {
+        if (KIND == NK_CAND) atomicMax(&status->cand_overflow, (unsigned)cnt);
+        else note_overflow(status, ns, cnt);
+    }
 }
 
 // STEINH Q cap: keep the `cap` nearest by (r2, caller index), the order of the

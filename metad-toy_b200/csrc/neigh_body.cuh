@@ -138,7 +138,10 @@ __device__ __forceinline__ void neighbors_fast_body(const CellGrid &g, const Sys
         }
     }
     nd.count[k] = cnt;
-    if (cnt > nd.M) atomicMax(KIND == NK_CAND ? &status->cand_overflow : &status->overflow, (unsigned)cnt);
+    if (cnt > nd.M) {
+        if (KIND == NK_CAND) atomicMax(&status->cand_overflow, (unsigned)cnt);
+        else note_overflow(status, ns, cnt);
+    }
 }
 
 }  // namespace mtd

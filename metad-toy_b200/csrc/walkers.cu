@@ -496,7 +496,8 @@ mtd_status mtd_walkers_sync(mtd_walkers *W) {
     bool overflow = false;
     for (mtd_ctx *c : W->w) {
         if (c->h_status->overflow || c->h_status->cand_overflow) {
-            const mtd_status s = grow_lists(c, c->h_status->overflow, c->h_status->cand_overflow);
+            const mtd_status s =
+                grow_lists(c, c->h_status->overflow, c->h_status->cand_overflow, c->h_status->cap_overflow);
             if (s != MTD_OK) return wfail(W, s, c->err);
             cudaMemset(c->d_status, 0, sizeof(DevStatus));
             c->h_status->overflow = 0;

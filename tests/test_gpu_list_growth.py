@@ -65,3 +65,27 @@ def test_a_capped_list_grows_to_64_entries_and_no_further(variant, members, more
     with pytest.raises(mtd.MetadError, match="more than 64 atoms"):
         m.post_force(1, x, f)
     m.close()
+
+
+@pytest.mark.parametrize("skin", [False, True])
+def test_another_cals_long_list_is_no_matter_of_the_capped_one(skin):
+    # 90 atoms within 6.0 of one another, up to 55 of them within 2.0
+    x = _clusters(90, 0, 3)
+    args = _deck(_q(2.0) + ["CAL", "NAME", "SF", "STRU_FACTOR", "all", "cutoff_r", RC, "q_factor", 2.8])
+    i = args.index("CV_dim")
+    args = args[:i] + ["SYMBOL", "v2", "SF.AVE", "CV_dim", 2, "DIM", 1, -1.0, 2.0, 400, "v1", "DIM", 2, -50.0, 50.0,
+                       400, "v2", "WT", 0]
+    if skin:
+        args += ["NEIGH_SKIN", 0.5, "NEIGH_EVERY", 10]
+    m = mtd.Metad(args, precision="fp64")
+    m.set_box([0, 0, 0], L)
+    near, r2 = _within(x, 2.0)
+    assert near.sum(1).max() <= 64 < _within(x, RC)[0].sum(1).max()
+    f = np.zeros_like(x)
+    m.post_force(0, x, f)
+    count, idx = m.neighbors("Q", len(x), 64)
+    for k, kept in enumerate(_nearest(near, r2, 12)):
+        assert np.array_equal(idx[k, :count[k]], kept)
+    count, _ = m.neighbors("SF", len(x))
+    assert np.array_equal(count, _within(x, RC)[0].sum(1))
+    m.close()
