@@ -86,7 +86,8 @@ __global__ void __launch_bounds__(256) k_hs_count(Cells c, int D, int npts, cons
         const double2 *src = reinterpret_cast<const double2 *>(hills + (size_t)h * kHillRec);
 #pragma unroll
         for (int e = 0; e < 4; ++e) r[e] = src[e];
-        r[2].y *= 1.4426950408889634074 * kTab;   // 32 log2(e) / (2 sigma^2)
+        // 32 log2(e) / (2 sigma^2); finite, so that a hill on the point itself has the exponent 0
+        r[2].y = fmin(r[2].y * (1.4426950408889634074 * kTab), 1.7976931348623157e308);
         if (!isfinite(r[3].x)) r[3].y = 0.0;      // a width whose 1 / sigma^2 overflows reaches no point
     }
 #pragma unroll
@@ -217,7 +218,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
         s[k] = i >= 0 && k < D ? pts[(size_t)i * ps + k] : 0.0;
         fin = fin && isfinite(s[k]);
     }
-    // a point that is not finite is within reach of no hill
+    // a point that is not finite is within reach of no hill: its box is empty and its sums are written as zeros
 #pragma unroll
     for (int k = 0; k < kIn; ++k) {
         plo[k] = fin ? s[k] : INFINITY;
@@ -288,6 +289,9 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
 #pragma unroll
                 for (int k = 0; k < 1 + kIn; ++k) o[k] += rb[k * kT + w * 32];
         }
+        if (!fin)
+#pragma unroll
+            for (int k = 0; k < 1 + kIn; ++k) o[k] = 0.0;
         if (i >= 0) {
             V[i] = o[0];
             if (dV)

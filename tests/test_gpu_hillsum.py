@@ -148,3 +148,15 @@ def test_two_threads_on_two_streams_share_one_object():
             V, dV = nb.exact(p)
             assert np.array_equal(v.cpu().numpy(), V) and np.array_equal(g.cpu().numpy(), dV)
     nb.close()
+
+
+def test_widths_at_the_ends_of_the_range():
+    # a hill wide enough to reach a stand-in coordinate, and one whose exponent's factor overflows
+    p = np.array([[0.1, 0.2, 0.3, 0.4], [np.nan, 0.2, 0.3, 0.4], [0.1, -np.inf, 0.3, 0.4], [0.5, 0.5, 0.5, 0.5]])
+    nb = mtd.NNBias(systems.CV4_LO, systems.CV4_HI)
+    nb.add_hills(np.array([p[0], p[3]]), np.array([0.25, 0.5]), np.array([1e151, 1.2e-154]))
+    V, dV = nb.exact(p)
+    assert np.array_equal(V, [0.25, 0.0, 0.0, 0.75]) and not np.any(dV[:3])
+    want = -0.25 * (p[3] - p[0]) / 1e302
+    assert np.all(np.abs(dV[3] - want) <= 1e-13 * np.abs(want))
+    nb.close()
