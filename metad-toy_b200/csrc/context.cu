@@ -129,6 +129,22 @@ bool skin_grid(const mtd_ctx *c, CellGrid &g) {
     return false;
 }
 
+// Whether an FP32 value of a smooth pair switch that is above 2 eps + 1e-5 shows
+// that the switch is at least eps, for a pair closer than the list bound less its
+// guard band.  The bound is where the switch equals eps, so for a falling switch
+// every such pair is above eps, and for a rising one (FERMI or TANH with a positive
+// alpha) none is, nor is its FP32 value: both whatever the steepness, since the band
+// (5e-5 of r and more) is wide against the error of r.  A rational switch falls from
+// d0 on; below d0 it mirrors that for an even power, where its error is held to a
+// tenth by the power and r0, and for an odd one it has a pole.  The general n / m
+// form cancels at x = d0 + r0.  Those are left to the FP64 test.
+static bool fp32_accepts(const SwParams &sw, double eps, double rc) {
+    if (!(eps > 0.0)) return false;
+    if (sw.type == SW_FERMI || sw.type == SW_TANH) return true;
+    if (sw.type != SW_RATIONAL || sw.n <= 0 || 2 * sw.n != sw.m || !(sw.r0 > 0.0)) return false;
+    return sw.d0 <= 0.0 || (sw.n % 2 == 0 && sw.n * 1e-5 * std::fmax(rc, sw.d0) <= 0.1 * sw.r0);
+}
+
 // Neighbour criterion of an environment; the FP32 band [lo2, hi2] around the
 // bound (2e-5 relative + 1e-4 A^2) is wide against the ~1e-6 A error of the
 // cell-relative FP32 displacements, so outside it FP32 decides exactly.
@@ -148,7 +164,7 @@ NeighSpec neigh_spec(const Env &e) {
     } else {
         ns.kind = NK_RANGE;
     }
-    ns.accept = (float)(2.0 * e.eps + 1e-5);
+    ns.accept = fp32_accepts(e.sw, e.eps, e.rc) ? (float)(2.0 * e.eps + 1e-5) : INFINITY;
     ns.lo2 = (float)(eff * (1.0 - 2e-5) - 1e-4);
     ns.hi2 = (float)(ns.kind == NK_SWITCH ? ns.rc2 * (1.0 + 2e-5) + 1e-4 : eff * (1.0 + 2e-5) + 1e-4);
     return ns;

@@ -126,7 +126,7 @@ struct NeighSpec {
     double eps;
     SwParams sw;
     float lo2, hi2;     // FP32 accept-below / reject-above
-    float accept;       // NK_SWITCH: an FP32 switch value above this is above eps
+    float accept;       // NK_SWITCH: an FP32 switch value above this is above eps (infinite: FP64 decides)
     int cap;            // STEINH Q cutoff_Natoms, 0 = none
     int variant;        // kernel shape of the fast path (0, 1, 2: see launch_neighbors); same lists
 };
