@@ -323,30 +323,61 @@ __device__ __forceinline__ void turn_sincos2(double ta, double tb, float2 &s0, f
     c0 = __ffma2_rn(q, z2, dup2(kCosQ0));
 }
 
-// FP64: sin(pi f) = f S(f^2) and cos(pi f) = C(f^2) on |f| <= 1/2 by their
-// Taylor polynomials (remainders (pi/2)^23 / 23! = 1e-18 and (pi/2)^22 / 22! =
-// 2e-17), for a phase u in half turns rounded to the nearest integer as above.
-// s and c come with the sign (-1)^n; |u| < 2^51.
-template <bool COS> __device__ __forceinline__ void halfturn_sincos_f64(double u, double &s, double &c) {
-    constexpr double S[11] = {3.141592653589793, -5.16771278004997, 2.5501640398773455, -0.5992645293207921,
-                              0.08214588661112823, -0.0073704309457143504, 0.00046630280576761255,
-                              -2.1915353447830217e-05, 7.952054001475513e-07, -2.2948428997269873e-08,
-                              5.392664662608129e-10};
-    constexpr double C[11] = {1.0, -4.934802200544679, 4.0587121264167685, -1.3352627688545895, 0.2353306303588932,
-                              -0.02580689139001406, 0.0019295743094039231, -0.0001046381049248457,
-                              4.303069587032947e-06, -1.3878952462213771e-07, 3.604730797462501e-09};
+// FP64: a phase in radians less n half turns (or quarters), pi in two words
+// (Cody and Waite, Software Manual for the Elementary Functions, 1980): both
+// products are exact inside their FMA up to n = 2^51, so the remainder is off by
+// its own rounding.  The phase itself is not scaled first: a k.x / pi is rounded
+// once more than k.x, and with k.x of some hundred radians that was a third of
+// the forces' error.  |phase| < 2^50 (kPhaseMax).
+constexpr double kPhaseMax = 1125899906842624.0;
+__device__ __forceinline__ double phase_units(double ph, double per_unit, int &n) {
     constexpr double kRound = 6755399441055744.0;   // 1.5 * 2^52
-    const double t = u + kRound, f = u - (t - kRound), z = f * f;
-    const unsigned sgn = (unsigned)__double2loint(t) << 31;
-    double p = S[10], q = C[10];
+    const double t = fma(ph, per_unit, kRound);
+    n = __double2loint(t);
+    return t - kRound;
+}
+__device__ __forceinline__ double flip(double v, int n) {   // (-1)^n v
+    return __hiloint2double(__double2hiint(v) ^ (n << 31), __double2loint(v));
+}
+
+// sin(ph - shift) by its Taylor polynomial on |r| <= pi / 2 (remainder r^23 / 23!
+// = 1e-18); the shift, |shift| <= pi, is taken off the small remainder.
+__device__ __forceinline__ double phase_sin_f64(double ph, double shift) {
+    constexpr double S[10] = {-0.16666666666666666, 0.008333333333333333, -0.0001984126984126984,
+                              2.7557319223985893e-06, -2.505210838544172e-08, 1.6059043836821613e-10,
+                              -7.647163731819816e-13, 2.8114572543455206e-15, -8.22063524662433e-18,
+                              1.9572941063391263e-20};
+    int n;
+    const double q = phase_units(ph - shift, kInvPi, n);
+    const double r = fma(-q, 1.2246467991473532e-16, fma(-q, 3.141592653589793, ph) - shift), z = r * r;
+    double p = S[9];
 #pragma unroll
-    for (int k = 9; k >= 0; --k) {
+    for (int k = 8; k >= 0; --k) p = fma(p, z, S[k]);
+    return flip(fma(r * z, p, r), n);
+}
+
+// sin and cos by theirs on |r| <= pi / 4 (remainders r^19 / 19! = 8e-20 and
+// r^18 / 18! = 2e-18), exchanged in odd quarters.
+__device__ __forceinline__ void phase_sincos_f64(double ph, double &s, double &c) {
+    constexpr double S[8] = {-0.16666666666666666, 0.008333333333333333, -0.0001984126984126984,
+                             2.7557319223985893e-06, -2.505210838544172e-08, 1.6059043836821613e-10,
+                             -7.647163731819816e-13, 2.8114572543455206e-15};
+    constexpr double C[8] = {-0.5, 0.041666666666666664, -0.001388888888888889, 2.48015873015873e-05,
+                             -2.755731922398589e-07, 2.08767569878681e-09, -1.1470745597729725e-11,
+                             4.779477332387385e-14};
+    int n;
+    const double u = phase_units(ph, 2.0 * kInvPi, n);
+    const double r = fma(-u, 6.123233995736766e-17, fma(-u, 1.5707963267948966, ph)), z = r * r;
+    double p = S[7], q = C[7];
+#pragma unroll
+    for (int k = 6; k >= 0; --k) {
         p = fma(p, z, S[k]);
-        if (COS) q = fma(q, z, C[k]);
+        q = fma(q, z, C[k]);
     }
-    p *= f;
-    s = __hiloint2double(__double2hiint(p) ^ (int)sgn, __double2loint(p));
-    if (COS) c = __hiloint2double(__double2hiint(q) ^ (int)sgn, __double2loint(q));
+    p = fma(r * z, p, r);
+    q = fma(q, z, 1.0);
+    s = flip(n & 1 ? q : p, n >> 1);
+    c = flip(n & 1 ? p : q, (n + 1) >> 1);
 }
 
 // The same for a phase in radians (one FP64 multiply by 1 / pi first).

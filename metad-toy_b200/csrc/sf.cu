@@ -171,7 +171,8 @@ __global__ void __launch_bounds__(kBlock) k_debye_force(DebyeDev<T> d, const dou
 // in FP64, those reductions were 10 of 26 instructions per atom-k pair.)
 // In mixed precision the phase (k / pi).x is formed in FP64 (B200 runs FP64 at
 // half the FP32 rate) with its fraction left in the low word (kTurnBase), and
-// finished with FP32 polynomials on the pair of k-vectors (turn_sincos2); a
+// finished with FP32 polynomials on the pair of k-vectors (turn_sincos2); FP64
+// mode keeps the phase in radians (phase_sincos_f64).  A
 // per-dimension FP32 phase-table variant (three shared-memory loads and an
 // FP32 reduction per pair) measured 2.2x slower and was removed.
 // The shapes the autotuner picks (SkDev::qv: 2, 4 or 8 atoms in flight per
@@ -210,6 +211,19 @@ __device__ __forceinline__ void sk_pair(bool far, double2 kx, double2 ky, double
     }
 }
 
+// Phases beyond kPhaseMax, out of the passes' way: sin and cos, and sin(ph - shift).
+// There the last bit of a phase is a quarter radian and more, so the rounding of
+// ph / pi adds nothing (sincos() has a stack frame, 1.3 us on a 20 us kernel).
+__device__ __noinline__ double2 far_sincos(double ph) {
+    double2 v;
+    sincospi(ph * kInvPi, &v.x, &v.y);
+    return v;
+}
+__device__ __noinline__ double far_sin(double ph, double shift) {
+    const double2 a = far_sincos(ph), b = far_sincos(shift);
+    return a.x * b.y - a.y * b.x;
+}
+
 // Threads are streams of np (a tile's pairs of k) each: stream s of S takes
 // staged atoms s, s + S, ....  Block b sums atoms b * per .. (b + 1) * per - 1.
 // Bound by the SM's dispatch: 21 instructions per atom-k pair, of which the 3
@@ -226,16 +240,17 @@ template <bool FP64, int U> __global__ void __launch_bounds__(256, FP64 ? 2 : 4)
     const int np = (d.K + 1) / 2, ntile = (np + 63) / 64, TP = (np + ntile - 1) / ntile, S = (int)blockDim.x / TP;
     const int st = threadIdx.x / TP, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int a0 = min(blockIdx.x * per, d.nown), a1 = min(a0 + per, d.nown);
-    const double reach = FP64 ? 0.0 : kTurnMax / fmax(sk_kmax(d, smem), 1e-300);
+    const double reach = (FP64 ? kPhaseMax * kInvPi : kTurnMax) / fmax(sk_kmax(d, smem), 1e-300);
     int total = 0;
     for (int tile = 0; tile < ntile; ++tile) {
         const int p = tile * TP + (int)threadIdx.x % TP;
         const bool active = st < S && p < np;
+        constexpr double unit = FP64 ? 1.0 : kInvPi;
         double2 kv[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c)   // an odd K is filled up with a zero vector, whose sums are not written
-            kv[c] = make_double2(active ? d.k[6 * p + c] * kInvPi : 0.0,
-                                 active && 2 * p + 1 < d.K ? d.k[6 * p + 3 + c] * kInvPi : 0.0);
+            kv[c] = make_double2(active ? d.k[6 * p + c] * unit : 0.0,
+                                 active && 2 * p + 1 < d.K ? d.k[6 * p + 3 + c] * unit : 0.0);
         double c64[2] = {0.0, 0.0}, s64[2] = {0.0, 0.0};
         for (int c0 = a0; c0 < a1; c0 += kSkChunk) {
             // the group's atoms of the chunk, in order
@@ -270,22 +285,35 @@ template <bool FP64, int U> __global__ void __launch_bounds__(256, FP64 ? 2 : 4)
                     zz[at] = pz[r];
                 }
             }
-            const bool any_far = __syncthreads_or(is_far && !FP64);
+            const bool any_far = __syncthreads_or(is_far);
             total += m;
             if (!active) continue;
             int j = st;
             if constexpr (FP64) {
-#pragma unroll U
-                for (; j < m; j += S) {
+                auto sum = [&](double ph, bool far, int e) {
+                    double s, c;
+                    if (far) {
+                        const double2 v = far_sincos(ph);
+                        s = v.x;
+                        c = v.y;
+                    } else {
+                        phase_sincos_f64(ph, s, c);
+                    }
+                    c64[e] += c;
+                    s64[e] += s;
+                };
+                auto add = [&](bool far) {
                     const double2 q = xy[j];
                     const double z = zz[j];
-                    double s, c;
-                    halfturn_sincos_f64<true>(fma(kv[2].x, z, fma(kv[1].x, q.y, kv[0].x * q.x)), s, c);
-                    c64[0] += c;
-                    s64[0] += s;
-                    halfturn_sincos_f64<true>(fma(kv[2].y, z, fma(kv[1].y, q.y, kv[0].y * q.x)), s, c);
-                    c64[1] += c;
-                    s64[1] += s;
+                    sum(fma(kv[2].x, z, fma(kv[1].x, q.y, kv[0].x * q.x)), far, 0);
+                    sum(fma(kv[2].y, z, fma(kv[1].y, q.y, kv[0].y * q.x)), far, 1);
+                };
+                if (!any_far) {
+#pragma unroll U
+                    for (; j < m; j += S) add(false);
+                } else {
+#pragma unroll 1
+                    for (; j < m; j += S) add(!(fabs(xy[j].x) + fabs(xy[j].y) + fabs(zz[j]) < reach));
                 }
             } else {
                 while (j < m) {
@@ -375,9 +403,10 @@ __device__ __forceinline__ void sk_apply(const SkDev &d, const SysDev &s, const 
 
 // Force pass, AT atoms per thread and tile (atoms tile * 256 * AT + a * 256 +
 // threadIdx.x), tiles over a grid of resident blocks.  One sine per pair:
-// Im rho cos(k.x) - Re rho sin(k.x) = -|rho| sin(pi (u - u_rho)), with the
-// phase of rho(k) in half turns u_rho set off the phase sum's start and |rho|
-// multiplied into k, both formed once per block.  k-vectors go in pairs, with
+// Im rho cos(k.x) - Re rho sin(k.x) = -|rho| sin(k.x - arg rho), with the
+// phase of rho(k) set off the phase sum's start (FP64: taken off its remainder) and
+// |rho| multiplied into k (FP64: the sine), both formed once per block; phases in
+// half turns in mixed precision.  k-vectors go in pairs, with
 // the sums over the even and the odd k kept apart and added at the end, so the
 // forces do not depend on U, AT or the grid.
 // Bound by dispatch as the value pass (16 instructions a pair, 27 cycles).
@@ -397,17 +426,17 @@ __global__ void __launch_bounds__(256, FP64 ? 2 : 4)
     for (int q = threadIdx.x; q < 2 * np; q += blockDim.x) {
         const bool real = q < d.K;   // an odd K is filled up with a zero vector
         const double re = real ? d.rho[2 * q] : 0.0, im = real ? d.rho[2 * q + 1] : 0.0;
-        const double amp = -sqrt(re * re + im * im), ph = atan2(im, re) * kInvPi;
+        const double amp = -sqrt(re * re + im * im), ph = atan2(im, re);
         double *kd = reinterpret_cast<double *>(kp) + q / 2 * 8 + q % 2;
         for (int c = 0; c < 3; ++c) {
             const double kc = real ? d.k[3 * q + c] : 0.0;
-            kd[2 * c] = kc * kInvPi;
+            kd[2 * c] = FP64 ? kc : kc * kInvPi;
             if (!FP64) reinterpret_cast<float *>(wf)[q / 2 * 6 + 2 * c + q % 2] = (float)(amp * kc);
         }
-        if (FP64) reinterpret_cast<double *>(wd)[q] = amp * kPi;   // on k / pi
-        kd[6] = FP64 ? -ph : kTurnBase - ph;
+        if (FP64) reinterpret_cast<double *>(wd)[q] = amp;
+        kd[6] = FP64 ? ph : kTurnBase - ph * kInvPi;
     }
-    const double reach = FP64 ? 0.0 : kTurnMax / fmax(sk_kmax(d, smem), 1e-300);
+    const double reach = (FP64 ? kPhaseMax * kInvPi : kTurnMax) / fmax(sk_kmax(d, smem), 1e-300);
     __syncthreads();
     for (int tile = blockIdx.x; tile * 256 * AT < d.n; tile += gridDim.x) {
         using R2 = typename std::conditional<FP64, double2, float2>::type;
@@ -422,20 +451,17 @@ __global__ void __launch_bounds__(256, FP64 ? 2 : 4)
             y[t] = on[t] ? d.x[3 * i + 1] : 0.0;
             z[t] = on[t] ? d.x[3 * i + 2] : 0.0;
             fx[t].x = fy[t].x = fz[t].x = fx[t].y = fy[t].y = fz[t].y = 0;
-            far[t] = !FP64 && !(fabs(x[t]) + fabs(y[t]) + fabs(z[t]) < reach);
+            far[t] = !(fabs(x[t]) + fabs(y[t]) + fabs(z[t]) < reach);
             any = any || on[t];
             any_far = any_far || far[t];
         }
         auto add_pair = [&](int q, int t, bool is_far) {
             const double2 kx = kp[4 * q], ky = kp[4 * q + 1], kz = kp[4 * q + 2], base = kp[4 * q + 3];
-            double ua = fma(kz.x, z[t], fma(ky.x, y[t], fma(kx.x, x[t], base.x)));
-            double ub = fma(kz.y, z[t], fma(ky.y, y[t], fma(kx.y, x[t], base.y)));
+            double ua = fma(kz.x, z[t], fma(ky.x, y[t], FP64 ? kx.x * x[t] : fma(kx.x, x[t], base.x)));
+            double ub = fma(kz.y, z[t], fma(ky.y, y[t], FP64 ? kx.y * x[t] : fma(kx.y, x[t], base.y)));
             if constexpr (FP64) {
-                double sa, sb, c;
-                halfturn_sincos_f64<false>(ua, sa, c);
-                halfturn_sincos_f64<false>(ub, sb, c);
-                sa *= wd[q].x;
-                sb *= wd[q].y;
+                const double sa = (is_far ? far_sin(ua, base.x) : phase_sin_f64(ua, base.x)) * wd[q].x;
+                const double sb = (is_far ? far_sin(ub, base.y) : phase_sin_f64(ub, base.y)) * wd[q].y;
                 fx[t] = make_double2(fma(sa, kx.x, fx[t].x), fma(sb, kx.y, fx[t].y));
                 fy[t] = make_double2(fma(sa, ky.x, fy[t].x), fma(sb, ky.y, fy[t].y));
                 fz[t] = make_double2(fma(sa, kz.x, fz[t].x), fma(sb, kz.y, fz[t].y));
