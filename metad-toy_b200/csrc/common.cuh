@@ -292,6 +292,9 @@ __device__ __forceinline__ void halfturn_sincos_f32(double u, float &s, float &c
 // in the bit above it and the low word's sign.  Three FP64 additions and the
 // FP64-to-FP32 conversion (0.44 warp instructions per clock and SM, against
 // 0.95 for the integer one) are gone.  Valid for |u| < 2^18 (kTurnMax).
+// Rms errors against 80 bits of the passes that reduced each phase in FP64, and of
+// these (1,372 to 256,000 atoms, 12 and 24 k): S(k) 3.6e-8 to 5.9e-8 and 3.6e-8 to
+// 4.9e-8, forces 1.33e-7 to 1.66e-7 and 1.12e-7 to 1.54e-7, no size larger.
 constexpr double kTurnBase = 1572864.0;
 constexpr double kTurnMax = 262144.0;
 
@@ -326,9 +329,10 @@ __device__ __forceinline__ void turn_sincos2(double ta, double tb, float2 &s0, f
 // FP64: a phase in radians less n half turns (or quarters), pi in two words
 // (Cody and Waite, Software Manual for the Elementary Functions, 1980): both
 // products are exact inside their FMA up to n = 2^51, so the remainder is off by
-// its own rounding.  The phase itself is not scaled first: a k.x / pi is rounded
-// once more than k.x, and with k.x of some hundred radians that was a third of
-// the forces' error.  |phase| < 2^50 (kPhaseMax).
+// its own rounding.  The phase itself is not scaled first: k / pi is rounded once
+// more than k, and with k.x of some hundred radians the phase is most of an error
+// (rms of the forces against 80 bits, 55,296 atoms x 12 k: 2.9e-14 scaled, 2.2e-14
+// so, 2.6e-14 with sincos() of k.x).  |phase| < 2^50 (kPhaseMax).
 constexpr double kPhaseMax = 1125899906842624.0;
 __device__ __forceinline__ double phase_units(double ph, double per_unit, int &n) {
     constexpr double kRound = 6755399441055744.0;   // 1.5 * 2^52

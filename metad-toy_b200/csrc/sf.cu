@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kBlock) k_debye_force(DebyeDev<T> d, const dou
 // loop over k) leave every sum's order as it is.
 constexpr int kSkBlocks = 148 * 4;   // resident blocks of both passes
 constexpr int kSkChunk = 512;        // atoms staged at a time in the value pass
-constexpr int kSkFlush = 8;          // atoms summed in FP32 before they join the FP64 sums
+constexpr int kSkFlush = 8;          // most atoms summed in FP32 before they join the FP64 sums
 
 // Largest |component| of k / pi over all k-vectors, on every thread of the
 // block: |u| of an atom is at most that times |x| + |y| + |z|.
@@ -230,8 +230,10 @@ __device__ __noinline__ double far_sin(double ph, double shift) {
 // FP64 and 7 paired FP32 ones take two cycles each (38 cycles a pair are
 // measured, the FMA pipe is 46 % busy).  1,048,576 atoms x 96 k: 147 us before
 // (26 instructions with 6 FP64 and the slow conversion, atoms over the
-// threads), 112 now; FP64 at 108,000 x 24: 22 us (sincos()), 17 now.
-template <bool FP64, int U> __global__ void __launch_bounds__(256, FP64 ? 2 : 4) k_sk_partial(SkDev d, int per) {
+// threads), 114 now; FP64 at 108,000 x 24: 22 us (sincos()), 19 now, 157,216 x 90:
+// 80 and 44.
+template <bool FP64, int U, int F>
+__global__ void __launch_bounds__(256, FP64 ? 2 : 4) k_sk_partial(SkDev d, int per) {
     pdl_entry();
     __shared__ double2 xy[kSkChunk];
     __shared__ double zz[kSkChunk];
@@ -316,33 +318,46 @@ template <bool FP64, int U> __global__ void __launch_bounds__(256, FP64 ? 2 : 4)
                     for (; j < m; j += S) add(!(fabs(xy[j].x) + fabs(xy[j].y) + fabs(zz[j]) < reach));
                 }
             } else {
-                while (j < m) {
-                    float2 fc = make_float2(0.f, 0.f), fs = fc;
-                    auto add = [&](int e, bool far) {
-                        const double2 q = xy[e];
-                        float2 s0, c0f;
-                        unsigned ga, gb;
-                        sk_pair(far, kv[0], kv[1], kv[2], q.x, q.y, zz[e], s0, c0f, ga, gb);
-                        // the sign (-1)^n as a factor of exact FMAs: the same sums
-                        // as adding the signed sin and cos
-                        const float2 sg = make_float2(__uint_as_float(0x3f800000u | ga), __uint_as_float(0x3f800000u | gb));
-                        fc = __ffma2_rn(sg, c0f, fc);
-                        fs = __ffma2_rn(sg, s0, fs);
-                    };
-                    if (!any_far && j + (kSkFlush - 1) * S < m) {
-#pragma unroll U
-                        for (int e = 0; e < kSkFlush; ++e) add(j + e * S, false);
-                    } else {
-                        for (int e = j; e < min(m, j + kSkFlush * S); e += S) {
-                            const double2 q = xy[e];
-                            add(e, !(fabs(q.x) + fabs(q.y) + fabs(zz[e]) < reach));
-                        }
-                    }
-                    j += kSkFlush * S;
+                constexpr int kOuter = U > F ? U / F : 1, kInner = U < F ? U : F;
+                float2 fc, fs;
+                auto add = [&](int e, bool far) {
+                    const double2 q = xy[e];
+                    float2 s0, c0f;
+                    unsigned ga, gb;
+                    sk_pair(far, kv[0], kv[1], kv[2], q.x, q.y, zz[e], s0, c0f, ga, gb);
+                    // the sign (-1)^n as a factor of exact FMAs: the same sums
+                    // as adding the signed sin and cos
+                    const float2 sg = make_float2(__uint_as_float(0x3f800000u | ga), __uint_as_float(0x3f800000u | gb));
+                    fc = __ffma2_rn(sg, c0f, fc);
+                    fs = __ffma2_rn(sg, s0, fs);
+                };
+                auto flush = [&] {
                     c64[0] += (double)fc.x;
                     c64[1] += (double)fc.y;
                     s64[0] += (double)fs.x;
                     s64[1] += (double)fs.y;
+                };
+                for (; j < m; j += kSkFlush * S) {
+                    if (!any_far && j + (kSkFlush - 1) * S < m) {
+#pragma unroll kOuter
+                        for (int e = 0; e < kSkFlush; e += F) {
+                            fc = fs = make_float2(0.f, 0.f);
+#pragma unroll kInner
+                            for (int t = 0; t < F; ++t) add(j + (e + t) * S, false);
+                            flush();
+                        }
+                    } else {
+#pragma unroll 1
+                        for (int e = j; e < min(m, j + kSkFlush * S);) {
+                            fc = fs = make_float2(0.f, 0.f);
+#pragma unroll 1
+                            for (int t = 0; t < F && e < m; ++t, e += S) {
+                                const double2 q = xy[e];
+                                add(e, !(fabs(q.x) + fabs(q.y) + fabs(zz[e]) < reach));
+                            }
+                            flush();
+                        }
+                    }
                 }
             }
         }
@@ -411,7 +426,7 @@ __device__ __forceinline__ void sk_apply(const SkDev &d, const SysDev &s, const 
 // forces do not depend on U, AT or the grid.
 // Bound by dispatch as the value pass (16 instructions a pair, 27 cycles).
 // 1,048,576 atoms x 96 k: 119 us before (sine and cosine, 3 more FP64
-// additions), 82 now; FP64 at 108,000 x 24: 16 us, 14 now.
+// additions), 82 now; FP64 at 108,000 x 24: 16 us, 15 now, 157,216 x 90: 60 and 39.
 template <bool FP64, int U, int AT>
 __global__ void __launch_bounds__(256, FP64 ? 2 : 4)
     k_sk_force(SkDev d, const double *__restrict__ f_src, double *__restrict__ f_dst, SysDev s, CellGrid g,
@@ -548,10 +563,19 @@ int sk_blocks(int n) {
     return b < kSkBlocks ? (b < 1 ? 1 : b) : kSkBlocks;
 }
 
+// Atoms summed in FP32 before they join the FP64 sums: as many as a thread of a
+// grid-wide loop of 256 threads a block has, rounded down to a power of two, so one
+// (every term goes into an FP64 sum) up to 303,104 atoms and four at 1,048,576.
+// Value pass with one and with eight throughout: 42.6 us and 38.1 at 296,352 atoms x
+// 90, 16.3 and 15.7 at 108,000 x 24; with four and eight 113.6 and 111.3 at
+// 1,048,576 x 96.
 template <int U> static void launch_sk_partial_u(const SkDev &d, cudaStream_t st) {
     const int per = (d.nown + d.nblocks - 1) / d.nblocks;
-    if (d.fp64) launch_k(k_sk_partial<true, U>, d.nblocks, 256, 0, st, d, per);
-    else launch_k(k_sk_partial<false, U>, d.nblocks, 256, 0, st, d, per);
+    if (d.fp64) launch_k(k_sk_partial<true, U, 1>, d.nblocks, 256, 0, st, d, per);
+    else if (per < 2 * 256) launch_k(k_sk_partial<false, U, 1>, d.nblocks, 256, 0, st, d, per);
+    else if (per < 4 * 256) launch_k(k_sk_partial<false, U, 2>, d.nblocks, 256, 0, st, d, per);
+    else if (per < 8 * 256) launch_k(k_sk_partial<false, U, 4>, d.nblocks, 256, 0, st, d, per);
+    else launch_k(k_sk_partial<false, U, kSkFlush>, d.nblocks, 256, 0, st, d, per);
 }
 
 template <int U>

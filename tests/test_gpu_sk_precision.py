@@ -53,3 +53,34 @@ def test_fp64_phases_without_end_stay_sines_and_cosines(far, n):
     cv, f, _ = _step(x, 5, "fp64", hi=1000.0)
     assert abs(cv - n) <= n * 1e-13
     assert np.abs(f).max() <= 1e-10
+
+
+@pytest.mark.parametrize("n", [100, 5000, 108000, 250000])
+@pytest.mark.parametrize("nk", [3, 24])
+def test_mixed_terms_join_an_fp64_sum(n, nk):
+    """n atoms at one place: every term is the same FP32 number, its n-fold sum is
+    exact in FP64, so S(k) is n times that of one atom up to FP64 roundings (a few
+    2^-53 of the squares, their sums over k, the mean)."""
+    at = np.array([[11.3, 4.7, 29.9]])
+    one, _, _ = _step(at, nk, "mixed", L=[64.0] * 3)
+    cv, _, _ = _step(np.tile(at, (n, 1)), nk, "mixed", L=[64.0] * 3, hi=4.0 * n)
+    assert abs(cv - n * one) <= n * (nk + 8) * 2.0 ** -52
+
+
+@pytest.mark.parametrize("nk,far", [(13, 0), (129, 40)])
+@pytest.mark.parametrize("virial", [False, True])
+def test_mixed_forces_do_not_depend_on_the_atoms_per_thread(nk, far, virial):
+    """The same group of 20,000 atoms alone (one atom a thread in the force pass) and
+    with 160,000 others outside the group (two), some of the group so far out that
+    their phases leave the base's range: the FP32 sums over k are the same, and the
+    forces with them up to the FP64 sum over atoms, taken over other blocks
+    (1e-16 of it each, 2^-44 allowed; an FP32 sum in another order differs by 2^-24)."""
+    rng = np.random.default_rng(nk)
+    L = np.array([150.0] * 3)
+    x = rng.random((180000, 3)) * L
+    x[rng.choice(20000, far, replace=False)] += L * rng.integers(9000, 12000, (far, 3))
+    mask = np.where(np.arange(len(x)) < 20000, 3, 1).astype(np.int32)
+    cv1, f1, _ = _step(x[:20000].copy(), nk, "mixed", L=L, mask=mask[:20000], virial=virial)
+    cv2, f2, _ = _step(x, nk, "mixed", L=L, mask=mask, virial=virial)
+    assert abs(cv1 - cv2) <= 1e-13 * cv1 and not np.any(f2[20000:])
+    assert np.abs(f1).max() > 0 and np.all(np.abs(f1 - f2[:20000]) <= 2.0 ** -44 * np.abs(f1))
