@@ -294,7 +294,7 @@ __device__ __forceinline__ void halfturn_sincos_f32(double u, float &s, float &c
 // 0.95 for the integer one) are gone.  Valid for |u| < 2^18 (kTurnMax).
 // Rms errors against 80 bits of the passes that reduced each phase in FP64, and of
 // these (1,372 to 256,000 atoms, 12 and 24 k): S(k) 3.6e-8 to 5.9e-8 and 3.6e-8 to
-// 4.9e-8, forces 1.33e-7 to 1.66e-7 and 1.12e-7 to 1.54e-7, no size larger.
+// 4.9e-8, forces 1.33e-7 to 1.66e-7 and 1.12e-7 to 1.54e-7.
 constexpr double kTurnBase = 1572864.0;
 constexpr double kTurnMax = 262144.0;
 

@@ -163,8 +163,8 @@ __device__ __forceinline__ void pair_add(const double2 *__restrict__ rec, const 
     const double2 a = rec[0], b = rec[kBuf], wq = rec[2 * kBuf], ic = rec[3 * kBuf];
     const double d0 = s[0] - a.x, d1 = s[1] - a.y, d2 = s[2] - b.x, d3 = s[3] - b.y;
     double r2 = fma(d3, d3, fma(d2, d2, fma(d1, d1, d0 * d0)));
-    // r2 >= 0: the high words compare as integers (a NaN is above every cut)
-    const bool in = (unsigned)__double2hiint(r2) < (unsigned)__double2hiint(ic.y);
+    // r2 >= 0: it compares as an integer, off the FP64 pipe (a NaN is above every cut)
+    const bool in = (unsigned long long)__double_as_longlong(r2) < (unsigned long long)__double_as_longlong(ic.y);
     r2 = in ? r2 : 0.0;
     const double t = fma(r2, wq.y, kMagic);
     const int n = __double2loint(t);

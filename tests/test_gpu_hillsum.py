@@ -160,3 +160,22 @@ def test_widths_at_the_ends_of_the_range():
     want = -0.25 * (p[3] - p[0]) / 1e302
     assert np.all(np.abs(dV[3] - want) <= 1e-13 * np.abs(want))
     nb.close()
+
+
+@pytest.mark.parametrize("D", [1, 3, 4])
+def test_a_hill_counts_to_the_last_bit_of_its_cut(D):
+    """Points at r^2 = 80 sigma^2 (1 -+ 1e-9): within the cut the hill's full value,
+    40 * 2e-9 of the exponent off e^-40 at most, beyond it nothing."""
+    s = np.array([0.55, 1.1, 1.3])
+    e = np.array([-1e-9, 1e-9])
+    p = np.zeros((6, D))
+    p[:, D - 1] = np.sqrt(80 * s[:, None] ** 2 * (1 + e)).ravel()
+    for k in range(3):
+        nb = mtd.NNBias(np.full(D, -20.0), np.full(D, 20.0))
+        nb.add_hills(np.zeros((1, D)), np.array([1e18]), s[k:k + 1])
+        V, dV = nb.exact(p[2 * k:2 * k + 2])
+        want = 1e18 * np.exp(-40.0 * (1 - 1e-9))
+        assert abs(V[0] - want) <= 1e-12 * want and V[1] == 0
+        g = -want * p[2 * k, D - 1] / s[k] ** 2
+        assert abs(dV[0, D - 1] - g) <= 1e-12 * abs(g) and not np.any(dV[1])
+        nb.close()
