@@ -505,8 +505,12 @@ mtd_status mtd_nnbias_point_device(mtd_nnbias *nb, const double *d_s, double *d_
 
 /* Bias at npts device-resident points (rows of D doubles) into d_V (npts) and
  * d_dV (npts rows of D; NULL = values only), enqueued on `stream`; use_nn as
- * above.  The network path keeps grow-only scratch in the object (allocated
- * on the first call of a larger batch).  No counterpart in the reference. */
+ * above.  The exact sum keeps grow-only scratch in the object: a call whose
+ * batch or hill list is larger than any before allocates it, after waiting on
+ * the host for the object's previous batches; the network path needs none.  In
+ * a stream capture either path is one kernel node, without scratch, with the
+ * same results (of the exact sum at about three times the time of a large
+ * batch).  No counterpart in the reference. */
 mtd_status mtd_nnbias_eval_device(mtd_nnbias *nb, int npts, const double *d_pts, double *d_V, double *d_dV,
                                   int use_nn, void *stream);
 

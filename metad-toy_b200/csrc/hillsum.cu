@@ -65,6 +65,20 @@ __device__ __forceinline__ int cell_of(const Cells &c, int D, const double *__re
     return key;
 }
 
+// Hill h packed for pair_add; past nh a cut of 0, which reaches no point.
+__device__ __forceinline__ void load_hill(const double *__restrict__ hills, int h, int nh, double2 (&r)[4]) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) r[e] = make_double2(0.0, 0.0);
+    if (h < nh) {
+        const double2 *src = reinterpret_cast<const double2 *>(hills + (size_t)h * kHillRec);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) r[e] = src[e];
+        // 32 log2(e) / (2 sigma^2); finite, so that a hill on the point itself has the exponent 0
+        r[2].y = fmin(r[2].y * (1.4426950408889634074 * kTab), 1.7976931348623157e308);
+        if (!isfinite(r[3].x)) r[3].y = 0.0;      // a width whose 1 / sigma^2 overflows reaches no point
+    }
+}
+
 // Blocks below `npb` count the points of each cell; the others, one warp per
 // group of 32 hills (hills q, q + Q, ... of a run of 32 Q, for split q), write the groups' bounding boxes (rows of ng) and the
 // hills as four rows of pairs (c0 c1, c2 c3, w x/r^2, 1/sigma^2 cut), which a
@@ -81,17 +95,10 @@ __global__ void __launch_bounds__(256) k_hs_count(Cells c, int D, int npts, cons
     const int lane = threadIdx.x & 31, g = ((int)blockIdx.x - npb) * 8 + (threadIdx.x >> 5);
     const int h = g / Q * 32 * Q + lane * Q + g % Q;
     if (g >= ng) return;
-    double2 r[4] = {};
-    if (h < nh) {
-        const double2 *src = reinterpret_cast<const double2 *>(hills + (size_t)h * kHillRec);
+    double2 r[4];
+    load_hill(hills, h, nh, r);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) r[e] = src[e];
-        // 32 log2(e) / (2 sigma^2); finite, so that a hill on the point itself has the exponent 0
-        r[2].y = fmin(r[2].y * (1.4426950408889634074 * kTab), 1.7976931348623157e308);
-        if (!isfinite(r[3].x)) r[3].y = 0.0;      // a width whose 1 / sigma^2 overflows reaches no point
-    }
-#pragma unroll
-    for (int e = 0; e < 4; ++e) rows[((size_t)e * ng + g) * 32 + lane] = r[e];   // past nh: a cut of 0
+    for (int e = 0; e < 4; ++e) rows[((size_t)e * ng + g) * 32 + lane] = r[e];
     const double cen[kIn] = {r[0].x, r[0].y, r[1].x, r[1].y};
     double cut = r[3].y;
     for (int o = 16; o > 0; o >>= 1) cut = fmax(cut, __shfl_xor_sync(0xffffffffu, cut, o));
@@ -199,10 +206,13 @@ __device__ __forceinline__ double gap2(double plo, double phi, double lo, double
 // a cluster: split q of Q takes groups q, q + Q, ...; the splits' sums are
 // added in split order.  (Warps with points of their own finish apart, by their
 // share of the hills: 2.5 warps per issue waited at the block's end.)
+// RAW: the hills as they are, without the rows and boxes of a scratch, each group
+// tested hill by hill; the same sums bit for bit (a hill left out adds zeros).
+template <bool RAW>
 __global__ void __launch_bounds__(kWarps * 32, 2)
-    k_hillsum(int D, int npts, const double *__restrict__ pts, int ps, const int *__restrict__ perm, int ng,
-              const double2 *__restrict__ rows, const double *__restrict__ boxes, double *__restrict__ V,
-              double *__restrict__ dV, int gs) {
+    k_hillsum(int D, int npts, const double *__restrict__ pts, int ps, const int *__restrict__ perm, int nh,
+              const double *__restrict__ hills, int ng, const double2 *__restrict__ rows,
+              const double *__restrict__ boxes, double *__restrict__ V, double *__restrict__ dV, int gs) {
     __shared__ double2 buf[kWarps][4][kBuf];
     cg::cluster_group cl = cg::this_cluster();
     const int nsplit = cl.num_blocks(), rank = cl.block_rank();
@@ -236,8 +246,8 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
     double2 *mine = buf[warp][0];
     for (int g0 = q; g0 < ng; g0 += 32 * Q) {
         const int gl = g0 + lane * Q;
-        bool near = false;
-        if (gl < ng) {
+        bool near = RAW && gl < ng;
+        if (!RAW && gl < ng) {
             const double *bx = boxes + gl;
             double r2 = 0.0;
 #pragma unroll
@@ -248,10 +258,15 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
         while (todo) {
             const int t = __ffs(todo) - 1;
             todo &= todo - 1;
-            const double2 *src = rows + (size_t)(g0 + t * Q) * 32 + lane;
+            const int g = g0 + t * Q;
             double2 r[4];
+            if (RAW) {
+                load_hill(hills, g / Q * 32 * Q + lane * Q + g % Q, nh, r);
+            } else {
+                const double2 *src = rows + (size_t)g * 32 + lane;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) r[e] = src[(size_t)e * ng * 32];
+                for (int e = 0; e < 4; ++e) r[e] = src[(size_t)e * ng * 32];
+            }
             const double d2 = gap2(plo[0], phi[0], r[0].x, r[0].x) + gap2(plo[1], phi[1], r[0].y, r[0].y) +
                               gap2(plo[2], phi[2], r[1].x, r[1].x) + gap2(plo[3], phi[3], r[1].y, r[1].y);
             const bool hit = d2 < r[3].y;
@@ -343,15 +358,14 @@ cudaError_t hillsum_batch(int D, const double *lo, const double *hi, int npts, c
     int split = 1;
     while (split < kMaxSplit && groups * split < 148 * 2 * 8) split *= 2;
     const int Q = kWarps * split, ng = (nh + 32 * Q - 1) / (32 * Q) * Q;
-    const bool sorted = ncell > 1;
+    const bool raw = !scratch, sorted = !raw && ncell > 1;
     double2 *rows = static_cast<double2 *>(scratch);
     double *boxes = reinterpret_cast<double *>(rows + (size_t)4 * 32 * ng);
     int *count = reinterpret_cast<int *>(boxes + (size_t)kBoxRec * ng), *perm = count + ncell;
     const int npb = sorted ? (npts + 255) / 256 : 0;
     if (sorted) cudaMemsetAsync(count, 0, sizeof(int) * ncell, st);
-    if (npb + ng > 0)
-        k_hs_count<<<npb + (ng + 7) / 8, 256, 0, st>>>(c, D, npts, pts, ps, npb, count, nh, ng, Q, hills,
-                                                                       boxes, rows);
+    if (!raw && npb + ng > 0)
+        k_hs_count<<<npb + (ng + 7) / 8, 256, 0, st>>>(c, D, npts, pts, ps, npb, count, nh, ng, Q, hills, boxes, rows);
     if (sorted) {
         k_hs_scan<<<1, 1024, 0, st>>>(ncell, count);
         k_hs_place<<<npb, 256, 0, st>>>(c, D, npts, pts, ps, count, perm);
@@ -366,8 +380,10 @@ cudaError_t hillsum_batch(int D, const double *lo, const double *hi, int npts, c
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_hillsum, D, npts, pts, ps, (const int *)(sorted ? perm : nullptr),
-                                             ng, (const double2 *)rows, (const double *)boxes, V, dV, gs);
+    const cudaError_t e =
+        cudaLaunchKernelEx(&cfg, raw ? k_hillsum<true> : k_hillsum<false>, D, npts, pts, ps,
+                           (const int *)(sorted ? perm : nullptr), nh, hills, ng, (const double2 *)rows,
+                           (const double *)boxes, V, dV, gs);
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 

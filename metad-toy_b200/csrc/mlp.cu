@@ -843,20 +843,20 @@ mtd_status nb_refresh_forward(mtd_nnbias *b) {
     return MTD_OK;
 }
 
-// The batched hill sum with its scratch: the object's, or during a stream
-// capture memory of the graph's own (the object's may have grown, and so
-// moved, by the time the graph runs).
+// The batched hill sum with the object's scratch.  During a stream capture it runs
+// without any: the scratch may have grown, and so moved, by the time the graph
+// runs, and memory nodes would keep the graph from being cloned, nested or
+// instantiated twice.
 cudaError_t nb_hillsum(mtd_nnbias *b, int npts, const double *pts, int ps, double *V, double *dV, int gs,
                        cudaStream_t st) {
-    const size_t need = hillsum_scratch(npts, b->nh);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     cudaError_t e = cudaStreamIsCapturing(st, &cap);
     if (e != cudaSuccess) return e;
+    if (cap != cudaStreamCaptureStatusNone)
+        return hillsum_batch(b->D, b->lo, b->hi, npts, pts, ps, b->nh, b->d_hills, V, dV, gs, nullptr, st);
+    const size_t need = hillsum_scratch(npts, b->nh);
     std::lock_guard<std::mutex> lock(b->hs_mu);
-    void *scratch = b->d_hs;
-    if (cap != cudaStreamCaptureStatusNone) {
-        if ((e = cudaMallocAsync(&scratch, need, st)) != cudaSuccess) return e;
-    } else if (need > b->cap_hs) {
+    if (need > b->cap_hs) {
         // another thread's capture on another stream is no reason to refuse these
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
         if ((e = cudaThreadExchangeStreamCaptureMode(&mode)) != cudaSuccess) return e;
@@ -870,15 +870,10 @@ cudaError_t nb_hillsum(mtd_nnbias *b, int npts, const double *pts, int ps, doubl
         }
         cudaThreadExchangeStreamCaptureMode(&mode);
         if (e != cudaSuccess) return e;
-        scratch = b->d_hs;
     } else if ((e = cudaStreamWaitEvent(st, b->hs_ev, 0)) != cudaSuccess) {
         return e;
     }
-    e = hillsum_batch(b->D, b->lo, b->hi, npts, pts, ps, b->nh, b->d_hills, V, dV, gs, scratch, st);
-    if (cap != cudaStreamCaptureStatusNone) {
-        const cudaError_t ef = cudaFreeAsync(scratch, st);
-        return e != cudaSuccess ? e : ef;
-    }
+    e = hillsum_batch(b->D, b->lo, b->hi, npts, pts, ps, b->nh, b->d_hills, V, dV, gs, b->d_hs, st);
     const cudaError_t er = cudaEventRecord(b->hs_ev, st);
     return e != cudaSuccess ? e : er;
 }

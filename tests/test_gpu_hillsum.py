@@ -179,3 +179,48 @@ def test_a_hill_counts_to_the_last_bit_of_its_cut(D):
         g = -want * p[2 * k, D - 1] / s[k] ** 2
         assert abs(dV[0, D - 1] - g) <= 1e-12 * abs(g) and not np.any(dV[1])
         nb.close()
+
+
+@pytest.mark.parametrize("npts,nh,D", [(1, 40, 4), (500, 300, 3), (9000, 5000, 4), (40000, 700, 4)])
+def test_a_captured_batch_is_one_kernel_node(npts, nh, D):
+    """No memory nodes, so the graph can be instantiated twice and nested; the
+    sums are those of a call outside a capture, bit for bit."""
+    import torch
+    from cuda.bindings import runtime as rt
+
+    def ok(r):
+        assert r[0] == rt.cudaError_t.cudaSuccess, r[0]
+        return r[1:] if len(r) != 2 else r[1]
+
+    lo, hi = systems.CV4_LO[:D], systems.CV4_HI[:D]
+    nb = mtd.NNBias(lo, hi)
+    nb.add_hills(*_hills(nh, D, npts, True))
+    p = lo + (hi - lo) * np.random.default_rng(npts).random((npts, D))
+    d_p = torch.from_numpy(p).cuda()
+    d_v, d_g = torch.zeros(npts, dtype=torch.float64, device="cuda"), torch.zeros((npts, D), dtype=torch.float64,
+                                                                                  device="cuda")
+    torch.cuda.synchronize()
+    st = ok(rt.cudaStreamCreateWithFlags(rt.cudaStreamNonBlocking))
+    ok(rt.cudaStreamBeginCapture(st, rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal))
+    nb.eval_device(npts, d_p.data_ptr(), d_v.data_ptr(), d_g.data_ptr(), use_nn=0, stream=int(st))
+    graph = ok(rt.cudaStreamEndCapture(st))
+    n = ok(rt.cudaGraphGetNodes(graph, 0))[1]
+    nodes = ok(rt.cudaGraphGetNodes(graph, n))[0]
+    assert [ok(rt.cudaGraphNodeGetType(k)) for k in nodes[:n]] == [rt.cudaGraphNodeType.cudaGraphNodeTypeKernel]
+    outer = ok(rt.cudaGraphCreate(0))
+    ok(rt.cudaGraphAddChildGraphNode(outer, None, 0, graph))
+    execs = [ok(rt.cudaGraphInstantiate(g, 0)) for g in (graph, graph, outer)]
+    V, dV = nb.exact(p)
+    for ex in execs:
+        d_v.zero_()
+        d_g.zero_()
+        torch.cuda.synchronize()
+        ok(rt.cudaGraphLaunch(ex, st))
+        ok(rt.cudaStreamSynchronize(st))
+        assert np.array_equal(d_v.cpu().numpy(), V) and np.array_equal(d_g.cpu().numpy(), dV)
+    for ex in execs:
+        ok(rt.cudaGraphExecDestroy(ex))
+    for g in (outer, graph):
+        ok(rt.cudaGraphDestroy(g))
+    ok(rt.cudaStreamDestroy(st))
+    nb.close()
