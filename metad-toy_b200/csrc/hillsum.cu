@@ -29,11 +29,14 @@
 //     memory took 7 of the 11 wavefronts of a pair).
 // 65,536 uniform points in a 4D box, 20,000 hills (27 % of the pairs are near
 // a block's box): 5,274 us before, 990 now, with the FP64 pipe 60 % busy while
-// blocks run; error against 64-bit torch 1.9e-15 (5.4e-15 before).
+// blocks run; error against 64-bit torch 6.5e-16 (5.4e-15 before).  Sums of few
+// hills or few pairs go without the sorting, or without the blocks (few_hills,
+// few_pairs).
 #include "hillsum.h"
 
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <cmath>
 
 namespace mtd {
@@ -193,6 +196,53 @@ __device__ __forceinline__ void pair_add(const double2 *__restrict__ rec, const 
     acc.g[3] = fma(-ec, d3, acc.g[3]);
 }
 
+// A point's coordinates; one that is not finite stands at 1e150 and is written as zeros.
+__device__ __forceinline__ bool load_point(const double *__restrict__ pts, int ps, int D, int i, double (&s)[kIn]) {
+    bool fin = i >= 0;
+#pragma unroll
+    for (int k = 0; k < kIn; ++k) {
+        s[k] = i >= 0 && k < D ? pts[(size_t)i * ps + k] : 0.0;
+        fin = fin && isfinite(s[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < kIn; ++k)
+        if (!fin) s[k] = 1e150;
+    return fin;
+}
+
+// A thread per point over all hills in deposit order: for few hills, where a
+// block's box tests and the sum of its splits cost more than the pairs.
+constexpr int kPlainBlock = 128;
+__global__ void __launch_bounds__(kPlainBlock)
+    k_hillsum_plain(int D, int npts, const double *__restrict__ pts, int ps, int nh, const double *__restrict__ hills,
+                    double *__restrict__ V, double *__restrict__ dV, int gs) {
+    __shared__ double2 tile[4][kBuf];
+    const int slot = blockIdx.x * kPlainBlock + threadIdx.x, i = slot < npts ? slot : -1;
+    const double tab = exp2(-(double)(threadIdx.x & 31) / kTab);
+    double s[kIn];
+    const bool fin = load_point(pts, ps, D, i, s);
+    Acc acc{};
+    for (int h0 = 0; h0 < nh; h0 += kBuf) {
+        const int c = min(kBuf, nh - h0);
+        __syncthreads();
+        if (threadIdx.x < kBuf) {
+            double2 r[4];
+            load_hill(hills, h0 + threadIdx.x, nh, r);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) tile[e][threadIdx.x] = r[e];
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int e = 0; e < c; ++e) pair_add(tile[0] + e, s, tab, acc);
+    }
+    if (i < 0) return;
+    V[i] = fin ? acc.v : 0.0;
+    if (dV)
+#pragma unroll
+        for (int k = 0; k < kIn; ++k)
+            if (k < gs && (k < D || gs == kIn)) dV[(size_t)i * gs + k] = fin ? acc.g[k] : 0.0;
+}
+
 // Squared distance between two boxes (a point is a box of no size); NaN bounds
 // give NaN, which is below no cut.
 __device__ __forceinline__ double gap2(double plo, double phi, double lo, double hi) {
@@ -222,18 +272,12 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
     const int i = slot < npts ? (perm ? perm[slot] : slot) : -1;
     const double tab = exp2(-(double)lane / kTab);
     double s[kIn], plo[kIn], phi[kIn];
-    bool fin = i >= 0;
-#pragma unroll
-    for (int k = 0; k < kIn; ++k) {
-        s[k] = i >= 0 && k < D ? pts[(size_t)i * ps + k] : 0.0;
-        fin = fin && isfinite(s[k]);
-    }
-    // a point that is not finite is within reach of no hill: its box is empty and its sums are written as zeros
+    const bool fin = load_point(pts, ps, D, i, s);
+    // a point that is not finite is within reach of no hill: its box is empty
 #pragma unroll
     for (int k = 0; k < kIn; ++k) {
         plo[k] = fin ? s[k] : INFINITY;
         phi[k] = fin ? s[k] : -INFINITY;
-        if (!fin) s[k] = 1e150;
     }
 #pragma unroll
     for (int k = 0; k < kIn; ++k)
@@ -288,34 +332,35 @@ __global__ void __launch_bounds__(kWarps * 32, 2)
     }
     __syncwarp();
     for (int e = 0; e < held; ++e) pair_add(mine + e, s, tab, acc);
-    // the splits' sums, [5][block thread], over the hill buffers
+    // the warps' sums, [5][warp][lane] over the hill buffers, by five warps in warp
+    // order; then the blocks' of the cluster, [5][lane] behind them, in block order
     constexpr int kT = kWarps * 32;
+    static_assert(sizeof(buf) >= (1 + kIn) * (kT + 32) * sizeof(double) && kWarps > kIn, "room and warps for the sums");
     __syncthreads();
-    double *red = &buf[0][0][0].x;
+    double *red = &buf[0][0][0].x, *tot = red + (1 + kIn) * kT;
     red[threadIdx.x] = acc.v;
 #pragma unroll
     for (int k = 0; k < kIn; ++k) red[(1 + k) * kT + threadIdx.x] = acc.g[k];
-    cl.sync();
-    if (rank == 0 && warp == 0) {
-        double o[1 + kIn] = {0, 0, 0, 0, 0};
-        for (int b = 0; b < nsplit; ++b) {
-            const double *rb = cl.map_shared_rank(red, b) + lane;
-            for (int w = 0; w < kWarps; ++w)
+    __syncthreads();
+    double o = 0.0;
+    if (warp <= kIn) {
 #pragma unroll
-                for (int k = 0; k < 1 + kIn; ++k) o[k] += rb[k * kT + w * 32];
-        }
-        if (!fin)
-#pragma unroll
-            for (int k = 0; k < 1 + kIn; ++k) o[k] = 0.0;
-        if (i >= 0) {
-            V[i] = o[0];
-            if (dV)
-#pragma unroll
-                for (int k = 0; k < kIn; ++k)
-                    if (k < gs && (k < D || gs == kIn)) dV[(size_t)i * gs + k] = o[1 + k];
-        }
+        for (int w = 0; w < kWarps; ++w) o += red[warp * kT + w * 32 + lane];
     }
-    cl.sync();
+    if (nsplit > 1) {
+        if (warp <= kIn) tot[warp * 32 + lane] = o;
+        cl.sync();
+        if (rank == 0 && warp <= kIn) {
+            o = 0.0;
+            for (int b = 0; b < nsplit; ++b) o += cl.map_shared_rank(tot, b)[warp * 32 + lane];
+        }
+        cl.sync();   // no block leaves while another reads its sums
+    }
+    if (rank == 0 && i >= 0) {
+        if (!fin) o = 0.0;
+        if (warp == 0) V[i] = o;
+        else if (dV && warp <= gs && (warp <= D || gs == kIn)) dV[(size_t)i * gs + warp - 1] = o;
+    }
 }
 
 }  // namespace
@@ -340,7 +385,40 @@ int make_cells(Cells &c, int D, const double *lo, const double *hi, int npts) {
 }
 }  // namespace
 
+// The routes, by measurement (4D, 1 to 20,000 hills, 500 to 65,536 points; us):
+// Few hills on many points: a thread per point.  Blocks of 32 points cost 3 to 5 us
+// a round (two blocks an SM: 9,472 points) whatever the hills.  More than two
+// rounds: 100 hills, 37,000 points 15 and 21 in blocks, 65,536 points 21 and 35;
+// 300 hills 37 and 39, 54 and 57; but 600 hills on 65,536 points 101 and 70.  More
+// than one: 16,000 points 6.0 and 9.2 with 10 hills, 8.7 and 10.7 with 50, but 14
+// and 13 with 100.  8,000 points 8.6 and 6.7 with 50.
+static bool few_hills(int npts, int nh) {
+    constexpr int round = 32 * 2 * 148;
+    return (nh <= 300 && npts > 2 * round) || (nh <= 64 && npts > round);
+}
+
+// Few pairs: no sorting and no group boxes, whose kernels cost about 18 us.  1,000
+// hills, 4,000 points 19 and 33 sorted, 8,000 points 29 and 41, 16,000 points 54
+// and 48; 2,500 hills, 4,000 points 36 and 44, 8,000 points 64 and 56; 10,000
+// hills, 1,000 points 36 and 48; but 20,000 hills, 500 points 64 and 54: every
+// pair of an unsorted block is computed, 3.2 us per 1,000 hills at least.
+static bool few_pairs(int npts, int nh) { return nh <= 12000 && (long long)npts * nh <= 12000000; }
+
+// Blocks of a cluster that split the hills: as many as are resident (two an SM),
+// times a wave for each 2,500 hills up to eight, since the points' shares of the
+// hills are unequal.  A split costs each block its box tests, half-full buffers and
+// the sum over the cluster: 20,000 hills, 65,536 points 1,024 in one block each,
+// 989 in two, 1,076 in four, 4,000 points 269, 222, 154 and 144 in eight; 1,000
+// hills, 16,000 points 48, 53, 65 and 99, 500 points 33, 27, 24 and 23.
+static int splits(int npts, int nh) {
+    const double blocks = 148 * 2 * std::min(8.0, nh / 2500.0);
+    int split = 1;
+    while (split < kMaxSplit && (npts + 31) / 32 * split < blocks) split *= 2;
+    return split;
+}
+
 size_t hillsum_scratch(int npts, int nh) {
+    if (few_hills(npts, nh) || few_pairs(npts, nh)) return 0;
     const size_t run = 32 * kWarps * kMaxSplit, ng = (nh + run - 1) / run * (run / 32);
     return sizeof(double2) * 4 * 32 * ng + sizeof(double) * kBoxRec * ng + sizeof(int) * ((size_t)kMaxCells + npts);
 }
@@ -348,16 +426,15 @@ size_t hillsum_scratch(int npts, int nh) {
 cudaError_t hillsum_batch(int D, const double *lo, const double *hi, int npts, const double *pts, int ps, int nh,
                           const double *hills, double *V, double *dV, int gs, void *scratch, cudaStream_t st) {
     if (npts <= 0) return cudaSuccess;
+    const int nsplit = splits(npts, nh);
+    if (few_hills(npts, nh)) {
+        k_hillsum_plain<<<(npts + kPlainBlock - 1) / kPlainBlock, kPlainBlock, 0, st>>>(D, npts, pts, ps, nh, hills, V, dV,
+                                                                                       gs);
+        return cudaGetLastError();
+    }
     Cells c{};
     const int ncell = make_cells(c, D, lo, hi, npts);
-    // a cluster splits the hills further until there are eight waves of
-    // blocks (two an SM): the points' shares of the hills are unequal, and 65,536
-    // points took 1,040 us in one block each, 990 in two, 1,160 in four (the box
-    // tests and half-full buffers of each split)
-    const int groups = (npts + 31) / 32;
-    int split = 1;
-    while (split < kMaxSplit && groups * split < 148 * 2 * 8) split *= 2;
-    const int Q = kWarps * split, ng = (nh + 32 * Q - 1) / (32 * Q) * Q;
+    const int Q = kWarps * nsplit, ng = (nh + 32 * Q - 1) / (32 * Q) * Q;
     const bool raw = !scratch, sorted = !raw && ncell > 1;
     double2 *rows = static_cast<double2 *>(scratch);
     double *boxes = reinterpret_cast<double *>(rows + (size_t)4 * 32 * ng);
@@ -371,12 +448,12 @@ cudaError_t hillsum_batch(int D, const double *lo, const double *hi, int npts, c
         k_hs_place<<<npb, 256, 0, st>>>(c, D, npts, pts, ps, count, perm);
     }
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(groups * split));
+    cfg.gridDim = dim3((unsigned)((npts + 31) / 32 * nsplit));
     cfg.blockDim = dim3(kWarps * 32);
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)split;
+    at[0].val.clusterDim.x = (unsigned)nsplit;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;

@@ -14,8 +14,9 @@ constexpr int kHillRec = 8;
 // written, all gs when gs is 4) at npts device points (rows of ps >= D
 // doubles), enqueued on st.  [lo, hi] is the box that the points are expected
 // in: it shapes the spatial order only, points outside are as good.  `scratch`
-// (hillsum_scratch bytes, any contents) is in use until the call has run; without
-// it (null) the sum is one kernel that leaves out fewer hills, with the same results.
+// (hillsum_scratch bytes, any contents; small sums need none) is in use until the
+// call has run; without it (null) the sum is one kernel that leaves out fewer
+// hills, with the same results.
 size_t hillsum_scratch(int npts, int nh);
 cudaError_t hillsum_batch(int D, const double *lo, const double *hi, int npts, const double *pts, int ps, int nh,
                           const double *hills, double *V, double *dV, int gs, void *scratch, cudaStream_t st);

@@ -852,9 +852,8 @@ cudaError_t nb_hillsum(mtd_nnbias *b, int npts, const double *pts, int ps, doubl
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     cudaError_t e = cudaStreamIsCapturing(st, &cap);
     if (e != cudaSuccess) return e;
-    if (cap != cudaStreamCaptureStatusNone)
-        return hillsum_batch(b->D, b->lo, b->hi, npts, pts, ps, b->nh, b->d_hills, V, dV, gs, nullptr, st);
-    const size_t need = hillsum_scratch(npts, b->nh);
+    const size_t need = cap == cudaStreamCaptureStatusNone ? hillsum_scratch(npts, b->nh) : 0;
+    if (need == 0) return hillsum_batch(b->D, b->lo, b->hi, npts, pts, ps, b->nh, b->d_hills, V, dV, gs, nullptr, st);
     std::lock_guard<std::mutex> lock(b->hs_mu);
     if (need > b->cap_hs) {
         // another thread's capture on another stream is no reason to refuse these

@@ -224,3 +224,26 @@ def test_a_captured_batch_is_one_kernel_node(npts, nh, D):
         ok(rt.cudaGraphDestroy(g))
     ok(rt.cudaStreamDestroy(st))
     nb.close()
+
+
+@pytest.mark.parametrize("npts,nh", [(18944, 300), (18945, 300), (18945, 301), (20011, 1), (9472, 64), (9473, 64), (9473, 65),
+                                     (1000, 12000), (1001, 12000), (700, 12001), (12000, 1000), (12001, 1000),
+                                     (33, 2049)])
+@pytest.mark.parametrize("D", [3, 4])
+def test_sums_at_the_edges_of_the_routes(npts, nh, D):
+    lo, hi = systems.CV4_LO[:D], systems.CV4_HI[:D]
+    c, h, s = _hills(nh, D, npts, True)
+    rng = np.random.default_rng(npts)
+    p = lo + (hi - lo) * (1.2 * rng.random((npts, D)) - 0.1)
+    bad = rng.choice(npts, 3, replace=False)
+    p[bad, 0] = np.nan, np.inf, -np.inf
+    nb = mtd.NNBias(lo, hi)
+    nb.add_hills(c, h, s)
+    gv, gd = nb.exact(p)
+    nb.close()
+    assert not np.any(gv[bad]) and not np.any(gd[bad])
+    some = np.setdiff1d(np.concatenate([np.arange(40), rng.choice(npts, 400), np.arange(npts - 40, npts)]) % npts, bad)
+    V, dV, aV, adV = _sum(p[some], c, h, s)
+    cut = nh * np.abs(h).max() * np.exp(-40.0)
+    assert np.all(np.abs(gv[some] - V) <= 1e-13 * aV + cut)
+    assert np.all(np.abs(gd[some] - dV) <= 1e-13 * adV + 10 * cut / s.min())
