@@ -157,12 +157,15 @@ __global__ void k_place(CellGrid g, SysDev s) {
 // by cluster barriers instead of launches: bin, scan (a chunk of cells per
 // block, the blocks' totals read from each other's shared memory; the counts
 // are zeroed for the next build as they are read), scatter, place.  The same
-// per-atom work and the same order as the five kernels.  A small system's
-// kernels are all latency: 4,000 atoms 33 us (five kernels, event intervals)
-// and 17 now, 32,000 atoms 40 and 23, 61,000 atoms 34 and 34 on a tenth of
-// the SMs and with four launches fewer; beyond 65,536 the five kernels.
-// (A sparse system's empty cells, beyond 16 a thread, are left to them too.)
-constexpr int kClusterBlocks = 16, kClusterAtoms = 4, kClusterCells = 16;   // per thread
+// per-atom work and the same order as the five kernels, for up to an atom and
+// 16 cells a thread (a sparse system's empty cells are work for the whole GPU).
+// A small system's kernels are all latency, and five launches cost more than
+// 16 SMs do: a step of local Q4 + Q6, three contexts in turn, 21.8 us at 4,000
+// atoms and 29.2 with the five kernels, 24.9 and 29.3 at 8,000, 32.6 and 32.7 at
+// 16,000, but 39.7 and 37.5 at 20,000, 59.1 and 45.9 at 42,000, 76.7 and 59.6 at
+// 65,000 (a step alone 56 and 61, 62 and 63, 78 and 76, 97 and 96, 116 and 105,
+// 147 and 127).
+constexpr int kClusterBlocks = 16, kClusterAtoms = 1, kClusterCells = 16;   // per thread
 __global__ void __launch_bounds__(kScanBlock) k_cells_cluster(CellGrid g, SysDev s) {
     pdl_entry();
     __shared__ int sum;
