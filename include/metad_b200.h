@@ -113,7 +113,9 @@ mtd_status mtd_post_force(mtd_ctx *ctx, int64_t step, int n, const double *x, co
  * bias, HILLS rows) without waiting, and waits only when four are pending (or,
  * with the hill-list bias, for the previous step, whose hill joins the list
  * on the host).  mtd_compute_scalar / _vector report the last collected step;
- * mtd_sync() collects every step and reports device error flags. */
+ * mtd_sync() collects every step and reports device error flags.  A step gives
+ * the values of mtd_post_force up to the rounding of sums: STEINH Q of 16,385 to
+ * 32,768 atoms adds in another order there. */
 mtd_status mtd_post_force_device(mtd_ctx *ctx, int64_t step, int n, const double *d_x, const int *d_mask,
                                  const int *d_image, const double *d_f_in, double *d_f_out);
 

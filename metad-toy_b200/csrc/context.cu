@@ -210,9 +210,9 @@ mtd_status alloc_env(mtd_ctx *c, Env &e, int npad) {
 // virial partials.
 // (STEINH L of a walker keeps a thread per atom, as the one-launch step of all
 // walkers has it: the two give the same results bit for bit.)
-static int unit_block(const mtd_ctx *c, const Unit &u) {
+static int unit_block(const mtd_ctx *c, const Unit &u, bool host) {
     if (u.kind == CAL_STRU_FACTOR) return lanes_block(c->n, kLaneAtomsSf);
-    if (u.kind == CAL_STEINH_Q) return lanes_block(c->n, c->host_call ? kLaneAtomsHost : kLaneAtoms);
+    if (u.kind == CAL_STEINH_Q) return lanes_block(c->n, host ? kLaneAtomsHost : kLaneAtoms);
     return c->ring ? lanes_block(c->n) : kBlock;
 }
 
@@ -270,10 +270,9 @@ mtd_status ensure_capacity(mtd_ctx *c, int n) {
     const int npad = ((n + kBlock - 1) / kBlock) * kBlock + kBlock;
     c->n = n;
     c->npad = npad;
-    if (n != c->n_plan || c->host_call != c->host_plan) {   // the bias kernel reads ceil(n / block) partials per unit
+    if (n != c->n_plan) {   // the bias kernel reads ceil(n / block) partials per unit
         c->plan_dirty = true;
         c->n_plan = n;
-        c->host_plan = c->host_call;
     }
     if (npad > c->cap_n) {
         const int cap = npad + npad / 4;
@@ -366,7 +365,7 @@ mtd_status grow_lists(mtd_ctx *c, unsigned need_all, unsigned cand_need, unsigne
     return MTD_OK;
 }
 
-void build_plan(mtd_ctx *c) {
+void build_plan(mtd_ctx *c, bool host) {
     BiasPlan &P = c->plan;
     const Config &cfg = c->cfg;
     P.D = cfg.cv_dim;
@@ -404,7 +403,7 @@ void build_plan(mtd_ctx *c) {
             Q.sk_n = U.skn;
         } else {
             Q.partials = U.partials;
-            Q.nparts = (c->n + unit_block(c, U) - 1) / unit_block(c, U);
+            Q.nparts = (c->n + unit_block(c, U, host) - 1) / unit_block(c, U, host);
             Q.pstride = 8;
             Q.nvals = U.kind == CAL_STEINH_L ? 5 : 4;
             Q.rho = nullptr;
@@ -421,6 +420,18 @@ void build_plan(mtd_ctx *c) {
     P.status = c->d_status;
     P.save = c->d_ws1;
     P.gsum = c->nown >= 0 ? c->d_xchg : nullptr;
+}
+
+cudaError_t upload_plans(mtd_ctx *c) {
+    std::vector<BiasPlan> both;
+    for (int host = 0; host < 2; ++host) {
+        build_plan(c, host != 0);
+        both.push_back(c->plan);
+    }
+    cudaError_t e = cudaMemcpyAsync(c->d_plan, both.data(), 2 * sizeof(BiasPlan), cudaMemcpyHostToDevice, c->st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
+    c->plan_dirty = e != cudaSuccess;
+    return e;
 }
 
 // Neighbour-list and CV-unit layout from the parsed CAL table (env pooling as in
@@ -619,7 +630,7 @@ template <typename T> LocalDev<T> local_dev(mtd_ctx *c, Unit &u, const CellGrid 
     d.lam = (T *)u.lam; d.g = (T *)u.g; d.tu = (T *)u.tu; d.partials = u.partials; d.coef = u.coef;
     d.qblock = c->tune_q;
     d.lblock = c->tune_l;
-    d.lanes = unit_block(c, u) < kBlock;
+    d.lanes = unit_block(c, u, c->host_call) < kBlock;
     d.qsplit = c->tune_qsplit;
     return d;
 }
@@ -632,7 +643,7 @@ template <typename T> GlobalDev<T> global_dev(mtd_ctx *c, Unit &u, const CellGri
     d.smask = c->smask; d.perm = c->perm; d.geo = make_geo<T>(g, c->pf, c->xs); d.exact = geo_d(g, c->xs);
     d.nb = env_dev(c->envs[u.env]);
     d.q = (T *)u.q; d.Q = (T *)u.Q; d.partials = u.partials; d.coef = u.coef;
-    d.lanes = unit_block(c, u) < kBlock;
+    d.lanes = unit_block(c, u, c->host_call) < kBlock;
     return d;
 }
 
@@ -731,7 +742,7 @@ void run_forces(mtd_ctx *c, const SysDev &s, const CellGrid &g, const double *x,
         if (!u.used) continue;
         const double *src = first ? fin : fout;
         double *vp = virial ? c->d_vpart + (size_t)voff * 8 : nullptr;
-        const int nb = (c->n + unit_block(c, u) - 1) / unit_block(c, u);
+        const int nb = (c->n + unit_block(c, u, c->host_call) - 1) / unit_block(c, u, c->host_call);
         if (u.kind == CAL_STEINH_L) {
             launch_local_forces<T>(local_dev<T>(c, u, g), src, fout, s, g, vp, c->d_status, st);
             c->launches += 2;
@@ -785,7 +796,7 @@ mtd_status enqueue_values(mtd_ctx *c, int n, const double *x, const int *mask, c
         return fail(c, MTD_ERR_INVALID_ARG, "domain decomposition: nlocal " + std::to_string(c->nown) +
                                                 " exceeds the " + std::to_string(n) + " atoms of this step");
     if (c->nown >= 0 && !c->d_xchg) {
-        build_plan(c);
+        build_plan(c, c->host_call);
         c->xchg_n = unit_sums_count(c->plan);
         MTD_CU(dalloc(&c->d_xchg, sizeof(double) * (size_t)c->xchg_n), "domain totals");
         MTD_CU(cudaHostAlloc((void **)&c->h_xchg, sizeof(double) * (size_t)c->xchg_n, cudaHostAllocDefault),
@@ -795,12 +806,7 @@ mtd_status enqueue_values(mtd_ctx *c, int n, const double *x, const int *mask, c
     CellGrid g;
     const bool skin = skin_grid(c, g);
     c->last_grid = g;
-    if (c->plan_dirty) {
-        build_plan(c);
-        MTD_CU(cudaMemcpyAsync(c->d_plan, &c->plan, sizeof(BiasPlan), cudaMemcpyHostToDevice, c->st), "plan");
-        MTD_CU(cudaStreamSynchronize(c->st), "plan");
-        c->plan_dirty = false;
-    }
+    if (c->plan_dirty) MTD_CU(upload_plans(c), "plan");
     SysDev s = sys_dev(c, x, mask, image);
     if (!c->envs.empty()) {
         mtd_status sc = ensure_cells(c, g.ncell);
@@ -938,13 +944,13 @@ mtd_status enqueue_step(mtd_ctx *c, long long step, int n, const double *x, cons
         if (s != MTD_OK) return s;
     }
     if (c->nb) {   // hill-list bias: CVs, V and dV/ds at s, deposit and coefficients
-        launch_list_cvs(c->d_plan, c->d_ws1, c->st);
+        launch_list_cvs(plan_now(c), c->d_ws1, c->st);
         s = nnbias_enqueue_vdv(c->nb, c->d_out, c->d_vdv, c->nn_usable, c->h_fit, c->st);
         if (s != MTD_OK) return fail(c, s, mtd_nnbias_last_error(c->nb));
-        launch_list_finish(c->d_plan, step, c->d_ws1, c->d_vdv, c->st);
+        launch_list_finish(plan_now(c), step, c->d_ws1, c->d_vdv, c->st);
         c->launches += 4;
     } else {
-        launch_bias_step(c->d_plan, step, c->st);
+        launch_bias_step(plan_now(c), step, c->st);
         c->launches += 1;
     }
     if (f_ready) MTD_CU(cudaStreamWaitEvent(c->st, f_ready, 0), "force upload");
@@ -1058,12 +1064,7 @@ mtd_status walk_desc(mtd_ctx *c, int n, const double *x, double *f, WalkDesc<T> 
         if (g.periodic[a] && g.nc[a] < 3) *ok = false;
     if (!*ok) return MTD_OK;
     c->last_grid = g;
-    if (c->plan_dirty) {
-        build_plan(c);
-        MTD_CU(cudaMemcpyAsync(c->d_plan, &c->plan, sizeof(BiasPlan), cudaMemcpyHostToDevice, c->st), "plan");
-        MTD_CU(cudaStreamSynchronize(c->st), "plan");
-        c->plan_dirty = false;
-    }
+    if (c->plan_dirty) MTD_CU(upload_plans(c), "plan");
     st = ensure_cells(c, g.ncell);
     if (st != MTD_OK) return st;
     SysDev s = sys_dev(c, x, nullptr, nullptr);
@@ -1204,7 +1205,7 @@ mtd_status mtd_create(int narg, const char *const *arg, const mtd_options *opt, 
     mtd_status s = plan_units(c);
     if (s == MTD_OK) {
         cudaError_t ce = cudaSuccess;
-        ce = dalloc(&c->d_plan, sizeof(BiasPlan));
+        ce = dalloc(&c->d_plan, 2 * sizeof(BiasPlan));
         if (ce == cudaSuccess) ce = dalloc(&c->d_slot, sizeof(OutSlot));
         if (ce == cudaSuccess) ce = dalloc(&c->d_hills, sizeof(HillRec) * kHillCap);
         if (ce == cudaSuccess) ce = cudaMemset(c->d_slot, 0, sizeof(OutSlot));
@@ -1306,10 +1307,7 @@ mtd_status mtd_init(mtd_ctx *c) {
         MTD_CU(dalloc(&c->d_grid, sizeof(double) * (size_t)c->grid_size), "bias grid");
         MTD_CU(cudaMemset(c->d_grid, 0, sizeof(double) * (size_t)c->grid_size), "bias grid");
     }
-    c->plan_dirty = true;
-    build_plan(c);
-    MTD_CU(cudaMemcpy(c->d_plan, &c->plan, sizeof(BiasPlan), cudaMemcpyHostToDevice), "plan");
-    c->plan_dirty = false;
+    MTD_CU(upload_plans(c), "plan");
     const std::string hp = path_in(c, c->hills_path);
     bool appended = false;
     if (c->cfg.restart && !hp.empty()) {

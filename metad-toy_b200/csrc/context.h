@@ -137,9 +137,9 @@ struct mtd_ctx {
     std::vector<Env> envs;
     std::vector<Unit> units;
     BiasPlan plan{};
-    BiasPlan *d_plan = nullptr;
+    BiasPlan *d_plan = nullptr;          // [2]: of steps on device arrays and of host calls (unit_block)
     bool plan_dirty = true;
-    bool host_call = false, host_plan = false;   // inside a call that waits for its step (host arrays); the plan's
+    bool host_call = false;              // inside a call that waits for its step (host arrays)
     double *d_grid = nullptr;
     long long grid_size = 0;
     HillRec *d_hills = nullptr;
@@ -282,7 +282,11 @@ mtd_status ensure_capacity(mtd_ctx *c, int n);
 // a few MB back to back reach ~50 GB/s.
 cudaError_t h2d_pieces(void *dst, const void *src, size_t bytes, cudaStream_t st);
 mtd_status ensure_cells(mtd_ctx *c, int ncell);
-void build_plan(mtd_ctx *c);
+void build_plan(mtd_ctx *c, bool host);
+// Builds both plans and copies them to the device.
+cudaError_t upload_plans(mtd_ctx *c);
+// The device plan of the step being enqueued.
+inline const BiasPlan *plan_now(const mtd_ctx *c) { return c->d_plan + (c->host_call ? 1 : 0); }
 mtd_status plan_units(mtd_ctx *c);
 int owned(const mtd_ctx *c);
 NeighDev env_dev(const Env &e);

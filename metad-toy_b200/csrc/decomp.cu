@@ -18,7 +18,7 @@ namespace ctx {
 // bias force and return MTD_ERR_NAN.
 mtd_status exchange_totals(mtd_ctx *c) {
     const int cnt = c->xchg_n;
-    launch_unit_sums(c->d_plan, c->d_xchg, c->st);
+    launch_unit_sums(plan_now(c), c->d_xchg, c->st);
     c->launches += 1;
     if (c->dom_dev_fn) {   // the caller enqueues the sum over ranks on the step's stream
         if (c->dom_dev_fn(c->d_xchg, cnt, (void *)c->st, c->dom_user) != 0)

@@ -50,14 +50,12 @@ mtd_status replay_records(mtd_ctx *c, const std::vector<HillRec> &recs) {
     if (c->nb) return list_add_hills(c, recs);
     HillRec *d = nullptr;
     MTD_CU(dalloc(&d, sizeof(HillRec) * recs.size()), "replay");
-    cudaMemcpy(d, recs.data(), sizeof(HillRec) * recs.size(), cudaMemcpyHostToDevice);
-    if (c->plan_dirty) {
-        build_plan(c);
-        cudaMemcpy(c->d_plan, &c->plan, sizeof(BiasPlan), cudaMemcpyHostToDevice);
-        c->plan_dirty = false;
+    cudaError_t e = cudaMemcpy(d, recs.data(), sizeof(HillRec) * recs.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && c->plan_dirty) e = upload_plans(c);
+    if (e == cudaSuccess) {
+        launch_hills_replay(c->d_plan, d, (int)recs.size(), (int)c->grid_size, c->st);
+        e = cudaStreamSynchronize(c->st);
     }
-    launch_hills_replay(c->d_plan, d, (int)recs.size(), (int)c->grid_size, c->st);
-    cudaError_t e = cudaStreamSynchronize(c->st);
     cudaFree(d);
     return cuda_check(c, e, "HILLS replay");
 }

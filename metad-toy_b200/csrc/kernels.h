@@ -242,8 +242,11 @@ cudaError_t launch_rebuild(const CellGrid &g, const SysDev &s, const NeighSpec &
 // 32,000 (FERMI 28.9 and 52.4, 56.0 and 68.8, 96.5 and 93.7); Q4 with cutoff 6
 // 25.9 and 37.4 at 6,900, 42.6 and 45.8 at 16,384, 72.9 and 60.8 at 32,000;
 // Debye 29.3 and 40.5 at 16,384, 49.0 and 49.4 at 32,000, 85 and 79 at 62,500.
-// A call on host arrays waits for its step, so there a step alone counts: Q4
-// with cutoff 6 at 32,000 atoms 182 us a call with the lanes, 198 without.
+// A call of STEINH Q on host arrays waits for its step, so there a step alone
+// counts (us a call, lanes and thread per atom): Q4 with cutoff 6, cap 12, 140 and
+// 167 at 19,652 atoms, 187 and 195 at 32,000, 222 and 230 at 42,592, 258 and 248 at
+// 55,296; Q6 with cutoff 3.9, cap 18, 126 and 138, 167 and 161, 204 and 194, 219
+// and 211; in FP64 the same within 4 %.
 constexpr int kLaneAtoms = 16384, kLaneAtomsSf = 32768, kLaneAtomsHost = 32768;
 constexpr int kLanes = 8;
 inline int lanes_block(int n, int most = kLaneAtoms) { return n <= most ? kBlock / kLanes : kBlock; }

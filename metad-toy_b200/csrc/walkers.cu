@@ -323,9 +323,7 @@ mtd_status mtd_walkers_init(mtd_walkers *W) {
             cudaFree(c->d_grid);
             c->d_grid = c0->d_grid;   // one grid for the group
         }
-        build_plan(c);
-        MTD_WCU(cudaMemcpy(c->d_plan, &c->plan, sizeof(BiasPlan), cudaMemcpyHostToDevice), "plan");
-        c->plan_dirty = false;
+        MTD_WCU(upload_plans(c), "plan");
         plans[k] = c->d_plan;
     }
     W->initialized = true;
