@@ -578,6 +578,7 @@ mtd_status plan_units(mtd_ctx *c) {
             MTD_CU(dalloc(&u.kvec, sizeof(double) * 3 * u.K), "k vectors");
             MTD_CU(dalloc(&u.rho, sizeof(double) * 2 * u.K), "rho");
             MTD_CU(dalloc(&u.skn, sizeof(double)), "rho");
+            for (double k : d.kvecs) u.kmax = std::fmax(u.kmax, std::fabs(k));
             MTD_CU(cudaMemcpy(u.kvec, d.kvecs.data(), sizeof(double) * 3 * u.K, cudaMemcpyHostToDevice), "k vectors");
         }
     }
@@ -664,6 +665,7 @@ SkDev sk_dev(mtd_ctx *c, Unit &u, const double *x, const int *mask) {
     d.n = c->n; d.K = u.K; d.groupbit = u.groupbit; d.x = x; d.mask = mask; d.k = u.kvec;
     d.partials = u.partials; d.nblocks = u.nblocks; d.rho = u.rho; d.ngroup = u.skn; d.coef = u.coef;
     d.fp64 = c->fp64;
+    d.reach = (c->fp64 ? kPhaseMax : kTurnMax * kPi) / std::fmax(u.kmax, 1e-300);
     d.nown = owned(c);
     d.qv = c->tune_skq;
     d.qf = c->tune_skqf;

@@ -69,6 +69,7 @@ struct Unit {
     double *coef = nullptr;
     int K = 0;
     double *kvec = nullptr, *rho = nullptr, *skn = nullptr;
+    double kmax = 0;   // largest |component| of the k-vectors
     // S(k), mixed precision: per-dimension phase tables for the box they were built for
     // STRU_FACTOR Chemical: type-weight parameters, the table built from the
     // types of mtd_set_types, and the per-atom weights (sorted order)

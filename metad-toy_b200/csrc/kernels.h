@@ -346,7 +346,8 @@ struct SkDev {
     const double *x;            // caller order AoS
     const int *mask;
     const double *k;            // K*3
-    double *partials;           // [nblocks][2K]
+    double reach;               // |x| + |y| + |z| below this keeps every phase in the passes' range
+    double *partials;           // [2K + 1][nblocks]: (re, im) of each k, then the group count
     int nblocks;
     double *rho;                // 2K (re, im)
     double *ngroup;             // group count

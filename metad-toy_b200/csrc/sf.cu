@@ -182,18 +182,6 @@ constexpr int kSkBlocks = 148 * 4;   // resident blocks of both passes
 constexpr int kSkChunk = 512;        // atoms staged at a time in the value pass
 constexpr int kSkFlush = 8;          // most atoms summed in FP32 before they join the FP64 sums
 
-// Largest |component| of k / pi over all k-vectors, on every thread of the
-// block: |u| of an atom is at most that times |x| + |y| + |z|.
-__device__ __forceinline__ double sk_kmax(const SkDev &d, double *smem /* 8 */) {
-    double m = 0.0;
-    for (int t = threadIdx.x; t < 3 * d.K; t += blockDim.x) m = fmax(m, fabs(d.k[t]) * kInvPi);
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) smem[threadIdx.x >> 5] = m;
-    __syncthreads();
-    for (int w = 0; w < (int)blockDim.x >> 5; ++w) m = fmax(m, smem[w]);
-    return m;
-}
-
 // sin(pi f), cos(pi f) (unsigned) and the sign masks of one atom's phases with
 // a pair of k-vectors (/ pi); far: beyond the base's range or not finite, the
 // phase is then rounded in FP64.
@@ -237,12 +225,11 @@ __global__ void __launch_bounds__(256, FP64 ? 2 : 4) k_sk_partial(SkDev d, int p
     pdl_entry();
     __shared__ double2 xy[kSkChunk];
     __shared__ double zz[kSkChunk];
-    __shared__ double smem[8];
     __shared__ int wcount[2][8];
     const int np = (d.K + 1) / 2, ntile = (np + 63) / 64, TP = (np + ntile - 1) / ntile, S = (int)blockDim.x / TP;
     const int st = threadIdx.x / TP, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int a0 = min(blockIdx.x * per, d.nown), a1 = min(a0 + per, d.nown);
-    const double reach = (FP64 ? kPhaseMax * kInvPi : kTurnMax) / fmax(sk_kmax(d, smem), 1e-300);
+    const double reach = d.reach;
     int total = 0;
     for (int tile = 0; tile < ntile; ++tile) {
         const int p = tile * TP + (int)threadIdx.x % TP;
@@ -451,7 +438,7 @@ __global__ void __launch_bounds__(256, FP64 ? 2 : 4)
         if (FP64) reinterpret_cast<double *>(wd)[q] = amp;
         kd[6] = FP64 ? ph : kTurnBase - ph * kInvPi;
     }
-    const double reach = (FP64 ? kPhaseMax * kInvPi : kTurnMax) / fmax(sk_kmax(d, smem), 1e-300);
+    const double reach = d.reach;
     __syncthreads();
     for (int tile = blockIdx.x; tile * 256 * AT < d.n; tile += gridDim.x) {
         using R2 = typename std::conditional<FP64, double2, float2>::type;
