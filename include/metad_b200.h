@@ -115,7 +115,7 @@ mtd_status mtd_post_force(mtd_ctx *ctx, int64_t step, int n, const double *x, co
  * on the host).  mtd_compute_scalar / _vector report the last collected step;
  * mtd_sync() collects every step and reports device error flags.  A step gives
  * the values of mtd_post_force up to the rounding of sums: STEINH Q of 16,385 to
- * 32,768 atoms adds in another order there. */
+ * 32,768 atoms and STRU_FACTOR of 22,529 to 32,768 add in another order there. */
 mtd_status mtd_post_force_device(mtd_ctx *ctx, int64_t step, int n, const double *d_x, const int *d_mask,
                                  const int *d_image, const double *d_f_in, double *d_f_out);
 

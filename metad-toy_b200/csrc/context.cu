@@ -211,7 +211,8 @@ mtd_status alloc_env(mtd_ctx *c, Env &e, int npad) {
 // (STEINH L of a walker keeps a thread per atom, as the one-launch step of all
 // walkers has it: the two give the same results bit for bit.)
 static int unit_block(const mtd_ctx *c, const Unit &u, bool host) {
-    if (u.kind == CAL_STRU_FACTOR) return lanes_block(c->n, kLaneAtomsSf);
+    if (u.kind == CAL_STRU_FACTOR)
+        return lanes_block(c->n, host ? kLaneAtomsHost : c->fp64 ? kLaneAtomsSf64 : kLaneAtomsSf);
     if (u.kind == CAL_STEINH_Q) return lanes_block(c->n, host ? kLaneAtomsHost : kLaneAtoms);
     return c->ring ? lanes_block(c->n) : kBlock;
 }
@@ -219,7 +220,7 @@ static int unit_block(const mtd_ctx *c, const Unit &u, bool host) {
 mtd_status alloc_unit(mtd_ctx *c, Unit &u, int npad) {
     const size_t R = real_size(c);
     const int SQ = record_stride(c, u);
-    const int nb = std::max((npad + kBlock - 1) / kBlock, (std::min(npad, kLaneAtomsSf) * kLanes + kBlock - 1) / kBlock);
+    const int nb = std::max((npad + kBlock - 1) / kBlock, (std::min(npad, kLaneAtomsHost) * kLanes + kBlock - 1) / kBlock);
     void **arrs[] = {&u.q, &u.nf, &u.lq, &u.lqs, &u.e12, &u.lam, &u.g, &u.tu, &u.Q, &u.S, &u.w};
     for (void **a : arrs) dfree(*a);
     dfree(u.partials);
@@ -653,6 +654,7 @@ template <typename T> DebyeDev<T> debye_dev(mtd_ctx *c, Unit &u, const CellGrid 
     d.n = c->n; d.npad = c->cap_n; d.groupbit = u.groupbit; d.rc2 = u.rc * u.rc; d.qf = u.qf; d.sw = u.sf_sw;
     d.smask = c->smask; d.perm = c->perm; d.geo = make_geo<T>(g, c->pf, c->xs); d.nb = env_dev(c->envs[u.env]);
     d.S = (T *)u.S; d.partials = u.partials; d.coef = u.coef;
+    d.lanes = unit_block(c, u, c->host_call) < kBlock;
     d.w = u.chem ? (T *)u.w : nullptr;
     d.types = c->d_types;
     d.wtab = u.d_wtab;

@@ -241,13 +241,15 @@ cudaError_t launch_rebuild(const CellGrid &g, const SysDev &s, const NeighSpec &
 // precision 20.9 and 26.4 at 4,000, 32.7 and 34.1 at 16,000, 52.9 and 46.5 at
 // 32,000 (FERMI 28.9 and 52.4, 56.0 and 68.8, 96.5 and 93.7); Q4 with cutoff 6
 // 25.9 and 37.4 at 6,900, 42.6 and 45.8 at 16,384, 72.9 and 60.8 at 32,000;
-// Debye 29.3 and 40.5 at 16,384, 49.0 and 49.4 at 32,000, 85 and 79 at 62,500.
-// A call of STEINH Q on host arrays waits for its step, so there a step alone
+// Debye 28.1 and 37.6 at 16,384, 35.0 and 42.1 at 23,328, 44.8 and 42.5 at 32,000,
+// in FP64 33.3 and 39.6, 45.6 and 44.8, 57.3 and 46.8.
+// A call of STEINH Q or STRU_FACTOR on host arrays waits for its step, so there a step alone
 // counts (us a call, lanes and thread per atom): Q4 with cutoff 6, cap 12, 140 and
 // 167 at 19,652 atoms, 187 and 195 at 32,000, 222 and 230 at 42,592, 258 and 248 at
 // 55,296; Q6 with cutoff 3.9, cap 18, 126 and 138, 167 and 161, 204 and 194, 219
 // and 211; in FP64 the same within 4 %.
-constexpr int kLaneAtoms = 16384, kLaneAtomsSf = 32768, kLaneAtomsHost = 32768;
+// Debye, a step alone 82.8 and 109 at 32,000, in FP64 97 and 120.
+constexpr int kLaneAtoms = 16384, kLaneAtomsSf = 28672, kLaneAtomsSf64 = 22528, kLaneAtomsHost = 32768;
 constexpr int kLanes = 8;
 inline int lanes_block(int n, int most = kLaneAtoms) { return n <= most ? kBlock / kLanes : kBlock; }
 // Sum over the G lanes of an atom (G neighbouring lanes, all in the warp).
@@ -334,6 +336,7 @@ template <typename T> struct DebyeDev {
     const int *types;           // caller-order atom types (Chemical)
     const double *wtab;         // weight of each type 0..ntab-1 (Chemical)
     int ntab;
+    int lanes;                  // kLanes lanes per atom instead of one thread
 };
 template <typename T> void launch_debye_values(const DebyeDev<T> &d, cudaStream_t st);
 template <typename T>

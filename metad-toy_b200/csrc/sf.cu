@@ -523,8 +523,8 @@ __global__ void __launch_bounds__(256, FP64 ? 2 : 4)
 template <typename T> void launch_debye_values(const DebyeDev<T> &d, cudaStream_t st) {
     if (d.n == 0) return;
     if (d.w) launch_k(k_chem_weights<T>, (d.n + kBlock - 1) / kBlock, kBlock, 0, st, d);
-    const int ab = lanes_block(d.n, kLaneAtomsSf), nb = (d.n + ab - 1) / ab;
-    if (ab < kBlock) launch_k(k_debye_values<T, kLanes>, nb, kBlock, 0, st, d);
+    const int ab = d.lanes ? kBlock / kLanes : kBlock, nb = (d.n + ab - 1) / ab;
+    if (d.lanes) launch_k(k_debye_values<T, kLanes>, nb, kBlock, 0, st, d);
     else launch_k(k_debye_values<T, 1>, nb, kBlock, 0, st, d);
     prof_mark("debye_values", st);
 }
@@ -532,8 +532,8 @@ template <typename T>
 void launch_debye_forces(const DebyeDev<T> &d, const double *f_src, double *f_dst, const SysDev &s, const CellGrid &g,
                          double *vpart, DevStatus *status, cudaStream_t st) {
     if (d.n == 0) return;
-    const int ab = lanes_block(d.n, kLaneAtomsSf), nb = (d.n + ab - 1) / ab;
-    if (ab < kBlock) launch_k(k_debye_force<T, kLanes>, nb, kBlock, 0, st, d, f_src, f_dst, s, g, vpart, status);
+    const int ab = d.lanes ? kBlock / kLanes : kBlock, nb = (d.n + ab - 1) / ab;
+    if (d.lanes) launch_k(k_debye_force<T, kLanes>, nb, kBlock, 0, st, d, f_src, f_dst, s, g, vpart, status);
     else launch_k(k_debye_force<T, 1>, nb, kBlock, 0, st, d, f_src, f_dst, s, g, vpart, status);
     prof_mark("debye_force", st);
 }

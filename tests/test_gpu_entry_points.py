@@ -1,7 +1,8 @@
 """One context stepped through its host and its device entry points in turn, and
 through errors and replays in between.  STEINH Q splits an atom's neighbours over
-eight lanes up to 16,384 atoms, from host arrays up to 32,768, and the bias kernel
-has to read the partial sums of the split that ran.
+eight lanes up to 16,384 atoms (STRU_FACTOR up to 28,672, in FP64 22,528), from host
+arrays up to 32,768, and the bias kernel has to read the partial sums of the split
+that ran.
 
 Tolerance against the oracle: FP64 sums of n atoms in another order, 1e-12
 relative; forces 1e-10 of the largest.
@@ -17,9 +18,11 @@ pytestmark = pytest.mark.gpu
 RC, CAP = 4.0, 7
 
 
-def _args():
-    return ["GAUSSIAN", 0.01, 0.005, 10.0, "PACE", 1, "CAL", "NAME", "C", "STEINH", "Q", 4, "all", "cutoff_r", RC,
-            "cutoff_Natoms", CAP, "SYMBOL", "v1", "C.AVE", "CV_dim", 1, "DIM", 1, 0.0, 1.0, 400, "v1", "WT", 0]
+def _args(kind="Q"):
+    cal = ["STEINH", "Q", 4, "all", "cutoff_r", RC, "cutoff_Natoms", CAP] if kind == "Q" else \
+        ["STRU_FACTOR", "all", "cutoff_r", RC, "q_factor", 2.8]
+    return ["GAUSSIAN", 0.01, 0.005, 10.0, "PACE", 1, "CAL", "NAME", "C"] + cal + \
+        ["SYMBOL", "v1", "C.AVE", "CV_dim", 1, "DIM", 1, 0.0, 1.0, 400, "v1", "WT", 0]
 
 
 def _system(n):
@@ -43,11 +46,12 @@ def _host(m, step, x):
     return m.cv.copy(), f
 
 
-@pytest.mark.parametrize("n", [16384, 16385, 20000, 32768, 32769])
-def test_host_and_device_steps_in_turn(n):
+@pytest.mark.parametrize("kind,n", [("Q", 16384), ("Q", 16385), ("Q", 20000), ("Q", 32768), ("Q", 32769),
+                                    ("SF", 22528), ("SF", 22529), ("SF", 28673), ("SF", 32769)])
+def test_host_and_device_steps_in_turn(kind, n):
     x, L = _system(n)
-    o = O.steinh_q(4, x, L, RC, CAP)
-    m = mtd.Metad(_args(), precision="fp64")
+    o = O.steinh_q(4, x, L, RC, CAP) if kind == "Q" else O.debye(x, L, RC, 2.8)
+    m = mtd.Metad(_args(kind), precision="fp64")
     m.set_box([0, 0, 0], L)
     for step, call in enumerate((_device, _host, _host, _device, _device, _host)):
         cv, f = call(m, step, x)
