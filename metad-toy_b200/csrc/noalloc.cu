@@ -31,8 +31,9 @@ constexpr int kNaChunk = 8;                          // reals per register tile 
 
 static __device__ __align__(256) double g_na_scratch[kNaScratchDoubles];
 
-// FP64: sincos of the FP64 phase.  Mixed: FP64 quadrant reduction, FP32
-// series (phase_sincos_f32, the context's S(k) arithmetic).
+// FP64: sincos of the FP64 phase.  Mixed: half turns taken off in FP64, FP32
+// polynomials (phase_sincos_f32; the context's passes use the same polynomials on
+// phases with their fraction in the low word).
 template <bool FP64> __device__ __forceinline__ void na_sincos(double ph, double &s, double &c) {
     if (FP64) {
         sincos(ph, &s, &c);
