@@ -214,7 +214,7 @@ static int unit_block(const mtd_ctx *c, const Unit &u, bool host) {
     if (u.kind == CAL_STRU_FACTOR)
         return lanes_block(c->n, host ? kLaneAtomsHost : c->fp64 ? kLaneAtomsSf64 : kLaneAtomsSf);
     if (u.kind == CAL_STEINH_Q) return lanes_block(c->n, host ? kLaneAtomsHost : kLaneAtoms);
-    return c->ring ? lanes_block(c->n) : kBlock;
+    return u.kind == CAL_STEINH_L && c->ring ? lanes_block(c->n) : kBlock;
 }
 
 mtd_status alloc_unit(mtd_ctx *c, Unit &u, int npad) {
