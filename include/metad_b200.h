@@ -254,8 +254,9 @@ int mtd_profile_report(mtd_ctx *ctx, char *buf, int len);
 
 /* Autotuner: times the interchangeable kernel shapes on device positions
  * d_x (n x 3, caller order; d_mask may be NULL) over `reps` launches each and
- * keeps the fastest -- the neighbour search (0: 256-thread blocks, 1:
- * 128-thread blocks, 2: flat per-thread candidate loop) and the threads per
+ * keeps the fastest -- the neighbour search (0: a warp per atom up to 65,536
+ * atoms, 131,072 with a smooth switch, beyond that a thread per atom in
+ * 256-thread blocks, 1: 128-thread blocks, 2: flat per-thread candidate loop) and the threads per
  * block of the q and lambda passes (256 or 128).  Every shape gives
  * bitwise-identical results, so tuning never changes a step's output; it
  * records no step and deposits nothing.  choice (may be NULL) receives the

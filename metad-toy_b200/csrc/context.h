@@ -201,7 +201,7 @@ struct mtd_ctx {
     int *d_types = nullptr;
     int types_cap = 0, types_n = -1;
     // kernel shapes chosen by mtd_autotune (every choice gives bitwise-identical results)
-    int tune_nbr = 0;                    // neighbour search: 0 fast/256, 1 fast/128, 2 flat/128
+    int tune_nbr = 0;                    // neighbour search: 0 warp per atom or fast/256 (by size), 1 fast/128, 2 flat/128
     int tune_q = 0, tune_l = 0;          // threads per block of the q and lambda passes (0: 256)
     int tune_qsplit = 0;                 // skin lists: the q pass's filter in its own loop (1) or merged (0)
     int tune_skq = 8, tune_skqf = 2;     // S(k): phases in flight per thread of the value pass, unroll of the force pass
