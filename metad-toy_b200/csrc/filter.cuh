@@ -76,9 +76,9 @@ __device__ __forceinline__ bool decide(const GeoD &gd, const NeighSpec &ns, cons
 
 // Notes a list that found `cnt` neighbours where fewer fit; a capped list's
 // need is kept apart, since it can be met up to kMaxCapList entries only.
-__device__ __forceinline__ void note_overflow(DevStatus *status, const NeighSpec &ns, int cnt) {
+template <int KIND> __device__ __forceinline__ void note_overflow(DevStatus *status, const NeighSpec &ns, int cnt) {
     atomicMax(&status->overflow, (unsigned)cnt);
-    if (ns.cap > 0) atomicMax(&status->cap_overflow, (unsigned)cnt);
+    if (KIND == NK_RANGE && ns.cap > 0) atomicMax(&status->cap_overflow, (unsigned)cnt);
 }
 
 // Skin-list filter of sorted atom k: the candidates found within cutoff +
@@ -109,7 +109,7 @@ __device__ __forceinline__ int filter_atom(const GeoF &gf, const GeoD &gd, const
         ++cnt;
     }
     nd.count[k] = cnt;
-    if (cnt > nd.M) note_overflow(status, ns, cnt);
+    if (cnt > nd.M) note_overflow<KIND>(status, ns, cnt);
     return cnt;
 }
 

@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(kBlock) k_neighbors(CellGrid g, SysDev s, Neig
         }
     }
     nd.count[k] = cnt;
-    if (cnt > nd.M) note_overflow(status, ns, cnt);
+    if (cnt > nd.M) note_overflow<KIND>(status, ns, cnt);
 }
 
 
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(kBlock) k_neighbors_warp(CellGrid g, SysDev s,
     if (KIND == NK_SWITCH && wait > 0) decide_held(wait);
     if (lane == 0) {
         nd.count[k] = cnt;
-        if (cnt > (CAP ? most : nd.M)) note_overflow(status, ns, cnt);
+        if (cnt > (CAP ? most : nd.M)) note_overflow<KIND>(status, ns, cnt);
     }
     if (!CAP) return;
     __syncwarp();
@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(kFlatBlock) k_neighbors_flat(CellGrid g, SysDe
     nd.count[k] = cnt;
     if (cnt > nd.M) {
         if (KIND == NK_CAND) atomicMax(&status->cand_overflow, (unsigned)cnt);
-        else note_overflow(status, ns, cnt);
+        else note_overflow<KIND>(status, ns, cnt);
     }
 }
 

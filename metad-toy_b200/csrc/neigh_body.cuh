@@ -140,7 +140,7 @@ __device__ __forceinline__ void neighbors_fast_body(const CellGrid &g, const Sys
     nd.count[k] = cnt;
     if (cnt > nd.M) {
         if (KIND == NK_CAND) atomicMax(&status->cand_overflow, (unsigned)cnt);
-        else note_overflow(status, ns, cnt);
+        else note_overflow<KIND>(status, ns, cnt);
     }
 }
 
